@@ -124,17 +124,18 @@ int32_t gb_spect_subset_size(const gb_spect_plan *plan, int32_t subset);
 
 /* Tile configuration of a plan's PSF kernels.  Plan creation picks the widest tiles that
  * fit shared memory; gb_spect_autotune times candidates on the device and keeps the
- * fastest.  No counterpart in the reference (which has no device code). */
+ * fastest.  No counterpart in the reference (which has no device code).
+ * Plans with N and nz <= 128 whose attenuation, if any, comes before the PSF run the strip
+ * kernels: of these fields only the work items and osem_split change what runs there. */
 typedef struct gb_spect_tuning {
     int32_t fwd_tpb;   /* threads per forward CTA: 512 or 768 (one CTA per SM) */
     int32_t fwd_zt;    /* forward z-slab width; 0 = the widest that fits */
     int32_t fwd_items; /* forward work items per resident CTA slot and z slab: 1 or 2 */
     int32_t b1_zt;     /* back-projection (rotated frame) z-slab width; 0 = widest */
     int32_t b1_items;  /* back-projection work items per SM and z slab: 1 or 2 */
-    int32_t fwd_variant; /* forward kernel: 1 (samples gathered per plane, y blur first) or 2
-                            (corner rows staged through a cp.async ring, z blur first;
-                            attenuation before a 2-D PSF of at most 29 taps, N and
-                            nz <= 128); 0 keeps the plan's current one */
+    int32_t fwd_variant; /* 1, or 2 for attenuation before a 2-D PSF of at most 29 taps with N
+                            and nz <= 128 and nz % 4 == 0 (both values run the same kernels);
+                            0 keeps the plan's current one */
     int32_t osem_split;  /* 1: gb_spect_osem_step runs the two halves of a subset's angles on
                             two streams (fork / join by events, same kernels and results);
                             0: one stream */

@@ -104,9 +104,69 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// The same table in the strip kernels' rows (zg > 0, any nz): a thread owns the quad at one
+// position of a row; values beyond nz are zero.
+__global__ void __launch_bounds__(256)
+    k_atten_strip(SpectDev g, const float *__restrict__ mu, float dx, float *__restrict__ A) {
+    constexpr int PU = 4;
+    const int a = blockIdx.y, nq = g.nzs / 4;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.nya * nq) return;
+    const int r = i / nq, pos = i % nq, z = z_of_pos(g, pos), y = g.ya_lo + r;
+    const bool vec = g.nz % 4 == 0 && ((uintptr_t)mu & 15) == 0;
+    const int nv = min(4, g.nz - z);  // values of the quad inside the row
+    float th[6];
+#pragma unroll
+    for (int k = 0; k < 6; k++) th[k] = g.theta_fwd[6 * a + k];
+    const float lc = g.lin[y];
+    float *out = A + ((size_t)a * g.Lp * g.nya + r) * g.nzs + 4 * pos;
+    const size_t plane = (size_t)g.nya * g.nzs;
+    float run[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int x0 = g.Lp - 1; x0 >= 0; x0 -= PU) {
+        float v[PU][4];
+#pragma unroll
+        for (int u = 0; u < PU; u++) {
+            const int xp = max(x0 - u, 0);
+            float ix, iy;
+            rot_coords(th, g.lin[xp], lc, g.half, ix, iy);
+            const Bilin b = bilin(ix, iy);
+            if (vec && nv == 4) {
+                float4 s4;
+                sample4(mu, g.N, g.N, g.nz, g.pad, g.pad, b, z, s4);
+                v[u][0] = __fmul_rn(s4.x, dx);
+                v[u][1] = __fmul_rn(s4.y, dx);
+                v[u][2] = __fmul_rn(s4.z, dx);
+                v[u][3] = __fmul_rn(s4.w, dx);
+            } else {
+#pragma unroll
+                for (int w = 0; w < 4; w++)
+                    v[u][w] = w < nv ? __fmul_rn(sample(mu, g.N, g.N, g.nz, g.pad, g.pad, b, z + w),
+                                                 dx)
+                                     : 0.f;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < PU; u++) {
+            const int xp = x0 - u;
+            if (xp < 0) break;
+            float e[4];
+#pragma unroll
+            for (int w = 0; w < 4; w++) {
+                run[w] = __fadd_rn(run[w], v[u][w]);
+                e[w] = w < nv ? expf(-__fsub_rn(run[w], __fmul_rn(v[u][w], 0.5f))) : 0.f;
+            }
+            *reinterpret_cast<float4 *>(out + (size_t)xp * plane) =
+                make_float4(e[0], e[1], e[2], e[3]);
+        }
+    }
+}
+
 cudaError_t launch_atten(const SpectDev &g, const float *mu, float dx, int n_angles, float *A,
                          cudaStream_t st) {
-    if (g.nz % 4 == 0) {
+    if (g.zg) {
+        dim3 grid((g.nya * (g.nzs / 4) + 255) / 256, n_angles);
+        k_atten_strip<<<grid, 256, 0, st>>>(g, mu, dx, A);
+    } else if (g.nz % 4 == 0) {
         dim3 grid((g.nya * (g.nz / 4) + 255) / 256, n_angles);
         k_atten<true><<<grid, 256, 0, st>>>(g, mu, dx, A);
     } else {
@@ -549,6 +609,7 @@ cudaError_t launch_b1(const SpectDev &g, const float *proj, const int *alist, in
         }
         return cudaGetLastError();
     }
+    if (g.strip) return launch_b1_strip(g, proj, alist, items, n_items, W, st);
     switch (g.K) {
 #define GB_B1_CASE(KK) \
     case KK:           \
@@ -734,7 +795,7 @@ __device__ __forceinline__ void apply_update(int mode, const UpdateArgs &u, size
     }
 }
 
-// apply_update for the z quad z..z+3 (z % 4 == 0, nz % 4 == 0).  PRIOR (BSREM with the
+// apply_update for the z quad z..z+3 (z % 4 == 0; values from nz on are left out).  PRIOR (BSREM with the
 // RDP prior): the prior term comes from rdp_sum4, one neighbourhood load for the four
 // voxels; a separate instantiation, so the other modes keep their register count.
 template <bool PRIOR>
@@ -742,11 +803,11 @@ __device__ __forceinline__ void apply_update4(int mode, const UpdateArgs &u, siz
                                               int y, int z, int nx, int ny, int nz, float4 bp4,
                                               float *out) {
     const float bp[4] = {bp4.x, bp4.y, bp4.z, bp4.w};
-    if constexpr (!PRIOR) {
-        apply_update(mode, u, i, x, y, z, nx, ny, nz, bp[0], out);
-        apply_update(mode, u, i + 1, x, y, z + 1, nx, ny, nz, bp[1], out);
-        apply_update(mode, u, i + 2, x, y, z + 2, nx, ny, nz, bp[2], out);
-        apply_update(mode, u, i + 3, x, y, z + 3, nx, ny, nz, bp[3], out);
+    if (!PRIOR || nz % 4 != 0) {  // the last quad of a row may be partial
+#pragma unroll
+        for (int v = 0; v < 4; v++)
+            if (z + v < nz)
+                apply_update<PRIOR>(mode, u, i + v, x, y, z + v, nx, ny, nz, bp[v], out);
         return;
     }
     float f[4], rdp[4];
@@ -776,7 +837,7 @@ __device__ __forceinline__ void apply_update4(int mode, const UpdateArgs &u, siz
 __device__ __forceinline__ float4 b2_gather_sum4(const SpectDev &g, const float *__restrict__ W,
                                                   const int *__restrict__ alist, int n_slots,
                                                   int x, int y, int z) {
-    const int nz = g.nz;
+    const int nz = g.nzs;  // z: first value of the quad in its W row
     const float lr = g.lin[x + g.pad], lc = g.lin[y + g.pad];
     const size_t slab = (size_t)g.Lp * g.nya * nz;
     float4 bp = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -787,10 +848,10 @@ __device__ __forceinline__ float4 b2_gather_sum4(const SpectDev &g, const float 
         rot_coords(g.theta_bwd + 6 * alist[s + 1], lr, lc, g.half, ix2, iy2);
         Bilin b1 = bilin(ix, iy), b2 = bilin(ix2, iy2);
         float4 v1, v2;
-        sample4_ranged(W + s * slab, g.Lp, g.nya, nz, g.ya_lo, g.wrange + (size_t)s * g.Lp, b1,
-                       z, v1);
+        sample4_ranged(W + s * slab, g.Lp, g.nya, nz, g.ya_lo, w_ranges(g, s, alist[s]), b1, z,
+                       v1);
         sample4_ranged(W + (s + 1) * slab, g.Lp, g.nya, nz, g.ya_lo,
-                       g.wrange + (size_t)(s + 1) * g.Lp, b2, z, v2);
+                       w_ranges(g, s + 1, alist[s + 1]), b2, z, v2);
         bp.x = __fadd_rn(__fadd_rn(bp.x, v1.x), v2.x);
         bp.y = __fadd_rn(__fadd_rn(bp.y, v1.y), v2.y);
         bp.z = __fadd_rn(__fadd_rn(bp.z, v1.z), v2.z);
@@ -801,8 +862,8 @@ __device__ __forceinline__ float4 b2_gather_sum4(const SpectDev &g, const float 
         rot_coords(g.theta_bwd + 6 * alist[s], lr, lc, g.half, ix, iy);
         Bilin b1 = bilin(ix, iy);
         float4 v1;
-        sample4_ranged(W + s * slab, g.Lp, g.nya, nz, g.ya_lo, g.wrange + (size_t)s * g.Lp, b1,
-                       z, v1);
+        sample4_ranged(W + s * slab, g.Lp, g.nya, nz, g.ya_lo, w_ranges(g, s, alist[s]), b1, z,
+                       v1);
         bp.x = __fadd_rn(bp.x, v1.x);
         bp.y = __fadd_rn(bp.y, v1.y);
         bp.z = __fadd_rn(bp.z, v1.z);
@@ -830,7 +891,7 @@ __device__ __forceinline__ void b2_make_tap(const SpectDev &g, const int *__rest
     rot_coords(g.theta_bwd + 6 * alist[s], g.lin[x + g.pad], g.lin[y + g.pad], g.half, ix, iy);
     const Bilin b = bilin(ix, iy);
     const int r = b.r0, c = b.c0 - g.ya_lo;
-    const int2 *wr = g.wrange + (size_t)s * g.Lp;
+    const int2 *wr = w_ranges(g, s, alist[s]);
     const bool r0 = (unsigned)r < (unsigned)g.Lp, r1 = (unsigned)(r + 1) < (unsigned)g.Lp;
     const int2 g0 = r0 ? wr[r] : make_int2(0, 0);
     const int2 g1 = r1 ? wr[r + 1] : make_int2(0, 0);
@@ -839,7 +900,7 @@ __device__ __forceinline__ void b2_make_tap(const SpectDev &g, const int *__rest
     if (r0 && c + 1 >= g0.x && c + 1 < g0.y) m |= 2;
     if (r1 && c >= g1.x && c < g1.y) m |= 4;
     if (r1 && c + 1 >= g1.x && c + 1 < g1.y) m |= 8;
-    t.off = (r * g.nya + c) * g.nz;  // the slab has fewer than 2^31 elements (b2_tab_fits)
+    t.off = (r * g.nya + c) * g.nzs;  // the slab has fewer than 2^31 elements (b2_tab_fits)
     t.mask = m;
     t.pad0 = t.pad1 = 0;
     t.nw = b.nw;
@@ -849,7 +910,7 @@ __device__ __forceinline__ void b2_make_tap(const SpectDev &g, const int *__rest
 }
 
 __device__ __forceinline__ bool b2_tab_fits(const SpectDev &g, int n_rows, int n_slots) {
-    return n_rows * n_slots <= kB2Taps && (long long)g.Lp * g.nya * g.nz < (1LL << 31);
+    return n_rows * n_slots <= kB2Taps && (long long)g.Lp * g.nya * g.nzs < (1LL << 31);
 }
 
 __device__ __forceinline__ float4 b2_tap_sample(const float *__restrict__ Ws, const B2Tap &t,
@@ -930,12 +991,12 @@ __global__ void __launch_bounds__(256)
         }
         __syncthreads();
     }
-    if (4 * q >= nz || y >= N) return;
-    const int z = 4 * q;
+    const int z = z_of_pos(g, q);  // q: quad position in the W rows
+    if (4 * q >= g.nzs || z >= nz || y >= N) return;
     const float4 bp = use_tab ? b2_gather_sum4_tab<kB2Unroll>(
-                                    W, (size_t)g.Lp * g.nya * nz, tab + threadIdx.y * n_slots,
-                                    n_slots, g.nya, nz, z)
-                              : b2_gather_sum4(g, W, alist, n_slots, x, y, z);
+                                    W, (size_t)g.Lp * g.nya * g.nzs, tab + threadIdx.y * n_slots,
+                                    n_slots, g.nya, g.nzs, 4 * q)
+                              : b2_gather_sum4(g, W, alist, n_slots, x, y, 4 * q);
     const size_t i = ((size_t)x * N + y) * nz + z;
     apply_update4<PRIOR>(mode, u, i, x, y, z, N, N, nz, bp, out);
 }
@@ -949,7 +1010,7 @@ __device__ __forceinline__ int batch_entry(const int *block_off, int b) {
 }
 
 int b2_gather_blocks(const SpectDev &g) {
-    return (int)(((long long)g.N * g.N * (g.nz / 4) + 255) / 256);
+    return (int)(((long long)g.N * g.N * (g.nzs / 4) + 255) / 256);
 }
 
 // Batched reference back-projector with its epilogue: a thread per (x, y, z quad) of an
@@ -960,7 +1021,7 @@ __global__ void __launch_bounds__(256) k_b2_gather_batch(const __grid_constant__
     const SpectDev &g = p.g[e];
     const long long q0 = (long long)(blockIdx.x - p.block_off[e]) * 256;
     const long long q = q0 + threadIdx.x;
-    const int N = g.N, nz = g.nz, nq = nz / 4, ns = p.n_slots[e];
+    const int N = g.N, nz = g.nz, nq = g.nzs / 4, ns = p.n_slots[e];
     const long long total = (long long)N * N * nq;
     // rows (x N + y) of the block's voxels
     const long long row0 = q0 / nq;
@@ -974,11 +1035,14 @@ __global__ void __launch_bounds__(256) k_b2_gather_batch(const __grid_constant__
         __syncthreads();
     }
     if (q >= total) return;
-    const int z = 4 * (int)(q % nq), y = (int)((q / nq) % N), x = (int)(q / ((long long)nq * N));
+    const int zw = 4 * (int)(q % nq), z = z_of_pos(g, zw / 4);
+    const int y = (int)((q / nq) % N), x = (int)(q / ((long long)nq * N));
+    if (z >= nz) return;
     const float4 bp =
-        use_tab ? b2_gather_sum4_tab<kB2Unroll>(p.W[e], (size_t)g.Lp * g.nya * nz,
-                                               tab + (int)(q / nq - row0) * ns, ns, g.nya, nz, z)
-                : b2_gather_sum4(g, p.W[e], p.alist[e], ns, x, y, z);
+        use_tab ? b2_gather_sum4_tab<kB2Unroll>(p.W[e], (size_t)g.Lp * g.nya * g.nzs,
+                                               tab + (int)(q / nq - row0) * ns, ns, g.nya, g.nzs,
+                                               zw)
+                : b2_gather_sum4(g, p.W[e], p.alist[e], ns, x, y, zw);
     const size_t i = ((size_t)x * N + y) * nz + z;
     UpdateArgs u{};
     u.f = p.out[e];
@@ -1020,10 +1084,10 @@ __global__ void __launch_bounds__(256)
 cudaError_t launch_b2_gather(const SpectDev &g, const float *W, const int *alist, int n_slots,
                              float *out, int mode, const UpdateArgs &u, cudaStream_t st) {
     dim3 block(32, 8);
-    if (g.nz % 4 == 0) {
+    if (g.zg || g.nz % 4 == 0) {
         // blocks of 256 threads shaped to the z quads of a row: when the quads of a row
         // divide a warp (1, 2, 4, 8 or 16), a warp takes whole rows and no lane idles
-        const int qx = g.nz / 4;
+        const int qx = g.nzs / 4;
         const bool packed = qx < 32 && 32 % qx == 0;
         const dim3 b4(packed ? qx : 32, packed ? 256 / qx : 8);
         dim3 grid((qx + b4.x - 1) / b4.x, (g.N + b4.y - 1) / b4.y, g.N);
@@ -1050,14 +1114,16 @@ __global__ void __launch_bounds__(256)
                  float *__restrict__ out) {
     constexpr int V = VEC ? 4 : 1;
     const int slot = blockIdx.z, xp = blockIdx.y;
-    const int nzv = g.nz / V;
+    const int nzv = g.nzs / V;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.nya * nzv) return;
-    const int r = i / nzv, z = (i % nzv) * V;
+    const int r = i / nzv, zw = (i % nzv) * V;  // position in the W row
+    const int z = z_of_pos(g, zw / 4) + (zw & 3);
+    if (z >= g.nz) return;
     const int yp = g.ya_lo + r;
-    const int2 rg = g.wrange[(size_t)slot * g.Lp + xp];
+    const int2 rg = w_ranges(g, slot, alist[slot])[xp];
     if (r < rg.x || r >= rg.y) return;
-    const float *wp = W + (((size_t)slot * g.Lp + xp) * g.nya + r) * g.nz + z;
+    const float *wp = W + (((size_t)slot * g.Lp + xp) * g.nya + r) * g.nzs + zw;
     float v[V];
     if constexpr (VEC) {
         const float4 t = *reinterpret_cast<const float4 *>(wp);
@@ -1092,7 +1158,7 @@ __global__ void __launch_bounds__(256)
 }
 
 int b2_scatter_blocks(const SpectDev &g, int n_slots) {
-    return n_slots * g.Lp * ((g.nya * (g.nz / 4) + 255) / 256);
+    return n_slots * g.Lp * ((g.nya * (g.nzs / 4) + 255) / 256);
 }
 
 // Batched exact adjoint: the blocks of an entry cover (slot, plane, 256 (row, z quad) of
@@ -1100,17 +1166,18 @@ int b2_scatter_blocks(const SpectDev &g, int n_slots) {
 __global__ void __launch_bounds__(256) k_b2_scatter_batch(const __grid_constant__ B2Batch p) {
     const int e = batch_entry(p.block_off, blockIdx.x);
     const SpectDev &g = p.g[e];
-    const int per_plane = (g.nya * (g.nz / 4) + 255) / 256;
+    const int per_plane = (g.nya * (g.nzs / 4) + 255) / 256;
     const int b = blockIdx.x - p.block_off[e];
     const int slot = b / (per_plane * g.Lp), xp = (b / per_plane) % g.Lp;
     const int i = (b % per_plane) * 256 + threadIdx.x;
-    const int nzv = g.nz / 4;
+    const int nzv = g.nzs / 4;
     if (slot >= p.n_slots[e] || i >= g.nya * nzv) return;
-    const int r = i / nzv, z = (i % nzv) * 4;
-    const int2 rg = g.wrange[(size_t)slot * g.Lp + xp];
+    const int r = i / nzv, zw = (i % nzv) * 4, z = z_of_pos(g, zw / 4);
+    if (z >= g.nz) return;
+    const int2 rg = w_ranges(g, slot, p.alist[e][slot])[xp];
     if (r < rg.x || r >= rg.y) return;
     const float4 t = *reinterpret_cast<const float4 *>(
-        p.W[e] + (((size_t)slot * g.Lp + xp) * g.nya + r) * g.nz + z);
+        p.W[e] + (((size_t)slot * g.Lp + xp) * g.nya + r) * g.nzs + zw);
     if (t.x == 0.f && t.y == 0.f && t.z == 0.f && t.w == 0.f) return;
     float ix, iy;
     rot_coords(g.theta_fwd + 6 * p.alist[e][slot], g.lin[xp], g.lin[g.ya_lo + r], g.half, ix, iy);
@@ -1137,10 +1204,10 @@ cudaError_t launch_b2_scatter_batch(const B2Batch &p, int n_blocks, cudaStream_t
 cudaError_t launch_b2_scatter(const SpectDev &g, const float *W, const int *alist, int n_slots,
                               float *out, cudaStream_t st) {
     if (g.nz % 4 == 0 && ((uintptr_t)out & 15) == 0) {
-        dim3 grid((g.nya * (g.nz / 4) + 255) / 256, g.Lp, n_slots);
+        dim3 grid((g.nya * (g.nzs / 4) + 255) / 256, g.Lp, n_slots);
         k_b2_scatter<true><<<grid, 256, 0, st>>>(g, W, alist, out);
     } else {
-        dim3 grid((g.nya * g.nz + 255) / 256, g.Lp, n_slots);
+        dim3 grid((g.nya * g.nzs + 255) / 256, g.Lp, n_slots);
         k_b2_scatter<false><<<grid, 256, 0, st>>>(g, W, alist, out);
     }
     return cudaGetLastError();

@@ -4,6 +4,5 @@
 namespace gb {
 
 GB_FWD_PSF_INSTANCE(11)
-GB_FWD2_INSTANCE(11)
 
 }  // namespace gb

@@ -4,6 +4,5 @@
 namespace gb {
 
 GB_FWD_PSF_INSTANCE(15)
-GB_FWD2_INSTANCE(15)
 
 }  // namespace gb

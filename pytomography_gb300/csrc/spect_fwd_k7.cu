@@ -4,6 +4,5 @@
 namespace gb {
 
 GB_FWD_PSF_INSTANCE(7)
-GB_FWD2_INSTANCE(7)
 
 }  // namespace gb

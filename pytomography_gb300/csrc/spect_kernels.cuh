@@ -4,9 +4,13 @@
 //   object f      [N][N][nz]   unpadded, z fastest
 //   padded frame  Lp = N + 2*pad rows (x) and cols (y); f_pad[r][c] = f[r-pad][c-pad]
 //   projections   [n_sel][N][nz]
-//   A (attenuation factors, per angle, rotated padded frame)  [n_angles][Lp][nya][nz],
+//   A (attenuation factors, per angle, rotated padded frame)  [n_angles][Lp][nya][nzs],
 //                 rows y in [ya_lo, ya_hi) only (the rows the PSF halo can reach)
-//   W (back-projection stack of one angle group)              [G][Lp][nya][nz]
+//   W (rotated-frame stack of one angle group)                [G][Lp][nya][nzs]
+//   Rows of A and W hold nzs values.  Plain rows: nzs = nz, in z order.  Rows of the strip
+//   kernels (zg > 0): nzs = 16 zg, padded, and the z quads are permuted so that quad k of
+//   the 16-value z group c (quad index 4 c + k) lies at quad position k zg + c: the lanes of
+//   a z pass (one z group each) then read and write whole 128-byte lines per instruction.
 //
 // Rotation convention (kornia, align_corners=True; utils/spatial.py:8-34,
 // transforms/shared/spatial.py:21-53): an output voxel (row xp, col yp) samples
@@ -26,23 +30,35 @@ constexpr float kDelta = 1e-11f;  // pytomography.delta (src/pytomography/__init
 struct SpectDev {
     int *err;               // device error word (bounded waits that gave up), or null
     int2 *wrange;           // [G][Lp] W column range written per (slot, plane), or null
+                            // (strip kernels: wranges)
     int N, nz, pad, Lp;
     int n_angles;
     int ya_lo, ya_hi, nya;  // stored row range of A and W
+    int nzs, zg;            // row length of A and W, 16-value z groups (0: plain rows)
     float half;             // (Lp - 1) / 2
     const float *lin;       // [Lp]
     const float *theta_fwd; // [n_angles][6]
     const float *theta_bwd; // [n_angles][6]
-    const float *A;         // [n_angles][Lp][nya][nz] or null
+    const float *A;         // [n_angles][Lp][nya][nzs] or null
     const float *taps_r;    // [n_groups][Lp][K]
     const float *taps_z;    // [n_groups][Lp][K]
     const int *group;       // [n_angles]
     const signed char *tier;  // [n_groups][Lp] tap tier of each plane, or null (full taps)
+    // strip kernels: (first row, last row, tap ladder entry, 0) of every plane of every angle
+    // for the forward (half a pixel around the object square) and the back projection (1.5
+    // pixels), [n_angles][Lp] each, last < first: no row; the back projection's rows as W
+    // column ranges; and the taps, centred per ladder entry, [n_groups][Lp][2][kStripTaps]
+    const int4 *planes_fwd, *planes_bwd;
+    const int2 *wranges;
+    const float *staps;
     int K;                  // taps per row (odd)
     int att;                // attenuation present
     int att_first;          // forward order: attenuation before PSF ("ap")
     int psf;                // PSF present
     int psf2d;              // PSF blurs z as well
+    // strip kernels (spect_strip.cuh): warps of the back projection's and the forward's
+    // CTAs, 0: not used
+    int strip, strip_fwd;
     unsigned long long *phase;  // diagnostic builds: per-CTA forward phase cycles, or null
     unsigned wait_polls;        // polls of a bounded mbarrier wait before it gives up
     int dbg_skip_first_copy;    // test hook: the forward never issues its first TMA copy
@@ -80,6 +96,18 @@ __device__ __forceinline__ void rot_coords(const float *__restrict__ th, float l
     float gy = __fadd_rn(__fadd_rn(__fmul_rn(th[3], lin_col), __fmul_rn(th[4], lin_row)), th[5]);
     ix = __fmul_rn(__fadd_rn(gx, 1.f), half);
     iy = __fmul_rn(__fadd_rn(gy, 1.f), half);
+}
+
+// W column ranges of the planes of a slot that holds angle ga.
+__device__ __forceinline__ const int2 *w_ranges(const SpectDev &g, int slot, int ga) {
+    return g.strip ? g.wranges + (size_t)ga * g.Lp : g.wrange + (size_t)slot * g.Lp;
+}
+
+// First z of the quad at position pos of a row of A or W.
+__device__ __forceinline__ int z_of_pos(const SpectDev &g, int pos) {
+    if (g.zg == 0) return 4 * pos;
+    const int k = pos / g.zg;
+    return 16 * (pos - k * g.zg) + 4 * k;
 }
 
 struct Bilin {
@@ -241,6 +269,10 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long *bar, u
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
                  "r"(bytes)
                  : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ void mbar_inval(unsigned long long *bar) {

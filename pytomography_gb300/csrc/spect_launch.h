@@ -2,14 +2,14 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "gbtomo.h"
 #include "spect_kernels.cuh"
 
 // PSF tap-count buckets compiled into the library: a plan's taps are zero-padded
 // (centred) to the smallest bucket that holds its widest kernel.
 #define GB_FOR_EACH_K(X) X(7) X(11) X(15) X(21) X(25) X(29) X(37) X(45)
-// the buckets the second forward variant (k_fwd_psf2) is compiled for
-#define GB_FOR_EACH_K2(X) X(7) X(11) X(15) X(21) X(25) X(29)
 
 namespace gb {
 
@@ -36,19 +36,29 @@ cudaError_t setup_b1(int K, size_t smem);
 
 // Work items (int4: slot, first plane, end plane, unused) split each angle's planes
 // into ranges of about equal work; partial sums are indexed by item.
-// variant 1: k_fwd_psf (tpb 512 or 768); variant 2: k_fwd_psf2 (cp.async ring, z blur first;
-// attenuation before a 2-D PSF, N <= 128, nz <= 128, nz % 4 == 0, at most 29 taps)
+// tpb: 512 or 768.  Plans of the strip kernels do not come here.
 cudaError_t launch_fwd(const SpectDev &g, const float *f, const int *alist, const int4 *items,
-                       int n_items, int Zt, int tpb, int variant, float *partials,
-                       cudaStream_t st);
-bool fwd2_eligible(const SpectDev &g, size_t smem_cap);
-cudaError_t setup_fwd2(int K);
+                       int n_items, int Zt, int tpb, float *partials, cudaStream_t st);
 // ioff[slot] .. ioff[slot+1]: the items of a slot
 cudaError_t launch_reduce(int n_slots, const int *ioff, int NZ, const float *partials, float *out,
                           int ratio, const float *gproj, const float *sadd, const int *alist,
                           float *pred, cudaStream_t st);
 cudaError_t launch_b1(const SpectDev &g, const float *proj, const int *alist, int n_slots,
                       const int4 *items, int n_items, int Zt, float *W, cudaStream_t st);
+// Strip kernels (spect_strip.cu).  strip_configure sets strip, strip_fwd, zg and nzs of a PSF
+// plan whose attenuation, if any, comes before the PSF, with N and nz <= 128 and tiles that
+// fit `cap` bytes of shared memory; it leaves every other plan alone.
+void strip_configure(SpectDev &g, size_t cap);
+cudaError_t setup_strip(size_t cap);
+// Values of one slot (angle) of the W stack: rows of the back projection, or of the forward.
+inline size_t stack_slot(const SpectDev &g) {
+    return (size_t)g.Lp * g.nya * (g.strip ? std::max(g.nzs, 32 * ((g.zg + 1) / 2)) : g.nzs);
+}
+cudaError_t launch_fwd_strip(const SpectDev &g, const float *f, const int *alist,
+                             const int4 *items, int n_items, const int4 *yitems, int n_yitems,
+                             float *W, float *partials, cudaStream_t st);
+cudaError_t launch_b1_strip(const SpectDev &g, const float *proj, const int *alist,
+                            const int4 *items, int n_items, float *W, cudaStream_t st);
 cudaError_t launch_b2_gather(const SpectDev &g, const float *W, const int *alist, int n_slots,
                              float *out, int mode, const UpdateArgs &u, cudaStream_t st);
 cudaError_t launch_b2_scatter(const SpectDev &g, const float *W, const int *alist, int n_slots,
@@ -70,12 +80,15 @@ constexpr int kMaxBatch = 32;
 struct FwdBatch {
     CUtensorMap tm[kMaxBatch];  // attenuation boxes of each entry (64-byte aligned)
     SpectDev g[kMaxBatch];
+    float *W[kMaxBatch];            // strip entries: the rows between the two kernels
     const float *f[kMaxBatch];      // object of each entry
-    const int *alist[kMaxBatch];    // angle list of the launch's subset, per entry
+    const int *alist[kMaxBatch];    // the group's angles, per entry
     const int4 *items;              // (slot, first plane, end plane, entry), largest first
     int n_items;
+    const int4 *yitems;             // strip entries: items of the second kernel
+    int n_yitems;
     int *counter;                   // work-queue position, zeroed before the launch
-    float *partials;                // [n_items][nz_max]
+    float *partials;                // [n_items (strip entries: n_yitems)][nz_max]
     int nz_max;
 };
 
@@ -124,6 +137,9 @@ GB_FOR_EACH_K(GB_DECL_FWD_BATCH)
 // when the kernel makes none); s_cols is the kernel's S row length.
 cudaError_t make_att_tmap(const SpectDev &g, int s_cols, CUtensorMap *out);
 cudaError_t setup_b1_batch(int K);
+// n entries, of which those with g.strip > 0 have items
+cudaError_t launch_fwd_strip_batch(const FwdBatch &p, int n, int grid, cudaStream_t st);
+cudaError_t launch_b1_strip_batch(const B1Batch &p, int n, int grid, cudaStream_t st);
 cudaError_t launch_b1_batch(int K, const B1Batch &p, int grid, cudaStream_t st);
 cudaError_t launch_reduce_batch(const ReduceBatch &p, int n_rows, cudaStream_t st);
 cudaError_t launch_b2_gather_batch(const B2Batch &p, int n_blocks, cudaStream_t st);
@@ -132,19 +148,12 @@ cudaError_t launch_b2_scatter_batch(const B2Batch &p, int n_blocks, cudaStream_t
 int b2_gather_blocks(const SpectDev &g);
 int b2_scatter_blocks(const SpectDev &g, int n_slots);
 
-// Launch geometry of one forward projection of a plan (for entry points defined outside
-// spect_plan.cu): false when the subset is out of range.
-struct FwdArgs {
-    SpectDev g;
-    const int *alist;
-    int n_sel;
-    const int4 *items;
-    int n_items;
-    const int *ioff;
-    int Zt;
-    int tpb;
-    int variant;
-};
-bool plan_forward_args(const gb_spect_plan *p, int subset, FwdArgs *a);
+// One forward projection of a plan with the caller's partial-sum buffer (for entry points
+// defined outside spect_plan.cu): the work items and partial floats a subset needs (false when
+// the subset is out of range), and the projection itself.
+bool plan_forward_need(const gb_spect_plan *p, int subset, int *n_sel, int *n_items,
+                       size_t *floats);
+gb_status plan_forward(gb_spect_plan *p, const float *obj, int subset, float *out,
+                       float *partials, cudaStream_t st);
 
 }  // namespace gb

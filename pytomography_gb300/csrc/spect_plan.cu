@@ -12,6 +12,7 @@
 #include "common.cuh"
 #include "spect_blur.cuh"
 #include "spect_launch.h"
+#include "spect_strip.cuh"
 
 namespace gb {
 
@@ -162,8 +163,15 @@ struct gb_spect_plan {
     float *d_lin = nullptr, *d_theta_fwd = nullptr, *d_theta_bwd = nullptr;
     float *d_taps_r = nullptr, *d_taps_z = nullptr, *d_A = nullptr;
     signed char *d_tier = nullptr;
+    int4 *d_planes = nullptr;  // strip kernels: plane tables, forward then back projection
+    int2 *d_wranges = nullptr;
+    float *d_staps = nullptr;
     int *d_group = nullptr;
     std::vector<signed char> h_tier;  // tap tier per (PSF group, plane)
+    std::vector<signed char> h_ladder;  // tap ladder entry per (PSF group, plane)
+    // rows (first, last) of every (angle, plane) within half a pixel (forward) and 1.5 pixels
+    // (back projection) of the object square; last < first: none
+    std::vector<int2> h_rows_fwd, h_rows_bwd;
     std::vector<int> h_group;         // PSF group per angle
     // angle lists: [all][subset 0][subset 1]..., with their work items
     int *d_alist = nullptr;
@@ -171,12 +179,22 @@ struct gb_spect_plan {
     int *d_ioff = nullptr;
     int n_subsets = 0;
     std::vector<std::vector<int>> explicit_subsets;  // caller's subset lists, if set
+    // Forward items of one angle group (slots a0 .. a0 + n of the list, numbered from 0):
+    // every angle of the list, or G at a time for the strip kernels, whose rows between the
+    // two kernels lie in the W stack.
+    struct FwdGroup {
+        int a0 = 0, n = 0;
+        int item_off = 0, n_items = 0;  // items in d_items, one block of partial sums each
+        int ioff_off = 0;               // n + 1 item offsets per slot in d_ioff
+        int gather_off = 0, n_gather = 0;  // strip kernels: items of the first kernel
+        int half = 0, gather_half = 0;     // first items of slot n / 2
+    };
     struct List {
         int alist_off = 0, n = 0;
-        int fitem_off = 0, n_fitems = 0;  // forward items in d_items
-        int ioff_off = 0;                 // n + 1 item offsets per slot in d_ioff
+        std::vector<FwdGroup> fgroups;
+        int max_fitems = 0;  // largest group's items
         std::vector<int> gitem_off, n_gitems;  // B1 items of each angle group
-        int f_half = 0, b_half = 0;  // first forward / group-0 B1 item of slot n / 2
+        int b_half = 0;  // first group-0 B1 item of slot n / 2
     };
     std::vector<List> lists;
     std::vector<float> h_theta_fwd, h_lin;
@@ -190,7 +208,7 @@ struct gb_spect_plan {
     int *d_err = nullptr;
     int Zt_fwd = 0, Zt_b1 = 0;
     int fwd_tpb = 512;  // forward CTA size: 512 or 768 threads (one CTA per SM)
-    int fwd_variant = 1;  // 1: k_fwd_psf; 2: k_fwd_psf2
+    int fwd_variant = 1;  // kept for gb_spect_tuning: one forward kernel serves both values
     int fwd_items = 1, b1_items = 1;  // work items per resident CTA slot and z slab
     unsigned lists_version = 0;       // bumped whenever the subset / work lists change
     // fused OSEM step in two angle halves on two streams (the second half's forward and
@@ -205,6 +223,9 @@ static void free_plan(gb_spect_plan *p) {
     dev_free(p->d_lin); dev_free(p->d_theta_fwd); dev_free(p->d_theta_bwd);
     dev_free(p->d_taps_r); dev_free(p->d_taps_z); dev_free(p->d_A); dev_free(p->d_group);
     dev_free(p->d_tier);
+    dev_free(p->d_planes);
+    dev_free(p->d_wranges);
+    dev_free(p->d_staps);
     dev_free(p->dev.phase);
     dev_free(p->d_alist); dev_free(p->d_items); dev_free(p->d_ioff);
     dev_free(p->d_partials); dev_free(p->d_W); dev_free(p->d_ratio);
@@ -218,7 +239,8 @@ static void free_plan(gb_spect_plan *p) {
 }
 
 // Rows of plane xp whose rotated sample can reach the object square (host, double
-// precision; only used to estimate work, the kernels decide exactly).
+// precision, one row of slack on each side).  They bound the rows of the strip kernels; the
+// other kernels decide for themselves, and these only estimate their work.
 static bool host_plane_rows(const gb_spect_plan *p, int a, int xp, int ylo, int yhi,
                             double margin, int &ra, int &rb) {
     const float *th = p->h_theta_fwd.data() + 6 * a;
@@ -263,22 +285,33 @@ static bool host_plane_rows(const gb_spect_plan *p, int a, int xp, int ylo, int 
 // the launch from 0.1622 to 0.1641 ms and was not kept.)
 // (The forward skips empty planes with a support test; B1 also records their empty row
 // range.)
-static std::vector<double> plane_work(const gb_spect_plan *p, int a, bool fwd) {
-    std::vector<double> w(p->Lp, fwd ? 100.0 : 835.0);
+constexpr double kStripEmpty = 20.0;  // cost of a plane no sample reaches in the strip kernels
+static int strip_plane_cap(const gb_spect_plan *p) { return p->dev.strip ? kStripPlanes : 0; }
+enum WorkKind { WORK_FWD, WORK_B1, WORK_GATHER };
+static std::vector<double> plane_work(const gb_spect_plan *p, int a, WorkKind kind) {
+    const bool fwd = kind != WORK_B1;
+    std::vector<double> w(p->Lp, p->dev.strip ? kStripEmpty : fwd ? 100.0 : 835.0);
     const int H = p->H, K = p->dev.K;
-    const int ylo = std::max(0, p->pad - H), yhi = std::min(p->Lp, p->pad + p->N + H);
     const int grp = p->h_group.empty() ? 0 : p->h_group[a];
     for (int xp = 0; xp < p->Lp; xp++) {
-        int ra, rb;
-        if (!host_plane_rows(p, a, xp, ylo, yhi, fwd ? 0.5 : 1.5, ra, rb)) continue;
+        const int2 rows = (fwd ? p->h_rows_fwd : p->h_rows_bwd)[(size_t)a * p->Lp + xp];
+        const int ra = rows.x, rb = rows.y;
+        if (rb < ra) continue;
         const int tier = p->h_tier.empty() ? kTiers - 1 : p->h_tier[(size_t)grp * p->Lp + xp];
         const double kk = tier_taps(K, tier);
-        const double rows = rb - ra + 1;
-        if (fwd) {
+        const double nr = rb - ra + 1;
+        if (p->dev.strip) {
+            const int RS = 8 * (32 / strip_ql(p->nz));
+            const int taps = 2 * ladder_half(p->h_ladder[(size_t)grp * p->Lp + xp]) + 1;
+            const int strips = (rb - ra + RS) / RS;
+            w[xp] = kind == WORK_GATHER ? strips * (420.0 + 4.5 * taps)
+                    : kind == WORK_B1   ? strips * (142.0 + 15.0 * taps)
+                                        : 2400.0 + 46.0 * taps + 0.49 * taps * nr;
+        } else if (fwd) {
             const int o = std::min(p->N, rb + H - p->pad + 1) - std::max(0, ra - H - p->pad);
-            w[xp] = 6360.0 + 106.0 * rows + 2.76 * kk * std::max(0, o);
+            w[xp] = 6360.0 + 106.0 * nr + 2.76 * kk * std::max(0, o);
         } else {
-            w[xp] = 5370.0 + 67.0 * rows + 2.37 * kk * rows;
+            w[xp] = 5370.0 + 67.0 * nr + 2.37 * kk * nr;
         }
     }
     return w;
@@ -286,8 +319,10 @@ static std::vector<double> plane_work(const gb_spect_plan *p, int a, bool fwd) {
 
 // Split [0, Lp) into c contiguous plane ranges of about equal work: each boundary is put
 // where the running sum comes closest to its share.
+// With `cap` (the strip kernels) the ranges leave out the planes without work (w <= empty) at
+// their ends and hold at most `cap` planes.
 static void split_planes(const std::vector<double> &w, int c, int slot,
-                         std::vector<int4> &out) {
+                         std::vector<int4> &out, int cap = 0, double empty = 0) {
     const int L = (int)w.size();
     double total = 0;
     for (double v : w) total += v;
@@ -302,7 +337,13 @@ static void split_planes(const std::vector<double> &w, int c, int slot,
             end = std::max(x, prev + 1);
             while (x < end) acc += w[x++];
         }
-        out.push_back(make_int4(slot, prev, end, 0));
+        int from = prev, to = end;
+        if (cap) {
+            while (from < to && w[from] <= empty) from++;
+            while (to > from && w[to - 1] <= empty) to--;
+            for (; to - from > cap; from += cap) out.push_back(make_int4(slot, from, from + cap, 0));
+        }
+        out.push_back(make_int4(slot, from, to, 0));
         prev = end;
     }
 }
@@ -371,13 +412,14 @@ static gb_status upload_lists(gb_spect_plan *p, int n_subsets) {
         }
     }
     const bool psf = p->dev.psf;
-    const int zs_f = psf ? (p->nz + p->Zt_fwd - 1) / p->Zt_fwd : 1;
-    const int zs_b = psf ? (p->nz + p->Zt_b1 - 1) / p->Zt_b1 : 1;
-    std::vector<std::vector<double>> wf(p->n_angles), wb(p->n_angles);
+    const int zs_f = psf && !p->dev.strip ? (p->nz + p->Zt_fwd - 1) / p->Zt_fwd : 1;
+    const int zs_b = psf && !p->dev.strip ? (p->nz + p->Zt_b1 - 1) / p->Zt_b1 : 1;
+    std::vector<std::vector<double>> wf(p->n_angles), wb(p->n_angles), wg(p->n_angles);
     if (psf)
         for (int a = 0; a < p->n_angles; a++) {
-            wf[a] = plane_work(p, a, true);
-            wb[a] = plane_work(p, a, false);
+            wf[a] = plane_work(p, a, WORK_FWD);
+            wb[a] = plane_work(p, a, WORK_B1);
+            if (p->dev.strip) wg[a] = plane_work(p, a, WORK_GATHER);
         }
     size_t max_items = 0;
     for (const auto &l : angle_lists) {
@@ -386,28 +428,46 @@ static gb_status upload_lists(gb_spect_plan *p, int n_subsets) {
         L.n = (int)l.size();
         all.insert(all.end(), l.begin(), l.end());
         // forward items
-        L.fitem_off = (int)items.size();
-        L.ioff_off = (int)ioff.size();
-        if (psf) {
-            std::vector<double> wa(L.n);
-            for (int i = 0; i < L.n; i++) wa[i] = sum_of(wf[l[i]]);
-            std::vector<int> cnt = chunk_counts(p, wa, zs_f, p->fwd_items);
-            for (int i = 0; i < L.n; i++) {
-                ioff.push_back((int)items.size() - L.fitem_off);
-                if (i == L.n / 2) L.f_half = (int)items.size() - L.fitem_off;
-                split_planes(wf[l[i]], cnt[i], i, items);
+        const int gf = p->dev.strip ? p->G : L.n;
+        for (int a0 = 0; a0 < L.n; a0 += gf) {
+            gb_spect_plan::FwdGroup F;
+            F.a0 = a0;
+            F.n = std::min(gf, L.n - a0);
+            F.item_off = (int)items.size();
+            F.ioff_off = (int)ioff.size();
+            std::vector<int> cnt(F.n, psf ? 0 : nopsf_chunks(p, L.n));
+            if (psf) {
+                std::vector<double> wa(F.n);
+                for (int i = 0; i < F.n; i++) wa[i] = sum_of(wf[l[a0 + i]]);
+                cnt = chunk_counts(p, wa, zs_f, p->fwd_items);
             }
-        } else {
-            int c = nopsf_chunks(p, L.n);
-            for (int i = 0; i < L.n; i++) {
-                ioff.push_back((int)items.size() - L.fitem_off);
-                for (int k = 0; k < c; k++)
-                    items.push_back(make_int4(i, k * p->Lp / c, (k + 1) * p->Lp / c, 0));
+            for (int i = 0; i < F.n; i++) {
+                ioff.push_back((int)items.size() - F.item_off);
+                if (i == F.n / 2) F.half = (int)items.size() - F.item_off;
+                if (psf)
+                    split_planes(wf[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p), kStripEmpty);
+                else
+                    for (int k = 0; k < cnt[i]; k++)
+                        items.push_back(
+                            make_int4(i, k * p->Lp / cnt[i], (k + 1) * p->Lp / cnt[i], 0));
             }
+            F.n_items = (int)items.size() - F.item_off;
+            ioff.push_back(F.n_items);
+            L.max_fitems = std::max(L.max_fitems, F.n_items);
+            if (p->dev.strip) {
+                F.gather_off = (int)items.size();
+                std::vector<double> wa(F.n);
+                for (int i = 0; i < F.n; i++) wa[i] = sum_of(wg[l[a0 + i]]);
+                cnt = chunk_counts(p, wa, 1);
+                for (int i = 0; i < F.n; i++) {
+                    if (i == F.n / 2) F.gather_half = (int)items.size() - F.gather_off;
+                    split_planes(wg[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p), kStripEmpty);
+                }
+                F.n_gather = (int)items.size() - F.gather_off;
+            }
+            L.fgroups.push_back(F);
         }
-        L.n_fitems = (int)items.size() - L.fitem_off;
-        ioff.push_back(L.n_fitems);
-        max_items = std::max(max_items, (size_t)L.n_fitems);
+        max_items = std::max(max_items, (size_t)L.max_fitems);
         // B1 items per angle group
         for (int a0 = 0; a0 < L.n; a0 += p->G) {
             int na = std::min(p->G, L.n - a0);
@@ -418,7 +478,7 @@ static gb_status upload_lists(gb_spect_plan *p, int n_subsets) {
                 std::vector<int> cnt = chunk_counts(p, wa, zs_b, p->b1_items);
                 for (int i = 0; i < na; i++) {
                     if (a0 == 0 && i == L.n / 2) L.b_half = (int)items.size() - L.gitem_off.back();
-                    split_planes(wb[l[a0 + i]], cnt[i], i, items);
+                    split_planes(wb[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p), kStripEmpty);
                 }
             }
             L.n_gitems.push_back((int)items.size() - L.gitem_off.back());
@@ -583,6 +643,8 @@ gb_status gb_spect_plan_create(const gb_spect_desc *d, gb_spect_plan **out) {
     g.psf2d = psf ? (d->psf_2d ? 1 : 0) : 0;
     g.wait_polls = kWaitPolls;
     g.dbg_skip_first_copy = 0;
+    g.nzs = p->nz;
+    strip_configure(g, max_smem_optin());
 
 #define FAIL_CUDA(call)                                                                   \
     do {                                                                                  \
@@ -629,7 +691,10 @@ gb_status gb_spect_plan_create(const gb_spect_desc *d, gb_spect_plan **out) {
                 }
             }
         // tap tier of every plane: the narrowest unrolled loop that holds its nonzero taps
+        if (!d->psf_2d)  // the strip kernels' z pass copies the plane then
+            for (size_t r = 0; r < (size_t)ng * Lp; r++) tz[r * K + K / 2] = 1.f;
         std::vector<signed char> tier((size_t)ng * Lp, kTiers - 1);
+        std::vector<signed char> ladder((size_t)ng * Lp, 0);
         const int Hk = K / 2;
         for (int gi = 0; gi < ng; gi++)
             for (int x = 0; x < Lp; x++) {
@@ -642,14 +707,32 @@ gb_status gb_spect_plan_create(const gb_spect_desc *d, gb_spect_plan **out) {
                 int t = 0;
                 while (t < kTiers - 1 && h > tier_half(K, t)) t++;
                 tier[(size_t)gi * Lp + x] = (signed char)t;
+                ladder[(size_t)gi * Lp + x] = (signed char)ladder_index(h);
             }
         p->h_tier = tier;
+        p->h_ladder = ladder;
         FAIL_CUDA(dev_alloc(&p->d_tier, tier.size()));
         FAIL_CUDA(cudaMemcpy(p->d_tier, tier.data(), tier.size(), cudaMemcpyHostToDevice));
         FAIL_CUDA(dev_alloc(&p->d_taps_r, tr.size() * sizeof(float)));
         FAIL_CUDA(cudaMemcpy(p->d_taps_r, tr.data(), tr.size() * sizeof(float), cudaMemcpyHostToDevice));
         FAIL_CUDA(dev_alloc(&p->d_taps_z, tz.size() * sizeof(float)));
         FAIL_CUDA(cudaMemcpy(p->d_taps_z, tz.data(), tz.size() * sizeof(float), cudaMemcpyHostToDevice));
+        if (g.strip) {
+            std::vector<float> st((size_t)ng * Lp * 2 * kStripTaps, 0.f);
+            for (size_t r = 0; r < (size_t)ng * Lp; r++) {
+                const int half = ladder_half(ladder[r]);
+                for (int t = 0; t < 2 * half + 1; t++) {
+                    const int at = t - half + Hk;  // tap index of the plan's table
+                    if (at < 0 || at >= K) continue;
+                    st[(2 * r) * kStripTaps + t] = tr[r * K + at];
+                    st[(2 * r + 1) * kStripTaps + t] = tz[r * K + at];
+                }
+            }
+            FAIL_CUDA(dev_alloc(&p->d_staps, st.size() * sizeof(float)));
+            FAIL_CUDA(cudaMemcpy(p->d_staps, st.data(), st.size() * sizeof(float),
+                                 cudaMemcpyHostToDevice));
+            g.staps = p->d_staps;
+        }
         p->Zt_fwd = choose_zt(K, p->N, p->nz, true);
         p->Zt_b1 = choose_zt(K, p->N, p->nz, false);
         if (!p->Zt_fwd || !p->Zt_b1) {
@@ -672,8 +755,9 @@ gb_status gb_spect_plan_create(const gb_spect_desc *d, gb_spect_plan **out) {
     g.taps_r = p->d_taps_r;
     g.taps_z = p->d_taps_z;
     g.tier = p->d_tier;
+    if (g.strip) FAIL_CUDA(setup_strip(max_smem_optin()));
     if (att) {
-        size_t na = (size_t)n * Lp * g.nya * p->nz;
+        size_t na = (size_t)n * Lp * g.nya * g.nzs;
         FAIL_CUDA(dev_alloc(&p->d_A, na * sizeof(float)));
         g.A = p->d_A;
         FAIL_CUDA(launch_atten(g, d->mu, d->dx, n, p->d_A, 0));
@@ -681,7 +765,7 @@ gb_status gb_spect_plan_create(const gb_spect_desc *d, gb_spect_plan **out) {
     }
     // scratch: W for one angle group, likelihood ratio of all angles, multi-group bp
     p->G = std::min(n, 16);
-    FAIL_CUDA(dev_alloc(&p->d_W, (size_t)p->G * Lp * g.nya * p->nz * sizeof(float)));
+    FAIL_CUDA(dev_alloc(&p->d_W, p->G * stack_slot(g) * sizeof(float)));
     FAIL_CUDA(dev_alloc(&p->d_ratio, (size_t)n * p->N * p->nz * sizeof(float)));
     FAIL_CUDA(dev_alloc(&p->d_bp, (size_t)p->N * p->N * p->nz * sizeof(float)));
     FAIL_CUDA(dev_alloc(&p->d_wrange, (size_t)p->G * Lp * sizeof(int2)));
@@ -693,6 +777,39 @@ gb_status gb_spect_plan_create(const gb_spect_desc *d, gb_spect_plan **out) {
     FAIL_CUDA(cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming));
     g.wrange = p->d_wrange;
     g.err = p->d_err;
+    if (psf) {
+        p->h_rows_fwd.assign((size_t)n * Lp, make_int2(0, -1));
+        p->h_rows_bwd = p->h_rows_fwd;
+        for (int a = 0; a < n; a++)
+            for (int x = 0; x < Lp; x++)
+                for (int m = 0; m < 2; m++) {
+                    int2 &r = (m ? p->h_rows_bwd : p->h_rows_fwd)[(size_t)a * Lp + x];
+                    int ra, rb;
+                    if (host_plane_rows(p, a, x, g.ya_lo, g.ya_hi, m ? 1.5 : 0.5, ra, rb))
+                        r = make_int2(ra, rb);
+                }
+    }
+    if (g.strip) {
+        const size_t np = (size_t)n * Lp;
+        std::vector<int4> planes(2 * np);
+        std::vector<int2> wr(np);
+        for (size_t i = 0; i < np; i++) {
+            const int lad = p->h_ladder[(size_t)grp[i / Lp] * Lp + i % Lp];
+            const int2 f = p->h_rows_fwd[i], b = p->h_rows_bwd[i];
+            planes[i] = make_int4(f.x, f.y, lad, 0);
+            planes[np + i] = make_int4(b.x, b.y, lad, 0);
+            wr[i] = b.y >= b.x ? make_int2(b.x - g.ya_lo, b.y + 1 - g.ya_lo) : make_int2(0, 0);
+        }
+        FAIL_CUDA(dev_alloc(&p->d_planes, planes.size() * sizeof(int4)));
+        FAIL_CUDA(cudaMemcpy(p->d_planes, planes.data(), planes.size() * sizeof(int4),
+                             cudaMemcpyHostToDevice));
+        FAIL_CUDA(dev_alloc(&p->d_wranges, wr.size() * sizeof(int2)));
+        FAIL_CUDA(cudaMemcpy(p->d_wranges, wr.data(), wr.size() * sizeof(int2),
+                             cudaMemcpyHostToDevice));
+        g.planes_fwd = p->d_planes;
+        g.planes_bwd = p->d_planes + np;
+        g.wranges = p->d_wranges;
+    }
 #undef FAIL_CUDA
     gb_status st = upload_lists(p, 1);
     if (st != GB_OK) {
@@ -786,6 +903,13 @@ gb_status gb_spect_get_tuning(const gb_spect_plan *p, gb_spect_tuning *out) {
     return GB_OK;
 }
 
+// Plans that take fwd_variant 2: attenuation before a 2-D PSF of at most 29 taps, N and nz <=
+// 128, nz % 4 == 0.  (All of them run the strip kernels, whose z pass comes first.)
+static bool variant2_eligible(const SpectDev &g) {
+    return g.psf && g.psf2d && g.att && g.att_first && g.A && g.K <= 29 && g.N <= 128 &&
+           g.nz <= 128 && g.nz % 4 == 0;
+}
+
 // Check a tuning against the plan's limits and fill in the z slabs left at 0.
 static gb_status resolve_tuning(const gb_spect_plan *p, gb_spect_tuning &t) {
     const int K = p->dev.K, OB = (K <= 31) ? 8 : 4;
@@ -793,7 +917,7 @@ static gb_status resolve_tuning(const gb_spect_plan *p, gb_spect_tuning &t) {
     if (t.fwd_variant == 0) t.fwd_variant = p->fwd_variant;
     GB_CHECK_ARG(t.fwd_variant == 1 || t.fwd_variant == 2, "fwd_variant must be 1 or 2");
     GB_CHECK_ARG(t.osem_split == 0 || t.osem_split == 1, "osem_split must be 0 or 1");
-    if (t.fwd_variant == 2 && !fwd2_eligible(p->dev, max_smem_optin())) {
+    if (t.fwd_variant == 2 && !variant2_eligible(p->dev)) {
         set_error("forward variant 2 needs attenuation before a 2-D PSF of at most 29 taps, "
                   "N and nz <= 128 and nz %% 4 == 0");
         return GB_ERR_UNSUPPORTED;
@@ -826,7 +950,6 @@ gb_status gb_spect_set_tuning(gb_spect_plan *p, const gb_spect_tuning *tuning) {
     const int K = p->dev.K;
     GB_CUDA(setup_fwd(K, max_smem_optin(), t.fwd_tpb));
     GB_CUDA(setup_b1(K, max_smem_optin()));
-    if (t.fwd_variant == 2) GB_CUDA(setup_fwd2(K));
     p->fwd_tpb = t.fwd_tpb;
     p->fwd_variant = t.fwd_variant;
     p->osem_split = t.osem_split;
@@ -837,20 +960,38 @@ gb_status gb_spect_set_tuning(gb_spect_plan *p, const gb_spect_tuning *tuning) {
     return upload_lists(p, std::max(1, p->n_subsets));
 }
 
+// A forward group's angles of one half (0: slots before n / 2, 1: the others) or all of them
+// (-1); partials: of the whole group.
+static cudaError_t launch_fwd_group(gb_spect_plan *p, const gb_spect_plan::FwdGroup &F, int half,
+                                    const float *obj, const int *alist, float *partials,
+                                    cudaStream_t st) {
+    const int i0 = half == 1 ? F.half : 0, i1 = half == 0 ? F.half : F.n_items;
+    const int4 *items = p->d_items + F.item_off + i0;
+    partials += (size_t)i0 * p->N * p->nz;
+    if (p->dev.strip) {
+        const int g0 = half == 1 ? F.gather_half : 0, g1 = half == 0 ? F.gather_half : F.n_gather;
+        return launch_fwd_strip(p->dev, obj, alist, p->d_items + F.gather_off + g0, g1 - g0, items,
+                                i1 - i0, p->d_W, partials, st);
+    }
+    return launch_fwd(p->dev, obj, alist, items, i1 - i0, p->Zt_fwd, p->fwd_tpb, partials, st);
+}
+
 static gb_status run_forward(gb_spect_plan *p, const float *obj, int subset, float *out,
                              int ratio, const float *gproj, const float *sadd, float *pred,
-                             cudaStream_t st) {
+                             float *partials, cudaStream_t st) {
     const int li = list_index(p, subset);
     if (li < 0) {
         set_error("subset %d out of range (n_subsets=%d)", subset, p->n_subsets);
         return GB_ERR_STATE;
     }
     const gb_spect_plan::List &L = p->lists[li];
-    const int *alist = p->d_alist + L.alist_off;
-    GB_CUDA(launch_fwd(p->dev, obj, alist, p->d_items + L.fitem_off, L.n_fitems, p->Zt_fwd,
-                       p->fwd_tpb, p->fwd_variant, p->d_partials, st));
-    GB_CUDA(launch_reduce(L.n, p->d_ioff + L.ioff_off, p->N * p->nz, p->d_partials, out, ratio,
-                          gproj, sadd, alist, pred, st));
+    const size_t NZ = (size_t)p->N * p->nz;
+    for (const gb_spect_plan::FwdGroup &F : L.fgroups) {
+        const int *alist = p->d_alist + L.alist_off + F.a0;
+        GB_CUDA(launch_fwd_group(p, F, -1, obj, alist, partials, st));
+        GB_CUDA(launch_reduce(F.n, p->d_ioff + F.ioff_off, (int)NZ, partials, out + F.a0 * NZ,
+                              ratio, gproj, sadd, alist, pred ? pred + F.a0 * NZ : nullptr, st));
+    }
     return GB_OK;
 }
 
@@ -860,7 +1001,8 @@ gb_status gb_spect_forward(gb_spect_plan *p, const float *obj, float *proj, int3
     GB_INJECT_ARG();
     GB_CHECK_ARG(p && obj && proj, "null argument");
     GB_INJECT_LAUNCH();
-    return run_forward(p, obj, subset, proj, 0, nullptr, nullptr, nullptr, as_stream(stream));
+    return run_forward(p, obj, subset, proj, 0, nullptr, nullptr, nullptr, p->d_partials,
+                       as_stream(stream));
 }
 
 // Back-project `proj` (rows = the angles of list li) in groups of G angles.
@@ -972,17 +1114,18 @@ gb_status gb_spect_autotune(gb_spect_plan *p, int32_t subset, int32_t reps,
         return ms / reps;
     };
     auto fwd_call = [&]() {
-        return run_forward(p, obj, subset, proj, 0, nullptr, nullptr, nullptr, st);
+        return run_forward(p, obj, subset, proj, 0, nullptr, nullptr, nullptr, p->d_partials, st);
     };
     auto bwd_call = [&]() { return run_backward(p, proj, li, 0, back, B2_WRITE, UpdateArgs{}, st); };
     // forward candidates
     float best_ms = 1e30f;
     gb_spect_tuning fbest = best;
+    const bool strip = p->dev.strip > 0;  // only the work items matter to the strip kernels
     for (int tpb : {512, 768}) {
         const int zmax = choose_zt(K, p->N, p->nz, true, tpb);
-        if (!zmax) continue;
+        if (!zmax || (strip && tpb != 512)) continue;
         for (int zt : {zmax, (zmax / 2) / OB * OB}) {
-            if (zt < 2 * OB || (zt != zmax && zt >= p->nz)) continue;
+            if (zt < 2 * OB || (zt != zmax && (zt >= p->nz || strip))) continue;
             for (int items : {1, 2}) {
                 gb_spect_tuning t = best;
                 t.fwd_variant = 1;
@@ -998,19 +1141,6 @@ gb_status gb_spect_autotune(gb_spect_plan *p, int32_t subset, int32_t reps,
             }
         }
     }
-    if (fwd2_eligible(p->dev, max_smem_optin()))
-        for (int items : {1, 2}) {
-            gb_spect_tuning t = best;
-            t.fwd_variant = 2;
-            t.fwd_tpb = 512;
-            t.fwd_items = items;
-            if (gb_spect_set_tuning(p, &t) != GB_OK) continue;
-            const float ms = time_ms(fwd_call);
-            if (ms >= 0.f && ms < best_ms) {
-                best_ms = ms;
-                fbest = t;
-            }
-        }
     best.fwd_tpb = fbest.fwd_tpb;
     best.fwd_zt = fbest.fwd_zt;
     best.fwd_items = fbest.fwd_items;
@@ -1020,7 +1150,7 @@ gb_status gb_spect_autotune(gb_spect_plan *p, int32_t subset, int32_t reps,
     gb_spect_tuning bbest = best;
     const int zbmax = choose_zt(K, p->N, p->nz, false);
     for (int zt : {zbmax, (zbmax / 2) / OB * OB}) {
-        if (zt < 2 * OB || (zt != zbmax && zt >= p->nz)) continue;
+        if (zt < 2 * OB || (zt != zbmax && (zt >= p->nz || strip))) continue;
         for (int items : {1, 2}) {
             gb_spect_tuning t = best;
             t.b1_zt = zt;
@@ -1059,16 +1189,14 @@ static gb_status osem_split_step(gb_spect_plan *p, const gb_spect_plan::List &L,
     const int *alist = p->d_alist + L.alist_off;
     const int h = L.n / 2;
     const size_t NZ = (size_t)p->N * p->nz;
-    const int4 *fit = p->d_items + L.fitem_off;
-    const int *ioff = p->d_ioff + L.ioff_off;
+    const gb_spect_plan::FwdGroup &F = L.fgroups[0];  // the list is one group (n <= G)
+    const int *ioff = p->d_ioff + F.ioff_off;
     const int4 *bit = p->d_items + L.gitem_off[0];
     cudaStream_t s2 = p->st2;
     GB_CUDA(cudaEventRecord(p->ev_fork, st));
     GB_CUDA(cudaStreamWaitEvent(s2, p->ev_fork, 0));
-    GB_CUDA(launch_fwd(p->dev, obj, alist, fit, L.f_half, p->Zt_fwd, p->fwd_tpb, p->fwd_variant,
-                       p->d_partials, st));
-    GB_CUDA(launch_fwd(p->dev, obj, alist, fit + L.f_half, L.n_fitems - L.f_half, p->Zt_fwd,
-                       p->fwd_tpb, p->fwd_variant, p->d_partials + (size_t)L.f_half * NZ, s2));
+    GB_CUDA(launch_fwd_group(p, F, 0, obj, alist, p->d_partials, st));
+    GB_CUDA(launch_fwd_group(p, F, 1, obj, alist, p->d_partials, s2));
     GB_CUDA(launch_reduce(h, ioff, (int)NZ, p->d_partials, p->d_ratio, 1, g, s, alist, pred, st));
     GB_CUDA(launch_reduce(L.n - h, ioff + h, (int)NZ, p->d_partials, p->d_ratio + h * NZ, 1, g, s,
                           alist + h, pred ? pred + h * NZ : nullptr, s2));
@@ -1095,7 +1223,7 @@ gb_status gb_spect_osem_step(gb_spect_plan *p, float *obj, const float *g, const
     const int li = list_index(p, subset);
     if (li >= 0 && p->osem_split && p->dev.psf && p->lists[li].n >= 4 && p->lists[li].n <= p->G)
         return osem_split_step(p, p->lists[li], obj, g, s, nbp, pred, st);
-    gb_status r = run_forward(p, obj, subset, p->d_ratio, 1, g, s, pred, st);
+    gb_status r = run_forward(p, obj, subset, p->d_ratio, 1, g, s, pred, p->d_partials, st);
     if (r != GB_OK) return r;
     UpdateArgs u{};
     u.f = obj;
@@ -1124,7 +1252,7 @@ gb_status gb_spect_bsrem_step(gb_spect_plan *p, const float *in, float *out, con
     GB_CHECK_ARG(in != out, "BSREM needs distinct input and output objects");
     GB_INJECT_LAUNCH();
     cudaStream_t st = as_stream(stream);
-    gb_status r = run_forward(p, in, subset, p->d_ratio, 1, g, s, nullptr, st);
+    gb_status r = run_forward(p, in, subset, p->d_ratio, 1, g, s, nullptr, p->d_partials, st);
     if (r != GB_OK) return r;
     UpdateArgs u{};
     u.f_in = in;
@@ -1201,20 +1329,19 @@ gb_status gb_rdp_hessian_vector(const float *f, const float *x, float *out, int3
 
 namespace gb {
 
-bool plan_forward_args(const gb_spect_plan *p, int subset, FwdArgs *a) {
+bool plan_forward_need(const gb_spect_plan *p, int subset, int *n_sel, int *n_items,
+                       size_t *floats) {
     const int li = p ? list_index(p, subset) : -1;
     if (li < 0) return false;
-    const gb_spect_plan::List &L = p->lists[li];
-    a->g = p->dev;
-    a->alist = p->d_alist + L.alist_off;
-    a->n_sel = L.n;
-    a->items = p->d_items + L.fitem_off;
-    a->n_items = L.n_fitems;
-    a->ioff = p->d_ioff + L.ioff_off;
-    a->Zt = p->Zt_fwd;
-    a->tpb = p->fwd_tpb;
-    a->variant = p->fwd_variant;
+    *n_sel = p->lists[li].n;
+    *n_items = p->lists[li].max_fitems;
+    *floats = (size_t)*n_items * p->N * p->nz;
     return true;
+}
+
+gb_status plan_forward(gb_spect_plan *p, const float *obj, int subset, float *out,
+                       float *partials, cudaStream_t st) {
+    return run_forward(p, obj, subset, out, 0, nullptr, nullptr, nullptr, partials, st);
 }
 
 }  // namespace gb
@@ -1241,23 +1368,27 @@ struct gb_spect_batch {
     float *ratio[kMaxBatch] = {};
     float *bp[kMaxBatch] = {};
     int slots_cap[kMaxBatch] = {};  // W slots of each entry
-    CUtensorMap tm[kMaxBatch];  // 64-byte aligned type
-    struct Lists {
-        int4 *fitems = nullptr;
-        int n_fitems = 0;
-        int2 *rows = nullptr;
+    CUtensorMap tm[kMaxBatch] = {};  // 64-byte aligned type
+    // One angle group (G angles of every entry) of a list.  Items of the entries without
+    // strip kernels come first (n_plain of them), each part ordered by cost.
+    struct Group {
+        int4 *fitems = nullptr, *bitems = nullptr;
+        int n_fitems = 0, n_bitems = 0, f_plain = 0, b_plain = 0;
+        int4 *gitems = nullptr;  // first forward kernel of the strip entries
+        int n_gitems = 0, g_plain = 0;
+        int2 *rows = nullptr;  // (entry, slot in group) of every forward output row
         int *row_off = nullptr, *row_items = nullptr;
         int n_rows = 0;
-        std::vector<int4 *> bitems;  // per angle group
-        std::vector<int> n_bitems;
-        int n_groups = 0;
+    };
+    struct Lists {
+        std::vector<Group> groups;
         int n_sel[kMaxBatch] = {};
         const int *alist[kMaxBatch] = {};  // device angle list of each entry
     };
     std::vector<Lists> lists;
     float *partials = nullptr;
     int nz_max = 0;
-    int *counters = nullptr;  // [2]: forward and B1 queues
+    int *counters = nullptr;  // [2]: queues of the plain and of the strip items
 };
 
 static void free_batch(gb_spect_batch *b) {
@@ -1269,11 +1400,14 @@ static void free_batch(gb_spect_batch *b) {
         dev_free(b->bp[e]);
     }
     for (auto &L : b->lists) {
-        dev_free(L.fitems);
-        dev_free(L.rows);
-        dev_free(L.row_off);
-        dev_free(L.row_items);
-        for (int4 *p : L.bitems) dev_free(p);
+        for (auto &g : L.groups) {
+            dev_free(g.fitems);
+            dev_free(g.bitems);
+            dev_free(g.gitems);
+            dev_free(g.rows);
+            dev_free(g.row_off);
+            dev_free(g.row_items);
+        }
     }
     dev_free(b->partials);
     dev_free(b->counters);
@@ -1289,17 +1423,18 @@ static gb_status upload_vec(T **dst, const std::vector<T> &v) {
 }
 
 // Work items of the entries' angles (entry e: angles al[e][s0 .. s0 + n[e])), split by the
-// cost model into about kBatchWaves waves and sorted by cost, largest first; slot indices
-// are relative to s0.  order[k] = index of the k-th item in (entry, slot, plane) order.
+// cost model into about kBatchWaves waves and sorted by cost, largest first, the n_plain
+// items of entries without strip kernels before the others; slot indices are relative to s0.
+// order[k] = index of the k-th item in (entry, slot, plane) order.
 static void batch_items(const gb_spect_batch *b, const std::vector<std::vector<int>> &al,
-                        const std::vector<int> &s0, const std::vector<int> &n, bool fwd,
-                        std::vector<int4> &items, std::vector<int> &order) {
+                        const std::vector<int> &s0, const std::vector<int> &n, WorkKind kind,
+                        std::vector<int4> &items, std::vector<int> &order, int &n_plain) {
     std::vector<std::vector<double>> w;
     std::vector<int> ent, slot;
     double total = 0;
     for (int e = 0; e < b->n; e++)
         for (int i = 0; i < n[e]; i++) {
-            w.push_back(plane_work(b->plans[e], al[e][s0[e] + i], fwd));
+            w.push_back(plane_work(b->plans[e], al[e][s0[e] + i], kind));
             ent.push_back(e);
             slot.push_back(i);
             total += sum_of(w.back());
@@ -1313,7 +1448,7 @@ static void batch_items(const gb_spect_batch *b, const std::vector<std::vector<i
         const int c = std::max(1, std::min(std::max(1, Lp / 4),
                                            (int)std::lround(sum_of(w[k]) / std::max(target, 1.0))));
         std::vector<int4> part;
-        split_planes(w[k], c, slot[k], part);
+        split_planes(w[k], c, slot[k], part, strip_plane_cap(b->plans[ent[k]]), kStripEmpty);
         for (int4 it : part) {
             it.w = ent[k];
             double cst = 0;
@@ -1324,7 +1459,11 @@ static void batch_items(const gb_spect_batch *b, const std::vector<std::vector<i
     }
     std::vector<int> idx(raw.size());
     for (size_t k = 0; k < idx.size(); k++) idx[k] = (int)k;
-    std::stable_sort(idx.begin(), idx.end(), [&](int a, int c) { return cost[a] > cost[c]; });
+    auto strip = [&](int k) { return b->plans[raw[k].w]->dev.strip > 0; };
+    std::stable_sort(idx.begin(), idx.end(), [&](int a, int c) {
+        return strip(a) != strip(c) ? strip(c) : cost[a] > cost[c];
+    });
+    n_plain = (int)std::count_if(idx.begin(), idx.end(), [&](int k) { return !strip(k); });
     items.resize(raw.size());
     order.assign(raw.size(), 0);
     for (size_t k = 0; k < idx.size(); k++) {
@@ -1350,47 +1489,61 @@ static gb_status batch_forward(gb_spect_batch *b, int li, const float *const *ob
                                float *const *out, const float *const *gproj,
                                const float *const *sadd, cudaStream_t st) {
     const gb_spect_batch::Lists &L = b->lists[li];
-    FwdBatch fp;
-    std::memset(&fp, 0, sizeof(fp));
-    for (int e = 0; e < b->n; e++) {
-        fp.tm[e] = b->tm[e];
-        fp.g[e] = batch_dev(b, e);
-        fp.f[e] = objects[e];
-        fp.alist[e] = L.alist[e];
-    }
-    fp.items = L.fitems;
-    fp.n_items = L.n_fitems;
-    fp.counter = b->counters;
-    fp.partials = b->partials;
-    fp.nz_max = b->nz_max;
-    GB_CUDA(cudaMemsetAsync(b->counters, 0, sizeof(int), st));
-    const int grid = std::max(1, std::min(L.n_fitems, b->plans[0]->sm_count));
-    cudaError_t err = cudaErrorInvalidValue;
-    switch (b->K) {
-#define GB_BATCH_CASE(KK)                                  \
-    case KK:                                               \
-        err = launch_fwd_psf_batch_##KK(fp, grid, st);     \
+    for (size_t gi = 0; gi < L.groups.size(); gi++) {
+        const gb_spect_batch::Group &gr = L.groups[gi];
+        const int a0 = (int)gi * b->G;
+        FwdBatch fp;
+        std::memset(&fp, 0, sizeof(fp));
+        ReduceBatch rp;
+        std::memset(&rp, 0, sizeof(rp));
+        for (int e = 0; e < b->n; e++) {
+            const int NZ = b->plans[e]->N * b->plans[e]->nz;
+            fp.tm[e] = b->tm[e];
+            fp.g[e] = batch_dev(b, e);
+            fp.f[e] = objects[e];
+            fp.W[e] = b->W[e];
+            fp.alist[e] = rp.alist[e] = L.alist[e] + a0;
+            rp.out[e] = out[e] + (size_t)a0 * NZ;
+            rp.gproj[e] = gproj ? gproj[e] : nullptr;
+            rp.sadd[e] = sadd ? sadd[e] : nullptr;
+            rp.NZ[e] = NZ;
+        }
+        fp.nz_max = b->nz_max;
+        const int sms = b->plans[0]->sm_count;
+        GB_CUDA(cudaMemsetAsync(b->counters, 0, 2 * sizeof(int), st));
+        if (gr.f_plain > 0) {
+            fp.items = gr.fitems;
+            fp.n_items = gr.f_plain;
+            fp.counter = b->counters;
+            fp.partials = b->partials;
+            cudaError_t err = cudaErrorInvalidValue;
+            switch (b->K) {
+#define GB_BATCH_CASE(KK)                                                              \
+    case KK:                                                                           \
+        err = launch_fwd_psf_batch_##KK(fp, std::min(gr.f_plain, sms), st);            \
         break;
-        GB_FOR_EACH_K(GB_BATCH_CASE)
+                GB_FOR_EACH_K(GB_BATCH_CASE)
 #undef GB_BATCH_CASE
+            }
+            GB_CUDA(err);
+        }
+        if (gr.n_fitems > gr.f_plain) {
+            fp.items = gr.gitems + gr.g_plain;
+            fp.n_items = gr.n_gitems - gr.g_plain;
+            fp.yitems = gr.fitems + gr.f_plain;
+            fp.n_yitems = gr.n_fitems - gr.f_plain;
+            fp.counter = b->counters + 1;
+            fp.partials = b->partials + (size_t)gr.f_plain * b->nz_max;
+            GB_CUDA(launch_fwd_strip_batch(fp, b->n, std::min(fp.n_items, sms), st));
+        }
+        rp.rows = gr.rows;
+        rp.row_off = gr.row_off;
+        rp.row_items = gr.row_items;
+        rp.partials = b->partials;
+        rp.nz_max = b->nz_max;
+        rp.ratio = ratio;
+        GB_CUDA(launch_reduce_batch(rp, gr.n_rows, st));
     }
-    GB_CUDA(err);
-    ReduceBatch rp;
-    std::memset(&rp, 0, sizeof(rp));
-    for (int e = 0; e < b->n; e++) {
-        rp.out[e] = out[e];
-        rp.gproj[e] = gproj ? gproj[e] : nullptr;
-        rp.sadd[e] = sadd ? sadd[e] : nullptr;
-        rp.alist[e] = L.alist[e];
-        rp.NZ[e] = b->plans[e]->N * b->plans[e]->nz;
-    }
-    rp.rows = L.rows;
-    rp.row_off = L.row_off;
-    rp.row_items = L.row_items;
-    rp.partials = b->partials;
-    rp.nz_max = b->nz_max;
-    rp.ratio = ratio;
-    GB_CUDA(launch_reduce_batch(rp, L.n_rows, st));
     return GB_OK;
 }
 
@@ -1405,7 +1558,8 @@ static gb_status batch_backward(gb_spect_batch *b, int li, const float *const *p
             const gb_spect_plan *p = b->plans[e];
             GB_CUDA(cudaMemsetAsync(out[e], 0, (size_t)p->N * p->N * p->nz * sizeof(float), st));
         }
-    for (int gi = 0; gi < L.n_groups; gi++) {
+    for (int gi = 0; gi < (int)L.groups.size(); gi++) {
+        const gb_spect_batch::Group &gr = L.groups[gi];
         B1Batch bp1;
         std::memset(&bp1, 0, sizeof(bp1));
         B2Batch bp2;
@@ -1435,13 +1589,20 @@ static gb_status batch_backward(gb_spect_batch *b, int li, const float *const *p
                 blocks += kind == 1 ? b2_scatter_blocks(bp2.g[e], na) : b2_gather_blocks(bp2.g[e]);
         }
         for (int e = b->n; e <= kMaxBatch; e++) bp2.block_off[e] = blocks;
-        bp1.items = L.bitems[gi];
-        bp1.n_items = L.n_bitems[gi];
-        bp1.counter = b->counters + 1;
-        GB_CUDA(cudaMemsetAsync(b->counters + 1, 0, sizeof(int), st));
-        if (L.n_bitems[gi] > 0)
-            GB_CUDA(launch_b1_batch(b->K, bp1, std::min(L.n_bitems[gi], b->plans[0]->sm_count),
-                                    st));
+        const int sms = b->plans[0]->sm_count;
+        GB_CUDA(cudaMemsetAsync(b->counters, 0, 2 * sizeof(int), st));
+        if (gr.b_plain > 0) {
+            bp1.items = gr.bitems;
+            bp1.n_items = gr.b_plain;
+            bp1.counter = b->counters;
+            GB_CUDA(launch_b1_batch(b->K, bp1, std::min(gr.b_plain, sms), st));
+        }
+        if (gr.n_bitems > gr.b_plain) {
+            bp1.items = gr.bitems + gr.b_plain;
+            bp1.n_items = gr.n_bitems - gr.b_plain;
+            bp1.counter = b->counters + 1;
+            GB_CUDA(launch_b1_strip_batch(bp1, b->n, std::min(bp1.n_items, sms), st));
+        }
         if (kind == 1)
             GB_CUDA(launch_b2_scatter_batch(bp2, blocks, st));
         else
@@ -1523,7 +1684,7 @@ gb_status gb_spect_batch_create(gb_spect_plan *const *plans, int32_t n, gb_spect
     for (int li = 0; li < b->n_lists; li++) {
         gb_spect_batch::Lists &L = b->lists[li];
         std::vector<std::vector<int>> al(n);
-        std::vector<int> s0(n, 0), cnt(n);
+        int n_groups = 0;
         for (int e = 0; e < n; e++) {
             const gb_spect_plan *p = b->plans[e];
             const gb_spect_plan::List &pl = p->lists[li];
@@ -1531,54 +1692,54 @@ gb_status gb_spect_batch_create(gb_spect_plan *const *plans, int32_t n, gb_spect
             BCUDA(cudaMemcpy(h.data(), p->d_alist + pl.alist_off, pl.n * sizeof(int),
                              cudaMemcpyDeviceToHost));
             al[e] = h;
-            cnt[e] = pl.n;
             L.n_sel[e] = pl.n;
             alist_off[li][e] = all_angles.size();
             all_angles.insert(all_angles.end(), h.begin(), h.end());
             b->slots_cap[e] = std::max(b->slots_cap[e], std::min(b->G, pl.n));
-            L.n_groups = std::max(L.n_groups, (pl.n + b->G - 1) / b->G);
+            n_groups = std::max(n_groups, (pl.n + b->G - 1) / b->G);
         }
-        // forward items and the reduction rows
-        std::vector<int4> fit;
-        std::vector<int> order;
-        batch_items(b, al, s0, cnt, true, fit, order);
-        std::vector<int2> rows;
-        std::vector<int> row_off{0}, row_items;
-        {
-            // the unsorted items come in (entry, slot, plane) order: group them by row
-            std::vector<int4> raw(fit.size());
-            for (size_t k = 0; k < order.size(); k++) raw[k] = fit[order[k]];
-            size_t k = 0;
-            for (int e = 0; e < n; e++)
-                for (int s = 0; s < cnt[e]; s++) {
-                    rows.push_back(make_int2(e, s));
-                    while (k < raw.size() && raw[k].w == e && raw[k].x == s)
-                        row_items.push_back(order[k++]);
-                    row_off.push_back((int)row_items.size());
-                }
-        }
-        L.n_fitems = (int)fit.size();
-        L.n_rows = (int)rows.size();
-        max_items = std::max(max_items, fit.size());
-        BFAIL(upload_vec(&L.fitems, fit));
-        BFAIL(upload_vec(&L.rows, rows));
-        BFAIL(upload_vec(&L.row_off, row_off));
-        BFAIL(upload_vec(&L.row_items, row_items));
-        // B1 items per angle group
-        for (int gi = 0; gi < L.n_groups; gi++) {
-            std::vector<int> gs0(n), gcnt(n);
+        L.groups.resize(n_groups);
+        for (int gi = 0; gi < n_groups; gi++) {
+            gb_spect_batch::Group &gr = L.groups[gi];
+            std::vector<int> s0(n), cnt(n);
             for (int e = 0; e < n; e++) {
-                gs0[e] = gi * b->G;
-                gcnt[e] = std::max(0, std::min(b->G, cnt[e] - gs0[e]));
+                s0[e] = gi * b->G;
+                cnt[e] = std::max(0, std::min(b->G, L.n_sel[e] - s0[e]));
             }
-            std::vector<int4> bit;
-            std::vector<int> border;
-            batch_items(b, al, gs0, gcnt, false, bit, border);
-            int4 *d = nullptr;
-            gb_status st = upload_vec(&d, bit);
-            L.bitems.push_back(d);
-            L.n_bitems.push_back((int)bit.size());
-            BFAIL(st);
+            // forward items and the reduction rows
+            std::vector<int4> fit, bit;
+            std::vector<int> order, border;
+            batch_items(b, al, s0, cnt, WORK_FWD, fit, order, gr.f_plain);
+            std::vector<int2> rows;
+            std::vector<int> row_off{0}, row_items;
+            {
+                // the unsorted items come in (entry, slot, plane) order: group them by row
+                std::vector<int4> raw(fit.size());
+                for (size_t k = 0; k < order.size(); k++) raw[k] = fit[order[k]];
+                size_t k = 0;
+                for (int e = 0; e < n; e++)
+                    for (int s = 0; s < cnt[e]; s++) {
+                        rows.push_back(make_int2(e, s));
+                        while (k < raw.size() && raw[k].w == e && raw[k].x == s)
+                            row_items.push_back(order[k++]);
+                        row_off.push_back((int)row_items.size());
+                    }
+            }
+            gr.n_fitems = (int)fit.size();
+            gr.n_rows = (int)rows.size();
+            max_items = std::max(max_items, fit.size());
+            BFAIL(upload_vec(&gr.fitems, fit));
+            BFAIL(upload_vec(&gr.rows, rows));
+            BFAIL(upload_vec(&gr.row_off, row_off));
+            BFAIL(upload_vec(&gr.row_items, row_items));
+            batch_items(b, al, s0, cnt, WORK_B1, bit, border, gr.b_plain);
+            gr.n_bitems = (int)bit.size();
+            BFAIL(upload_vec(&gr.bitems, bit));
+            if (gr.n_fitems > gr.f_plain) {
+                batch_items(b, al, s0, cnt, WORK_GATHER, bit, border, gr.g_plain);
+                gr.n_gitems = (int)bit.size();
+                BFAIL(upload_vec(&gr.gitems, bit));
+            }
         }
     }
     BFAIL(upload_vec(&b->d_alists, all_angles));
@@ -1586,7 +1747,7 @@ gb_status gb_spect_batch_create(gb_spect_plan *const *plans, int32_t n, gb_spect
         for (int e = 0; e < n; e++) b->lists[li].alist[e] = b->d_alists + alist_off[li][e];
     for (int e = 0; e < n; e++) {
         const gb_spect_plan *p = b->plans[e];
-        const size_t slab = (size_t)p->Lp * p->dev.nya * p->nz;
+        const size_t slab = stack_slot(p->dev);
         BCUDA(dev_alloc(&b->W[e], (size_t)b->slots_cap[e] * slab * sizeof(float)));
         BCUDA(dev_alloc(&b->wrange[e], (size_t)b->slots_cap[e] * p->Lp * sizeof(int2)));
         BCUDA(cudaMemset(b->wrange[e], 0, (size_t)b->slots_cap[e] * p->Lp * sizeof(int2)));
@@ -1599,7 +1760,7 @@ gb_status gb_spect_batch_create(gb_spect_plan *const *plans, int32_t n, gb_spect
         BCUDA(dev_alloc(&b->ratio[e], max_sel * p->N * p->nz * sizeof(float)));
         if (multi) BCUDA(dev_alloc(&b->bp[e], (size_t)p->N * p->N * p->nz * sizeof(float)));
         const int HP = (b->K / 2 + 3) / 4 * 4;
-        BCUDA(make_att_tmap(p->dev, fwd_s_cols(128, HP), &b->tm[e]));
+        if (!p->dev.strip) BCUDA(make_att_tmap(p->dev, fwd_s_cols(128, HP), &b->tm[e]));
     }
     BCUDA(dev_alloc(&b->partials, max_items * b->nz_max * sizeof(float)));
     BCUDA(dev_alloc(&b->counters, 2 * sizeof(int)));

@@ -60,25 +60,20 @@ extern "C" gb_status gb_spect_forward_static(gb_spect_plan *plan, const float *o
                                              float *proj, int32_t subset, gb_stream_t stream) {
     clear_error();
     GB_CHECK_ARG(plan && object && proj, "null argument");
-    FwdArgs a;
-    if (!plan_forward_args(plan, subset, &a)) {
+    int n_sel = 0, n_items = 0;
+    size_t need = 0;
+    if (!plan_forward_need(plan, subset, &n_sel, &n_items, &need)) {
         set_error("subset %d out of range", subset);
         return GB_ERR_STATE;
     }
-    const size_t need = (size_t)a.n_items * a.g.N * a.g.nz;
     if (need > GB_FWD_STATIC_FLOATS) {
-        set_error("forward of %d angles (%d work items) x %d x %d needs %zu floats of scratch; "
-                  "the static array holds %u",
-                  a.n_sel, a.n_items, a.g.N, a.g.nz, need, (unsigned)GB_FWD_STATIC_FLOATS);
+        set_error("forward of %d angles (%d work items) needs %zu floats of scratch; the static "
+                  "array holds %u",
+                  n_sel, n_items, need, (unsigned)GB_FWD_STATIC_FLOATS);
         return GB_ERR_SHAPE;
     }
     float *scratch = nullptr;
     gb_status s = static_scratch(&scratch);
     if (s != GB_OK) return s;
-    cudaStream_t st = as_stream(stream);
-    GB_CUDA(launch_fwd(a.g, object, a.alist, a.items, a.n_items, a.Zt, a.tpb, a.variant, scratch,
-                       st));
-    GB_CUDA(launch_reduce(a.n_sel, a.ioff, a.g.N * a.g.nz, scratch, proj, 0, nullptr, nullptr,
-                          a.alist, nullptr, st));
-    return GB_OK;
+    return plan_forward(plan, object, subset, proj, scratch, as_stream(stream));
 }
