@@ -61,8 +61,8 @@ cudaError_t launch_b1_strip(const SpectDev &g, const float *proj, const int *ali
                             const int4 *items, int n_items, float *W, cudaStream_t st);
 cudaError_t launch_b2_gather(const SpectDev &g, const float *W, const int *alist, int n_slots,
                              float *out, int mode, const UpdateArgs &u, cudaStream_t st);
-cudaError_t launch_b2_scatter(const SpectDev &g, const float *W, const int *alist, int n_slots,
-                              float *out, cudaStream_t st);
+cudaError_t launch_b2_adjoint(const SpectDev &g, const float *W, const int *alist, int n_slots,
+                              float *out, bool first, cudaStream_t st);
 cudaError_t launch_atten(const SpectDev &g, const float *mu, float dx, int n_angles, float *A,
                          cudaStream_t st);
 cudaError_t launch_rdp(const float *f, float *grad, int nx, int ny, int nz, const UpdateArgs &u,
@@ -121,7 +121,7 @@ struct B2Batch {
     const float *W[kMaxBatch];
     const int *alist[kMaxBatch];    // the group's angles
     int n_slots[kMaxBatch];
-    float *out[kMaxBatch];          // target (write / add / scatter) or OSEM object
+    float *out[kMaxBatch];          // target (write / add) or OSEM object
     const float *nbp[kMaxBatch];    // OSEM: H_m^T 1
     const float *acc[kMaxBatch];    // OSEM: back projection of earlier groups, or null
     int block_off[kMaxBatch + 1];   // first block of each entry (total for unused entries)
@@ -143,10 +143,9 @@ cudaError_t launch_b1_strip_batch(const B1Batch &p, int n, int grid, cudaStream_
 cudaError_t launch_b1_batch(int K, const B1Batch &p, int grid, cudaStream_t st);
 cudaError_t launch_reduce_batch(const ReduceBatch &p, int n_rows, cudaStream_t st);
 cudaError_t launch_b2_gather_batch(const B2Batch &p, int n_blocks, cudaStream_t st);
-cudaError_t launch_b2_scatter_batch(const B2Batch &p, int n_blocks, cudaStream_t st);
-// blocks of 256 threads of one entry in the batched gather / scatter kernels
+cudaError_t launch_b2_adjoint_batch(const B2Batch &p, int n_blocks, cudaStream_t st);
+// blocks of 256 threads of one entry in the batched gather and adjoint kernels
 int b2_gather_blocks(const SpectDev &g);
-int b2_scatter_blocks(const SpectDev &g, int n_slots);
 
 // One forward projection of a plan with the caller's partial-sum buffer (for entry points
 // defined outside spect_plan.cu): the work items and partial floats a subset needs (false when

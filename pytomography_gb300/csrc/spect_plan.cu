@@ -1013,13 +1013,12 @@ static gb_status run_backward(gb_spect_plan *p, const float *proj, int li, int a
     const int n = L.n;
     const size_t NZ = (size_t)p->N * p->nz;
     const int n_groups = (n + p->G - 1) / p->G;
-    if (adjoint) GB_CUDA(cudaMemsetAsync(out, 0, (size_t)p->N * NZ * sizeof(float), st));
     for (int gi = 0; gi < n_groups; gi++) {
         int a0 = gi * p->G, na = std::min(p->G, n - a0);
         GB_CUDA(launch_b1(p->dev, proj + a0 * NZ, alist + a0, na, p->d_items + L.gitem_off[gi],
                           L.n_gitems[gi], p->Zt_b1, p->d_W, st));
         if (adjoint) {
-            GB_CUDA(launch_b2_scatter(p->dev, p->d_W, alist + a0, na, out, st));
+            GB_CUDA(launch_b2_adjoint(p->dev, p->d_W, alist + a0, na, out, gi == 0, st));
             continue;
         }
         const bool last = gi == n_groups - 1;
@@ -1553,11 +1552,6 @@ static gb_status batch_forward(gb_spect_batch *b, int li, const float *const *ob
 static gb_status batch_backward(gb_spect_batch *b, int li, const float *const *proj, int kind,
                                 float *const *out, const float *const *norm_bp, cudaStream_t st) {
     const gb_spect_batch::Lists &L = b->lists[li];
-    if (kind == 1)
-        for (int e = 0; e < b->n; e++) {
-            const gb_spect_plan *p = b->plans[e];
-            GB_CUDA(cudaMemsetAsync(out[e], 0, (size_t)p->N * p->N * p->nz * sizeof(float), st));
-        }
     for (int gi = 0; gi < (int)L.groups.size(); gi++) {
         const gb_spect_batch::Group &gr = L.groups[gi];
         B1Batch bp1;
@@ -1585,8 +1579,7 @@ static gb_status batch_backward(gb_spect_batch *b, int li, const float *const *p
                 bp2.out[e] = out[e];
                 bp2.mode[e] = gi == 0 ? B2_WRITE : B2_ADD;
             }
-            if (na > 0)
-                blocks += kind == 1 ? b2_scatter_blocks(bp2.g[e], na) : b2_gather_blocks(bp2.g[e]);
+            if (na > 0) blocks += b2_gather_blocks(bp2.g[e]);
         }
         for (int e = b->n; e <= kMaxBatch; e++) bp2.block_off[e] = blocks;
         const int sms = b->plans[0]->sm_count;
@@ -1604,7 +1597,7 @@ static gb_status batch_backward(gb_spect_batch *b, int li, const float *const *p
             GB_CUDA(launch_b1_strip_batch(bp1, b->n, std::min(bp1.n_items, sms), st));
         }
         if (kind == 1)
-            GB_CUDA(launch_b2_scatter_batch(bp2, blocks, st));
+            GB_CUDA(launch_b2_adjoint_batch(bp2, blocks, st));
         else
             GB_CUDA(launch_b2_gather_batch(bp2, blocks, st));
     }
