@@ -16,6 +16,12 @@
 
 namespace gb {
 
+// The TOF weight table into shared memory (whole block).
+__device__ __forceinline__ void load_tof_table(const PetDev &g, float *tab) {
+    for (int i = threadIdx.x; i < kTofTab + 2; i += blockDim.x) tab[i] = __ldg(g.tof_tab + i);
+    __syncthreads();
+}
+
 // Event tiles: the events of a list (every event, or one subset i::n) sorted by a
 // locality key, packed as {id1, id2, centred TOF bin, j} where j is the event's position
 // in the list (event index first + j * stride).  Threads of a warp then trace nearby,
@@ -23,17 +29,23 @@ namespace gb {
 // atomics share L2 sectors.  Outputs indexed by j keep the list order.
 //
 // mode 0: out[k or j] = H img;  mode 1 (ratio): out[k] = num[e] / (H img + s[e] + delta)
-template <bool TOF>
+// PATCH: the image also lies in the patch layout (pet_joseph.cuh).
+template <bool TOF, bool PATCH>
 __global__ void __launch_bounds__(256)
     k_pet_fwd(PetDev g, const int4 *__restrict__ rec, long long first, long long stride,
-              long long n, const float *__restrict__ img, float *__restrict__ out, int ratio,
-              const float *__restrict__ sadd, const float *__restrict__ gnum, int gnum_len) {
+              long long n, const float *__restrict__ img, PetPatches pq, float *__restrict__ out,
+              int ratio, const float *__restrict__ sadd, const float *__restrict__ gnum,
+              int gnum_len) {
+    __shared__ float tab[TOF ? kTofTab + 2 : 1];
+    if (TOF) load_tof_table(g, tab);
     long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int4 r = rec[k];
     const float *p0 = g.lut + 3 * (long long)r.x;
     const float *p1 = g.lut + 3 * (long long)r.y;
-    float v = joseph<false, TOF>(g, p0, p1, nullptr, img, r.z, 0.f);
+    float v;
+    if (!PATCH || !joseph_patch<false, TOF>(g, p0, p1, pq, tab, r.z, 0.f, v))
+        v = joseph<false, TOF>(g, p0, p1, nullptr, img, tab, r.z, 0.f);
     if (ratio) {  // internal ratio array, tile order
         const long long e = first + (long long)r.w * stride;
         float pr = sadd ? v + sadd[e] : v;
@@ -44,11 +56,14 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// proj in tile order (sorted = 1, the fused step's ratio array) or list order (0)
-template <bool TOF>
+// proj in tile order (sorted = 1, the fused step's ratio array) or list order (0); PATCH: the
+// sums go to the patch layout, those of LORs along z to img.
+template <bool TOF, bool PATCH>
 __global__ void __launch_bounds__(256)
     k_pet_bwd(PetDev g, const int4 *__restrict__ rec, long long n,
-              const float *__restrict__ proj, int sorted, float *__restrict__ img) {
+              const float *__restrict__ proj, int sorted, float *__restrict__ img, PetPatches pq) {
+    __shared__ float tab[TOF ? kTofTab + 2 : 1];
+    if (TOF) load_tof_table(g, tab);
     long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int4 r = rec[k];
@@ -56,7 +71,73 @@ __global__ void __launch_bounds__(256)
     if (v == 0.f) return;
     const float *p0 = g.lut + 3 * (long long)r.x;
     const float *p1 = g.lut + 3 * (long long)r.y;
-    joseph<true, TOF>(g, p0, p1, img, nullptr, r.z, v);
+    float unused;
+    if (PATCH && joseph_patch<true, TOF>(g, p0, p1, pq, tab, r.z, v, unused)) return;
+    joseph<true, TOF>(g, p0, p1, img, nullptr, tab, r.z, v);
+}
+
+// Both patch arrays of an image: a thread takes one (y, z) cell position through kBuildX
+// planes x (positions and planes from -1 on), so every image value it needs is loaded once;
+// lanes along z.  Bound by the 32 bytes a voxel it writes.
+constexpr int kBuildX = 8;
+__global__ void __launch_bounds__(256)
+    k_patch_build(PetDev g, const float *__restrict__ img, PetPatches q) {
+    const int nx = g.n[0], ny = g.n[1], nz = g.n[2], rs = nz + 1;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (ny + 1) * rs) return;
+    const int y = e / rs - 1, z = e % rs - 1;
+    const int xa = (int)blockIdx.y * kBuildX - 1, xb = min(xa + kBuildX, nx);
+    const bool z0 = z >= 0, z1 = z + 1 < nz, y0 = y >= 0, y1 = y + 1 < ny;
+    const float *p = img + ((ptrdiff_t)xa * ny + y) * nz + z;
+    const ptrdiff_t sx = (ptrdiff_t)ny * nz;
+    // c: corners (y, z), (y, z + 1), (y + 1, z), (y + 1, z + 1) of plane x
+    auto load = [&](int x, const float *a) {
+        const bool in = x >= 0 && x < nx;
+        return make_float4(in && y0 && z0 ? __ldg(a) : 0.f, in && y0 && z1 ? __ldg(a + 1) : 0.f,
+                           in && y1 && z0 ? __ldg(a + nz) : 0.f,
+                           in && y1 && z1 ? __ldg(a + nz + 1) : 0.f);
+    };
+    float4 c = load(xa, p);
+#pragma unroll 4
+    for (int x = xa; x < xb; x++) {
+        p += sx;
+        const float4 d = load(x + 1, p);
+        if (x >= 0) q.qx[((size_t)x * (ny + 1) + y + 1) * rs + z + 1] = c;
+        if (y0) q.qy[((size_t)y * (nx + 1) + x + 1) * rs + z + 1] = make_float4(c.x, c.y, d.x, d.y);
+        c = d;
+    }
+}
+
+// Back projection of a voxel from both patch arrays (each cell's corner that is the voxel).
+__device__ __forceinline__ float patch_fold(const PetDev &g, const PetPatches &pq, int x, int y,
+                                            int z) {
+    const size_t rs = g.n[2] + 1;
+    const float4 *a = pq.qx + ((size_t)x * (g.n[1] + 1) + y) * rs + z;  // cell (y - 1, z - 1)
+    const float4 *b = pq.qy + ((size_t)y * (g.n[0] + 1) + x) * rs + z;  // cell (x - 1, z - 1)
+    const float sx = (__ldg(&a[rs + 1].x) + __ldg(&a[rs].y)) + (__ldg(&a[1].z) + __ldg(&a[0].w));
+    const float sy = (__ldg(&b[rs + 1].x) + __ldg(&b[rs].y)) + (__ldg(&b[1].z) + __ldg(&b[0].w));
+    return sx + sy;
+}
+
+// img += folded patches (OSEM = false), or the listmode OSEM update of f with
+// bp = img + folded patches.
+template <bool OSEM>
+__global__ void __launch_bounds__(256)
+    k_patch_fold(PetDev g, PetPatches pq, float *__restrict__ img, float *__restrict__ f,
+                 const float *__restrict__ nbp) {
+    const int z = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+    const int x = blockIdx.z;
+    if (z >= g.n[2] || y >= g.n[1]) return;
+    const size_t o = ((size_t)x * g.n[1] + y) * g.n[2] + z;
+    const float bp = img[o] + patch_fold(g, pq, x, y, z);
+    if (!OSEM) {
+        img[o] = bp;
+        return;
+    }
+    const float fv = f[o], nb = nbp[o];
+    const float pre = __fmul_rn(fv, __frcp_rn(__fadd_rn(nb, 1e-11f)));
+    const float fn = __fadd_rn(fv, __fmul_rn(pre, __fsub_rn(bp, nb)));
+    f[o] = fn <= 0.f ? 0.f : fn;
 }
 
 // Deterministic back projection: the same traces accumulated as 64-bit fixed-point sums.
@@ -72,7 +153,8 @@ __global__ void __launch_bounds__(256)
     if (v == 0.f) return;
     const float *p0 = g.lut + 3 * (long long)r.x;
     const float *p1 = g.lut + 3 * (long long)r.y;
-    joseph<true, TOF, true>(g, p0, p1, reinterpret_cast<float *>(acc), nullptr, r.z, v, *scale);
+    joseph<true, TOF, true>(g, p0, p1, reinterpret_cast<float *>(acc), nullptr, g.tof_tab, r.z, v,
+                            *scale);
 }
 
 // Largest |proj| of the list (atomicMax on the bit patterns of non-negative floats, which
@@ -168,8 +250,9 @@ __device__ __forceinline__ void pair_from_index(long long p, int n, int &i, int 
     j = (int)(p - start(ib) + ib + 1);
 }
 
+template <bool PATCH>
 __global__ void __launch_bounds__(256)
-    k_pet_sens(PetDev g, const int *__restrict__ pairs, long long first, long long n,
+    k_pet_sens(PetDev g, PetPatches pq, const int *__restrict__ pairs, long long first, long long n,
                const float *__restrict__ w, const float *__restrict__ mu, float add,
                float *__restrict__ img) {
     long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -185,9 +268,11 @@ __global__ void __launch_bounds__(256)
     const float *p0 = g.lut + 3 * (long long)i;
     const float *p1 = g.lut + 3 * (long long)j;
     float v = w ? w[q] : 1.f;
-    if (mu) v *= expf(-joseph<false, false>(g, p0, p1, nullptr, mu, 0, 0.f));
+    if (mu) v *= expf(-joseph<false, false>(g, p0, p1, nullptr, mu, nullptr, 0, 0.f));
     v += add;
-    joseph<true, false>(g, p0, p1, img, nullptr, 0, v);
+    float unused;
+    if (PATCH && joseph_patch<true, false>(g, p0, p1, pq, nullptr, 0, v, unused)) return;
+    joseph<true, false>(g, p0, p1, img, nullptr, nullptr, 0, v);
 }
 
 // Listmode OSEM update: f <- f + f/(nbp + delta) * (bp - nbp); f[f <= 0] = 0
@@ -223,6 +308,8 @@ struct gb_pet_plan {
     unsigned long long *d_acc64 = nullptr;
     unsigned *d_maxbits = nullptr;
     float *d_scale = nullptr;
+    // patch layout (pet_joseph.cuh), null where it cannot pay
+    PetPatches patch{};
 };
 
 static void pet_free(gb_pet_plan *p) {
@@ -236,6 +323,8 @@ static void pet_free(gb_pet_plan *p) {
     dev_free(p->d_acc64);
     dev_free(p->d_maxbits);
     dev_free(p->d_scale);
+    dev_free(p->patch.qx);
+    dev_free(p->patch.qy);
     delete p;
 }
 
@@ -308,6 +397,95 @@ static gb_status build_tiles(gb_pet_plan *p, int n_subsets) {
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return fail(e);
     dev_free(keys); dev_free(keys2); dev_free(vals); dev_free(vals2); dev_free(tmp);
     return GB_OK;
+}
+
+// Whether n LORs pay for the passes over the patch layout: their planes (bounded by the image
+// and, with TOF, by the window) against the voxels.  Measured, single corners -> patches, us:
+//   200 x 200 x 96, 13 TOF bins      10k events   100k        300k        1M
+//     forward                        50 -> 70     87 -> 84    185 -> 148  480 -> 341
+//     back projection                70 -> 84     134 -> 122  320 -> 215  872 -> 419
+//   the same without TOF             61 -> 82     103 -> 101  239 -> 184  631 -> 448
+//                                    109 -> 88    261 -> 177  665 -> 351  1798 -> 804
+//   100 x 100 x 48, 13 TOF bins      29 -> 31     40 -> 35    89 -> 67    237 -> 161
+//                                    40 -> 36     87 -> 50    215 -> 98   542 -> 218
+// The forward, bound by the L1 lines its lanes touch (one per plane instead of up to four),
+// breaks even near 2.8 planes per voxel, the back projection near 1.
+constexpr double kPatchFwd = 2.8, kPatchBwd = 1.0;
+static bool patch_pays(const PetDev &g, double n, bool tof, double planes_per_voxel) {
+    double planes = 0.6 * std::max(g.n[0], g.n[1]);
+    if (tof) {
+        const double win = 2.0 * (g.nsig * g.sig) + g.bw;
+        planes = std::min(planes, win / std::min(g.vox[0], g.vox[1]));
+    }
+    return n * planes > planes_per_voxel * (double)g.n_vox;
+}
+// The largest patch layout a plan keeps.
+constexpr size_t kPatchMaxBytes = (size_t)2 << 30;
+
+static bool use_patches(const gb_pet_plan *p, long long n, bool tof, double planes_per_voxel) {
+    return p->patch.qx && patch_pays(p->dev, (double)n, tof, planes_per_voxel);
+}
+
+static cudaError_t build_patches(const gb_pet_plan *p, const float *img, cudaStream_t st) {
+    const PetDev &g = p->dev;
+    const dim3 grid(((g.n[1] + 1) * (g.n[2] + 1) + 255) / 256, (g.n[0] + kBuildX) / kBuildX);
+    k_patch_build<<<grid, 256, 0, st>>>(g, img, p->patch);
+    return cudaGetLastError();
+}
+static cudaError_t clear_patches(const gb_pet_plan *p, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(p->patch.qx, 0, patch_elems_x(p->dev) * sizeof(float4), st);
+    if (e != cudaSuccess) return e;
+    return cudaMemsetAsync(p->patch.qy, 0, patch_elems_y(p->dev) * sizeof(float4), st);
+}
+// img += patches, or (f) the OSEM update of f with bp = img + patches
+static cudaError_t fold_patches(const gb_pet_plan *p, float *img, float *f, const float *nbp,
+                                cudaStream_t st) {
+    const PetDev &g = p->dev;
+    const dim3 block(32, 8), grid((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]);
+    if (f)
+        k_patch_fold<true><<<grid, block, 0, st>>>(g, p->patch, img, f, nbp);
+    else
+        k_patch_fold<false><<<grid, block, 0, st>>>(g, p->patch, img, nullptr, nullptr);
+    return cudaGetLastError();
+}
+
+// Forward projection of n tiles (k_pet_fwd's outputs), building the patch layout if it pays.
+static cudaError_t pet_forward(const gb_pet_plan *p, const int4 *rec, long long first,
+                               long long stride, long long n, const float *img, float *out,
+                               int ratio, const float *sadd, const float *gnum, int gnum_len,
+                               bool tof, cudaStream_t st) {
+    const unsigned blocks = (unsigned)((n + 255) / 256);
+    const bool patch = use_patches(p, n, tof, kPatchFwd);
+    if (patch) {
+        cudaError_t e = build_patches(p, img, st);
+        if (e != cudaSuccess) return e;
+    }
+    auto *fn = tof ? (patch ? k_pet_fwd<true, true> : k_pet_fwd<true, false>)
+                   : (patch ? k_pet_fwd<false, true> : k_pet_fwd<false, false>);
+    fn<<<blocks, 256, 0, st>>>(p->dev, rec, first, stride, n, img, p->patch, out, ratio, sadd, gnum,
+                               gnum_len);
+    return cudaGetLastError();
+}
+
+// Back projection of n tiles into img, which is cleared first; f: followed by the OSEM update
+// of f (img is then scratch).
+static cudaError_t pet_backward(const gb_pet_plan *p, const int4 *rec, long long n,
+                                const float *proj, int sorted, float *img, float *f,
+                                const float *nbp, cudaStream_t st) {
+    const bool tof = p->dev.tof, patch = use_patches(p, n, tof, kPatchBwd);
+    cudaError_t e = cudaMemsetAsync(img, 0, (size_t)p->img_size * sizeof(float), st);
+    if (e == cudaSuccess && patch) e = clear_patches(p, st);
+    if (e != cudaSuccess) return e;
+    if (n > 0) {
+        auto *fn = tof ? (patch ? k_pet_bwd<true, true> : k_pet_bwd<true, false>)
+                       : (patch ? k_pet_bwd<false, true> : k_pet_bwd<false, false>);
+        fn<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p->dev, rec, n, proj, sorted, img, p->patch);
+    }
+    if (patch) return fold_patches(p, img, f, nbp, st);
+    if (f)
+        k_pet_update<<<(unsigned)((p->img_size + 255) / 256), 256, 0, st>>>(f, img, nbp,
+                                                                            p->img_size);
+    return cudaGetLastError();
 }
 
 // The tiles of a subset (-1 = every event).
@@ -389,6 +567,16 @@ gb_status gb_pet_plan_create(const gb_pet_desc *d, gb_pet_plan **out) {
                 }
             }
     }
+    // patch layout where the longest list, or a sensitivity image of as many LORs, pays for it
+    const size_t pb = (patch_elems_x(g) + patch_elems_y(g)) * sizeof(float4);
+    if (pb <= kPatchMaxBytes && patch_pays(g, (double)d->n_events, d->tof, kPatchBwd)) {
+        if ((e = dev_alloc(&p->patch.qx, patch_elems_x(g) * sizeof(float4))) != cudaSuccess ||
+            (e = dev_alloc(&p->patch.qy, patch_elems_y(g) * sizeof(float4))) != cudaSuccess) {
+            set_error("patch layout allocation failed: %s", cudaGetErrorString(e));
+            pet_free(p);
+            return e == cudaErrorMemoryAllocation ? GB_ERR_OOM : GB_ERR_CUDA;
+        }
+    }
     gb_status st = build_tiles(p, 1);
     if (st != GB_OK) {
         pet_free(p);
@@ -426,15 +614,8 @@ gb_status gb_pet_forward(gb_pet_plan *p, const float *img, float *proj, int32_t 
     long long first, stride, n;
     subset_range(p, subset, first, stride, n);
     if (n == 0) return GB_OK;
-    unsigned blocks = (unsigned)((n + 255) / 256);
-    const int4 *rec = list_tiles(p, subset);
-    if (p->dev.tof)
-        k_pet_fwd<true><<<blocks, 256, 0, as_stream(stream)>>>(p->dev, rec, first, stride, n, img,
-                                                               proj, 0, nullptr, nullptr, 0);
-    else
-        k_pet_fwd<false><<<blocks, 256, 0, as_stream(stream)>>>(p->dev, rec, first, stride, n,
-                                                                img, proj, 0, nullptr, nullptr, 0);
-    GB_LAUNCH_CHECK();
+    GB_CUDA(pet_forward(p, list_tiles(p, subset), first, stride, n, img, proj, 0, nullptr, nullptr,
+                        0, p->dev.tof, as_stream(stream)));
     return GB_OK;
 }
 
@@ -449,10 +630,12 @@ gb_status gb_pet_backward(gb_pet_plan *p, const float *proj, float *img, int32_t
     long long first, stride, n;
     subset_range(p, subset, first, stride, n);
     cudaStream_t st = as_stream(stream);
-    GB_CUDA(cudaMemsetAsync(img, 0, (size_t)p->img_size * sizeof(float), st));
-    if (n == 0) return GB_OK;
-    unsigned blocks = (unsigned)((n + 255) / 256);
     const int4 *rec = list_tiles(p, subset);
+    unsigned blocks = (unsigned)((n + 255) / 256);
+    if (n == 0) {
+        GB_CUDA(cudaMemsetAsync(img, 0, (size_t)p->img_size * sizeof(float), st));
+        return GB_OK;
+    }
     if (p->d_acc64) {  // deterministic mode
         const float cf_max = 1.7320509f * std::max(p->dev.vox[0], std::max(p->dev.vox[1], p->dev.vox[2]));
         GB_CUDA(cudaMemsetAsync(p->d_maxbits, 0, sizeof(unsigned), st));
@@ -468,11 +651,7 @@ gb_status gb_pet_backward(gb_pet_plan *p, const float *proj, float *img, int32_t
         GB_LAUNCH_CHECK();
         return GB_OK;
     }
-    if (p->dev.tof)
-        k_pet_bwd<true><<<blocks, 256, 0, st>>>(p->dev, rec, n, proj, 0, img);
-    else
-        k_pet_bwd<false><<<blocks, 256, 0, st>>>(p->dev, rec, n, proj, 0, img);
-    GB_LAUNCH_CHECK();
+    GB_CUDA(pet_backward(p, rec, n, proj, 0, img, nullptr, nullptr, st));
     return GB_OK;
 }
 
@@ -505,30 +684,11 @@ gb_status gb_pet_osem_step(gb_pet_plan *p, float *img, const float *numerator,
     long long first, stride, n;
     subset_range(p, subset, first, stride, n);
     cudaStream_t st = as_stream(stream);
-    unsigned blocks = (unsigned)((n + 255) / 256);
     const int4 *rec = list_tiles(p, subset);
-    if (n > 0) {
-        if (p->dev.tof)
-            k_pet_fwd<true><<<blocks, 256, 0, st>>>(p->dev, rec, first, stride, n, img,
-                                                    p->d_ratio, 1, additive, numerator,
-                                                    (int)numerator_len);
-        else
-            k_pet_fwd<false><<<blocks, 256, 0, st>>>(p->dev, rec, first, stride, n, img,
-                                                     p->d_ratio, 1, additive, numerator,
-                                                     (int)numerator_len);
-        GB_LAUNCH_CHECK();
-    }
-    GB_CUDA(cudaMemsetAsync(p->d_bp, 0, (size_t)p->img_size * sizeof(float), st));
-    if (n > 0) {
-        if (p->dev.tof)
-            k_pet_bwd<true><<<blocks, 256, 0, st>>>(p->dev, rec, n, p->d_ratio, 1, p->d_bp);
-        else
-            k_pet_bwd<false><<<blocks, 256, 0, st>>>(p->dev, rec, n, p->d_ratio, 1, p->d_bp);
-        GB_LAUNCH_CHECK();
-    }
-    k_pet_update<<<(unsigned)((p->img_size + 255) / 256), 256, 0, st>>>(img, p->d_bp, norm_bp,
-                                                                         p->img_size);
-    GB_LAUNCH_CHECK();
+    if (n > 0)
+        GB_CUDA(pet_forward(p, rec, first, stride, n, img, p->d_ratio, 1, additive, numerator,
+                            (int)numerator_len, p->dev.tof, st));
+    GB_CUDA(pet_backward(p, rec, n, p->d_ratio, 1, p->d_bp, img, norm_bp, st));
     return GB_OK;
 }
 
@@ -543,13 +703,17 @@ gb_status gb_pet_sensitivity(gb_pet_plan *p, const int32_t *pairs, int64_t n_pai
     GB_CHECK_ARG(n_pairs >= 0, "negative pair count");
     cudaStream_t st = as_stream(stream);
     GB_CUDA(cudaMemsetAsync(img, 0, (size_t)p->img_size * sizeof(float), st));
+    const bool patch = use_patches(p, n_pairs, false, kPatchBwd);
+    if (patch) GB_CUDA(clear_patches(p, st));
     const long long chunk = 1LL << 28;  // launch in chunks of 2^28 LORs
     for (long long first = 0; first < n_pairs; first += chunk) {
         long long n = std::min(chunk, (long long)n_pairs - first);
-        k_pet_sens<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p->dev, pairs, first, n, weights,
-                                                                mu, add, img);
+        auto *fn = patch ? k_pet_sens<true> : k_pet_sens<false>;
+        fn<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p->dev, p->patch, pairs, first, n, weights,
+                                                        mu, add, img);
         GB_LAUNCH_CHECK();
     }
+    if (patch) GB_CUDA(fold_patches(p, img, nullptr, nullptr, st));
     return GB_OK;
 }
 
@@ -561,15 +725,8 @@ gb_status gb_pet_lor_forward(gb_pet_plan *p, const float *img, float *proj, int3
     long long first, stride, n;
     subset_range(p, subset, first, stride, n);
     if (n == 0) return GB_OK;
-    unsigned blocks = (unsigned)((n + 255) / 256);
-    const int4 *rec = list_tiles(p, subset);
-    if (use_tof && p->dev.tof)
-        k_pet_fwd<true><<<blocks, 256, 0, as_stream(stream)>>>(p->dev, rec, first, stride, n, img,
-                                                               proj, 0, nullptr, nullptr, 0);
-    else
-        k_pet_fwd<false><<<blocks, 256, 0, as_stream(stream)>>>(p->dev, rec, first, stride, n,
-                                                                img, proj, 0, nullptr, nullptr, 0);
-    GB_LAUNCH_CHECK();
+    GB_CUDA(pet_forward(p, list_tiles(p, subset), first, stride, n, img, proj, 0, nullptr, nullptr,
+                        0, use_tof && p->dev.tof, as_stream(stream)));
     return GB_OK;
 }
 

@@ -63,14 +63,16 @@ __device__ __forceinline__ int pick(int a, int b, int c, int k) {
 // other axes (in voxel units) and the TOF distance s are linear in the plane index i and
 // are evaluated as base + i * step.  Axis-dependent quantities are selected into
 // registers once (no dynamically indexed local arrays).
+// tab: the TOF weight table, in shared memory where a block traces many LORs (the lanes of a
+// warp look up 32 places of it: about 4 shared-memory wavefronts, but 32 L1 lines).
 // DET (back projection only): img is an array of 64-bit integers holding fixed-point sums
 // with `scale` units per 1.0; each contribution is rounded to that grid and added with an
 // integer atomic, so the sums do not depend on the order of the additions.
 template <bool BACK, bool TOF, bool DET = false>
 __device__ __forceinline__ float joseph(const PetDev &g, const float *__restrict__ p0,
                                         const float *__restrict__ p1, float *img,
-                                        const float *__restrict__ cimg, int tbin, float val,
-                                        float scale = 0.f) {
+                                        const float *__restrict__ cimg, const float *tab,
+                                        int tbin, float val, float scale = 0.f) {
     auto add = [&](int off, float v) {
         if constexpr (DET)
             atomicAdd(reinterpret_cast<unsigned long long *>(img) + off,
@@ -152,7 +154,7 @@ __device__ __forceinline__ float joseph(const PetDev &g, const float *__restrict
                     } else {
                         const float t = as * g.tof_inv_step;
                         const int m = min((int)t, kTofTab);
-                        const float t0w = __ldg(g.tof_tab + m), t1w = __ldg(g.tof_tab + m + 1);
+                        const float t0w = tab[m], t1w = tab[m + 1];
                         w *= fmaf(t - (float)m, t1w - t0w, t0w);
                     }
                 }
@@ -187,7 +189,7 @@ __device__ __forceinline__ float joseph(const PetDev &g, const float *__restrict
             if (as > lim) continue;
             const float u = as * g.tof_inv_step;
             const int m = min((int)u, kTofTab);
-            const float t0w = __ldg(g.tof_tab + m), t1w = __ldg(g.tof_tab + m + 1);
+            const float t0w = tab[m], t1w = tab[m + 1];
             w *= fmaf(u - (float)m, t1w - t0w, t0w);
         }
         const float fa = fmaf((float)i, dfa, fa0), fb = fmaf((float)i, dfb, fb0);
@@ -243,6 +245,124 @@ __device__ __forceinline__ float joseph(const PetDev &g, const float *__restrict
         }
     }
     return acc;
+}
+
+// ------------------------------------------------------------------ patches
+// The four image values a plane contributes are the 2 x 2 corners of one cell of the plane.
+// In the patch layout each cell holds its four corners in 16 bytes, one array per transaxial
+// principal axis:
+//   qx[x][jy + 1][jz + 1] = corners (jy, jz), (jy, jz + 1), (jy + 1, jz), (jy + 1, jz + 1)
+//   qy[y][jx + 1][jz + 1] likewise over (x, z);  jy, jx, jz from -1 on, zero outside the image
+// A plane is then one 16-byte load forward and one 16-byte atomic back, instead of four loads
+// and about 2.5 atomics (two of the four lanes of each zero).  Building the layout (or
+// clearing and folding it) costs passes over 32 bytes a voxel, so it pays from a few planes
+// per voxel on (patch_pays).
+struct PetPatches {
+    float4 *qx, *qy;
+};
+
+inline size_t patch_elems_x(const PetDev &g) {
+    return (size_t)g.n[0] * (g.n[1] + 1) * (g.n[2] + 1);
+}
+inline size_t patch_elems_y(const PetDev &g) {
+    return (size_t)g.n[1] * (g.n[0] + 1) * (g.n[2] + 1);
+}
+
+// joseph() through the patch layout.  LORs whose principal axis is z (the caller's `steep`
+// path) return false and leave v alone.
+template <bool BACK, bool TOF>
+__device__ __forceinline__ bool joseph_patch(const PetDev &g, const float *__restrict__ p0,
+                                             const float *__restrict__ p1, const PetPatches &q,
+                                             const float *tab, int tbin, float val, float &v) {
+    const float ax = p0[0], ay = p0[1], az = p0[2];
+    const float dx = p1[0] - ax, dy = p1[1] - ay, dz = p1[2] - az;
+    const float len = sqrtf(dx * dx + dy * dy + dz * dz);
+    v = 0.f;
+    if (len == 0.f) return true;
+    // principal axis from exact differences, as joseph() decides
+    const double ex = fabs((double)p1[0] - (double)ax), ey = fabs((double)p1[1] - (double)ay),
+                 ez = fabs((double)p1[2] - (double)az);
+    const bool ky = ey > ex;
+    if (ez > (ky ? ey : ex)) return false;
+    const float dk = ky ? dy : dx, dt_ = ky ? dx : dy;
+    const float pk = ky ? ay : ax, pt = ky ? ax : ay;
+    const float vk = ky ? g.vox[1] : g.vox[0], vt = ky ? g.vox[0] : g.vox[1];
+    const float ok = ky ? g.org[1] : g.org[0], ot = ky ? g.org[0] : g.org[1];
+    const int nk = ky ? g.n[1] : g.n[0], nt = ky ? g.n[0] : g.n[1], nz = g.n[2];
+    const float cf = vk * len / fabsf(dk);
+    const float pk1 = ky ? p1[1] : p1[0];
+    int i0 = max((int)ceilf((fminf(pk, pk1) - ok) / vk), 0);
+    int i1 = min((int)floorf((fmaxf(pk, pk1) - ok) / vk), nk - 1);
+    const float idk = 1.f / dk;
+    const float t0 = (ok - pk) * idk, dt = vk * idk;
+    const float ivt = 1.f / vt, ivz = 1.f / g.vox[2];
+    const float ft0 = (pt - ot + t0 * dt_) * ivt, dft = dt * dt_ * ivt;
+    const float fz0 = (az - g.org[2] + t0 * dz) * ivz, dfz = dt * dz * ivz;
+    float s0 = 0.f, ds = 0.f, lim = 0.f;
+    if (TOF) {
+        const float tc = tbin * g.bw + g.co;
+        lim = g.nsig * g.sig + g.bw / 2;
+        s0 = (t0 - 0.5f) * len - tc;
+        ds = dt * len;
+        const float s_a = (((-lim + tc) / len + 0.5f) * dk + pk - ok) / vk;
+        const float s_b = (((lim + tc) / len + 0.5f) * dk + pk - ok) / vk;
+        i0 = max(i0, (int)floorf(fminf(s_a, s_b)) - 1);
+        i1 = min(i1, (int)ceilf(fmaxf(s_a, s_b)) + 1);
+    }
+    float4 *qa = ky ? q.qy : q.qx;
+    const int rs = nz + 1, ps = (nt + 1) * rs;
+    constexpr int PU = BACK ? 2 : 4;  // planes whose accesses are in flight together
+    for (int i = i0; i <= i1; i += PU) {
+        float w[PU], wt[PU], wz[PU];
+        bool in[PU];
+        int at[PU];
+#pragma unroll
+        for (int u = 0; u < PU; u++) {
+            const int ip = i + u;
+            w[u] = cf;
+            in[u] = ip <= i1;
+            if (TOF && in[u]) {
+                const float as = fabsf(fmaf((float)ip, ds, s0));
+                if (as > lim) {
+                    in[u] = false;
+                } else {
+                    const float t = as * g.tof_inv_step;
+                    const int m = min((int)t, kTofTab);
+                    const float t0w = tab[m], t1w = tab[m + 1];
+                    w[u] *= fmaf(t - (float)m, t1w - t0w, t0w);
+                }
+            }
+            const float ft = fmaf((float)ip, dft, ft0), fz = fmaf((float)ip, dfz, fz0);
+            const float gt = floorf(ft), gz = floorf(fz);
+            const int jt = (int)gt + 1, jz = (int)gz + 1;
+            wt[u] = ft - gt;
+            wz[u] = fz - gz;
+            in[u] = in[u] && (unsigned)jt <= (unsigned)nt && (unsigned)jz <= (unsigned)nz;
+            at[u] = ip * ps + jt * rs + jz;
+        }
+        if constexpr (BACK) {
+#pragma unroll
+            for (int u = 0; u < PU; u++) {
+                if (!in[u]) continue;
+                const float a = val * w[u], a0 = a * (1.f - wt[u]), a1 = a * wt[u];
+                atomicAdd(qa + at[u], make_float4(a0 * (1.f - wz[u]), a0 * wz[u],
+                                                  a1 * (1.f - wz[u]), a1 * wz[u]));
+            }
+        } else {
+            float4 c[PU];
+#pragma unroll
+            for (int u = 0; u < PU; u++)
+                c[u] = in[u] ? __ldg(qa + at[u]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < PU; u++) {
+                if (!in[u]) continue;
+                const float b0 = fmaf(c[u].y, wz[u], c[u].x * (1.f - wz[u]));
+                const float b1 = fmaf(c[u].w, wz[u], c[u].z * (1.f - wz[u]));
+                v = fmaf(w[u], fmaf(b1, wt[u], b0 * (1.f - wt[u])), v);
+            }
+        }
+    }
+    return true;
 }
 
 inline void tof_weight_table(float bw, float sigma, float n_sigmas, std::vector<float> &tab,

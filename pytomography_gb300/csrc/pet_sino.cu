@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(256)
     const int r = (int)(t % sg.R), slot = (int)(t / sg.R);
     float p0[3], p1[3];
     sino_lor(sg, first + slot * stride, r, p, p0, p1);
-    const float v = joseph<false, TOF>(g, p0, p1, nullptr, img, bin - g.bin_shift, 0.f);
+    const float v = joseph<false, TOF>(g, p0, p1, nullptr, img, g.tof_tab, bin - g.bin_shift, 0.f);
     proj[q] = atten ? expf(-v) : v;
 }
 
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256)
     const int r = (int)(t % sg.R), slot = (int)(t / sg.R);
     float p0[3], p1[3];
     sino_lor(sg, first + slot * stride, r, p, p0, p1);
-    joseph<true, TOF>(g, p0, p1, img, nullptr, bin - g.bin_shift, v);
+    joseph<true, TOF>(g, p0, p1, img, nullptr, g.tof_tab, bin - g.bin_shift, v);
 }
 
 // ------------------------------------------------------------- line kernels
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(256)
             } else if (firstc) {  // principal axis z: traced on its own
                 float p0[3], p1[3];
                 sino_lor(sg, a, r, p, p0, p1);
-                v = joseph<false, TOF>(g, p0, p1, nullptr, img, bin - g.bin_shift, 0.f);
+                v = joseph<false, TOF>(g, p0, p1, nullptr, img, g.tof_tab, bin - g.bin_shift, 0.f);
             }
             if (!firstc) v += out[q];
             out[q] = lastc && atten ? expf(-v) : v;
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(128)
             const float v = in[(size_t)p * nb + bin];
             float p0[3], p1[3];
             sino_lor(sg, a, r, p, p0, p1);
-            if (v != 0.f) joseph<true, TOF>(g, p0, p1, img, nullptr, bin - g.bin_shift, v);
+            if (v != 0.f) joseph<true, TOF>(g, p0, p1, img, nullptr, g.tof_tab, bin - g.bin_shift, v);
         }
     }
     const int b0 = max(l.i0, (int)(blockIdx.y * T));
