@@ -119,6 +119,8 @@ class PETLMSystemMatrix(SystemMatrix):
         _lib.check(self._lib.gb_pet_set_deterministic(self._plan, int(bool(on))))
 
     def set_n_subsets(self, n_subsets: int) -> None:
+        if self.subset_indices_array is not None and int(n_subsets) == self.n_subsets:
+            return  # the same split: indices and the plan's sorted event tiles are unchanged
         idx = torch.arange(self.proj_meta.detector_ids.shape[0]).to(torch.long).cpu()
         self.subset_indices_array = [idx[i::n_subsets] for i in range(n_subsets)]
         self.n_subsets = n_subsets
