@@ -474,6 +474,8 @@ __global__ void __launch_bounds__(256)
     k_b1_nopsf(SpectDev g, const float *__restrict__ proj, const int *__restrict__ alist,
                float *__restrict__ W) {
     constexpr int V = VEC ? 4 : 1;
+    grid_release();
+    grid_wait();
     const int slot = blockIdx.z, xp = blockIdx.y;
     const int nzv = g.nz / V;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -603,12 +605,11 @@ cudaError_t launch_b1(const SpectDev &g, const float *proj, const int *alist, in
         // a user projection pointer may not be 16-byte aligned: scalar kernel then
         if (g.nz % 4 == 0 && ((uintptr_t)proj & 15) == 0) {
             dim3 grid((g.nya * (g.nz / 4) + 255) / 256, g.Lp, n_slots);
-            k_b1_nopsf<true><<<grid, 256, 0, st>>>(g, proj, alist, W);
+            return launch_dependent(k_b1_nopsf<true>, grid, 256, 0, st, g, proj, alist, W);
         } else {
             dim3 grid((g.nya * g.nz + 255) / 256, g.Lp, n_slots);
-            k_b1_nopsf<false><<<grid, 256, 0, st>>>(g, proj, alist, W);
+            return launch_dependent(k_b1_nopsf<false>, grid, 256, 0, st, g, proj, alist, W);
         }
-        return cudaGetLastError();
     }
     if (g.strip) return launch_b1_strip(g, proj, alist, items, n_items, W, st);
     switch (g.K) {
@@ -978,6 +979,8 @@ __global__ void __launch_bounds__(256)
     k_b2_gather4(SpectDev g, const float *__restrict__ W, const int *__restrict__ alist,
                  int n_slots, float *__restrict__ out, int mode, UpdateArgs u) {
     __shared__ B2Tap tab[kB2Taps];
+    grid_release();
+    if (!g.strip) grid_wait();  // the row ranges come from the kernel before (strip: the plan)
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int x = blockIdx.z;
@@ -992,6 +995,7 @@ __global__ void __launch_bounds__(256)
         }
         __syncthreads();
     }
+    if (g.strip) grid_wait();
     const int z = z_of_pos(g, q);  // q: quad position in the W rows
     if (4 * q >= g.nzs || z >= nz || y >= N) return;
     const float4 bp = use_tab ? b2_gather_sum4_tab<kB2Unroll>(
@@ -1093,10 +1097,8 @@ cudaError_t launch_b2_gather(const SpectDev &g, const float *W, const int *alist
         const dim3 b4(packed ? qx : 32, packed ? 256 / qx : 8);
         dim3 grid((qx + b4.x - 1) / b4.x, (g.N + b4.y - 1) / b4.y, g.N);
         block = b4;
-        if (mode == B2_BSREM && u.prior)
-            k_b2_gather4<true><<<grid, block, 0, st>>>(g, W, alist, n_slots, out, mode, u);
-        else
-            k_b2_gather4<false><<<grid, block, 0, st>>>(g, W, alist, n_slots, out, mode, u);
+        return launch_dependent(mode == B2_BSREM && u.prior ? k_b2_gather4<true> : k_b2_gather4<false>,
+                                grid, block, 0, st, g, W, alist, n_slots, out, mode, u);
     } else {
         dim3 grid((g.nz + 31) / 32, (g.N + 7) / 8, g.N);
         k_b2_gather<<<grid, block, 0, st>>>(g, W, alist, n_slots, out, mode, u);
@@ -1229,6 +1231,8 @@ __global__ void __launch_bounds__(256)
     k_b2_adjoint(SpectDev g, const float *__restrict__ W, const int *__restrict__ alist,
                  int n_slots, float *__restrict__ out, int mode) {
     __shared__ AdjTable t;
+    grid_release();
+    grid_wait();
     b2_adjoint_block(g, W, alist, n_slots, (long long)blockIdx.x * 256, out, mode, t);
 }
 
@@ -1278,8 +1282,8 @@ cudaError_t launch_b2_adjoint(const SpectDev &g, const float *W, const int *alis
                               float *out, bool first, cudaStream_t st) {
     // (a list entry holds a slab offset of 31 bits)
     if ((g.zg || g.nz % 4 == 0) && (long long)g.Lp * g.nya * g.nzs < (1LL << 31)) {
-        k_b2_adjoint<<<b2_gather_blocks(g), 256, 0, st>>>(g, W, alist, n_slots, out,
-                                                          first ? B2_WRITE : B2_ADD);
+        return launch_dependent(k_b2_adjoint, b2_gather_blocks(g), 256, 0, st, g, W, alist, n_slots,
+                                out, first ? (int)B2_WRITE : (int)B2_ADD);
     } else {
         if (first) {
             cudaError_t e = cudaMemsetAsync(out, 0, (size_t)g.N * g.N * g.nz * sizeof(float), st);

@@ -32,6 +32,8 @@ __global__ void __launch_bounds__(256)
     k_fwd_nopsf(SpectDev g, const float *__restrict__ f, const int *__restrict__ alist,
                 const int4 *__restrict__ items, float *__restrict__ partials) {
     constexpr int V = VEC ? 4 : 1, PU = VEC ? 4 : 8;
+    grid_release();
+    grid_wait();
     const int4 item = items[blockIdx.x];
     const int ga = alist[item.x];
     const int N = g.N, nz = g.nz, nzv = nz / V;
@@ -93,6 +95,8 @@ __global__ void k_reduce(const int *__restrict__ ioff, int NZ, const float *__re
                          float *__restrict__ pred) {
     const int slot = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_release();
+    grid_wait();
     if (i >= NZ) return;
     const int c0 = ioff[slot], c1 = ioff[slot + 1];
     float v = 0.f;
@@ -212,12 +216,12 @@ cudaError_t launch_fwd(const SpectDev &g, const float *f, const int *alist, cons
     if (!g.psf) {
         if (g.nz % 4 == 0) {
             dim3 grid(n_items, (g.N * (g.nz / 4) + 255) / 256);
-            k_fwd_nopsf<true><<<grid, 256, 0, st>>>(g, f, alist, items, partials);
+            return launch_dependent(k_fwd_nopsf<true>, grid, 256, 0, st, g, f, alist, items, partials);
         } else {
             dim3 grid(n_items, (g.N * g.nz + 255) / 256);
-            k_fwd_nopsf<false><<<grid, 256, 0, st>>>(g, f, alist, items, partials);
+            return launch_dependent(k_fwd_nopsf<false>, grid, 256, 0, st, g, f, alist, items,
+                                    partials);
         }
-        return cudaGetLastError();
     }
     switch (g.K) {
 #define GB_FWD_CASE(KK) \
@@ -235,8 +239,8 @@ cudaError_t launch_reduce(int n_slots, const int *ioff, int NZ, const float *par
                           int ratio, const float *gproj, const float *sadd, const int *alist,
                           float *pred, cudaStream_t st) {
     dim3 grid((NZ + 255) / 256, n_slots);
-    k_reduce<<<grid, 256, 0, st>>>(ioff, NZ, partials, out, ratio, gproj, sadd, alist, pred);
-    return cudaGetLastError();
+    return launch_dependent(k_reduce, grid, 256, 0, st, ioff, NZ, partials, out, ratio, gproj, sadd,
+                            alist, pred);
 }
 
 }  // namespace gb

@@ -254,6 +254,38 @@ __device__ __forceinline__ bool plane_rows(const SpectDev &g, const float *th, i
     return ra <= rb;
 }
 
+// ---------------------------------------------------------------- dependent launches
+// The kernels of a projection follow one another on a stream, each launched while the one
+// before still runs (launch_dependent): its blocks take free SMs and set up their tables.
+// grid_wait() returns when the kernel before has finished and its writes are visible; every
+// thread calls it before it touches anything an earlier call or kernel writes (objects,
+// projections, scratch), so that completion carries over the whole chain.  Plan tables are
+// written at set-up only and may be read before.  An OSEM iteration of 8 subsets at 64^3 without
+// PSF (32 kernels of 4 to 9 us) goes from 265 to 215 us, one of 5 subsets at 101^3 x 83 from 706
+// to 668 us, at 128^3 it makes no difference.  The batch kernels keep plain launches: their
+// waves of uneven blocks ran 5% longer when blocks of the next kernel took SMs early.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launch that may start while the previous kernel of the stream runs.
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*fn)(P...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t st, A... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+}
+
 // ---------------------------------------------------------------- TMA / mbarrier
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
     return (unsigned)__cvta_generic_to_shared(p);

@@ -76,7 +76,11 @@ __device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *__
     float *taps = sm + L.taps;
     float2 *buf = reinterpret_cast<float2 *>(sm + L.bufs) + (size_t)warp * strip_buf(QL, HB);
     strip_taps(g, ga, x0, x1, taps);
-    // P with its zero halo, the warps' buffers (their z halo stays zero)
+    for (int i = lane; i < strip_buf(QL, HB) / 2; i += 32)  // the z halo stays zero
+        reinterpret_cast<float4 *>(buf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (warp == 0) strip_planes<RS>(g.planes_bwd + (size_t)ga * g.Lp, x0, x1, it);
+    grid_wait();
+    // P with its zero halo
     const bool vec = nz % 4 == 0 && ((uintptr_t)P & 15) == 0;
     for (int i = threadIdx.x; i < L.rows * QL; i += blockDim.x) {
         const int r = i / QL - L.top, z = 4 * (i % QL);
@@ -90,9 +94,6 @@ __device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *__
         if (in) v = ld_quad(p, z, nz, false);
         *reinterpret_cast<float4 *>(sm + 4 * i) = v;
     }
-    for (int i = lane; i < strip_buf(QL, HB) / 2; i += 32)
-        reinterpret_cast<float4 *>(buf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (warp == 0) strip_planes<RS>(g.planes_bwd + (size_t)ga * g.Lp, x0, x1, it);
     cp_async_wait_all();
     __syncthreads();
     const int q = lane % QL, grp = lane / QL;  // y pass: z quad, row group
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(512, 1)
     k_b1_strip(SpectDev g, const float *__restrict__ proj, const int *__restrict__ alist,
                const int4 *__restrict__ items, float *__restrict__ W) {
     extern __shared__ __align__(128) float sm[];
+    grid_release();
     const int4 item = items[blockIdx.x];
     b1_strip_item<QL, HB>(g, proj + (size_t)item.x * g.N * g.nz, alist[item.x], item.y, item.z,
                           W + (size_t)item.x * g.Lp * g.nya * g.nzs, sm);
@@ -287,6 +289,7 @@ __device__ __forceinline__ void fwd_strip_item(const SpectDev &g, const float *_
         reinterpret_cast<float4 *>(buf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (warp == 0) strip_planes<RS>(g.planes_fwd + (size_t)ga * g.Lp, x0, x1, it);
     cp_async_wait_all();
+    grid_wait();
     __syncthreads();
     float th[6];
 #pragma unroll
@@ -373,6 +376,7 @@ __global__ void __launch_bounds__(512, 1)
     k_fwd_strip(SpectDev g, const float *__restrict__ f, const int *__restrict__ alist,
                 const int4 *__restrict__ items, float *__restrict__ W) {
     extern __shared__ __align__(128) float sm[];
+    grid_release();
     const int4 item = items[blockIdx.x];
     fwd_strip_item<QL, HB>(g, f, alist[item.x], item.y, item.z,
                            W + (size_t)item.x * g.Lp * g.nya * 32 * strip_slabs(g), sm);
@@ -441,6 +445,7 @@ __device__ __forceinline__ void ysum_item(const SpectDev &g, const float *__rest
     if (threadIdx.x < 32) sm[L.zero + threadIdx.x] = 0.f;
     if (warp == 0) strip_planes<0>(g.planes_fwd + (size_t)ga * g.Lp, x0, x1, it);
     cp_async_wait_all();
+    grid_wait();
     __syncthreads();
     const int np = it->n_planes;
     if (warp >= nw) {
@@ -521,6 +526,7 @@ __global__ void __launch_bounds__(160, 4)
                const float *__restrict__ W, float *__restrict__ partials) {
     extern __shared__ __align__(128) float sm[];
     __shared__ unsigned long long full[kYStages], empty[kYStages];
+    grid_release();
     const int4 item = items[blockIdx.x];
     ysum_item(g, W + (size_t)item.x * g.Lp * g.nya * 32 * strip_slabs(g), alist[item.x], item.y,
               item.z, blockIdx.y, partials + (size_t)blockIdx.x * g.N * g.nz, sm, full, empty);
@@ -564,17 +570,17 @@ cudaError_t launch_fwd_strip(const SpectDev &g, const float *f, const int *alist
                              float *W, float *partials, cudaStream_t st) {
     const int QL = strip_ql(g.nz), HB = strip_halo(g);
     const size_t smem = fwd_strip_layout(QL, HB, g.strip_fwd).total * sizeof(float);
+    cudaError_t e = cudaErrorInvalidValue;
 #define GB_CASE(Q, B)                                                                        \
     if (QL == Q && HB == B)                                                                  \
-        k_fwd_strip<Q, B><<<n_items, 32 * g.strip_fwd, smem, st>>>(g, f, alist, items, W);
+        e = launch_dependent(k_fwd_strip<Q, B>, n_items, 32 * g.strip_fwd, smem, st, g, f,    \
+                             alist, items, W);
     GB_FOR_EACH_STRIP(GB_CASE)
 #undef GB_CASE
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const dim3 grid(n_yitems, strip_slabs(g));
-    k_fwd_ysum<<<grid, 32 * ((g.N + 31) / 32 + 1), ysum_layout(g).total * sizeof(float), st>>>(
-        g, alist, yitems, W, partials);
-    return cudaGetLastError();
+    return launch_dependent(k_fwd_ysum, dim3(n_yitems, strip_slabs(g)),
+                            32 * ((g.N + 31) / 32 + 1), ysum_layout(g).total * sizeof(float), st, g,
+                            alist, yitems, W, partials);
 }
 
 cudaError_t launch_b1_strip(const SpectDev &g, const float *proj, const int *alist,
@@ -583,10 +589,11 @@ cudaError_t launch_b1_strip(const SpectDev &g, const float *proj, const int *ali
     const size_t smem = b1_strip_layout(g, QL, warps).total * sizeof(float);
 #define GB_CASE(Q, B)                                                                        \
     if (QL == Q && HB == B)                                                                  \
-        k_b1_strip<Q, B><<<n_items, 32 * warps, smem, st>>>(g, proj, alist, items, W);
+        return launch_dependent(k_b1_strip<Q, B>, n_items, 32 * warps, smem, st, g, proj,     \
+                                alist, items, W);
     GB_FOR_EACH_STRIP(GB_CASE)
 #undef GB_CASE
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 // The strip entries of a batch: those with g.strip > 0 (the others have no item here).
