@@ -16,12 +16,6 @@
 
 namespace gb {
 
-// The TOF weight table into shared memory (whole block).
-__device__ __forceinline__ void load_tof_table(const PetDev &g, float *tab) {
-    for (int i = threadIdx.x; i < kTofTab + 2; i += blockDim.x) tab[i] = __ldg(g.tof_tab + i);
-    __syncthreads();
-}
-
 // Event tiles: the events of a list (every event, or one subset i::n) sorted by a
 // locality key, packed as {id1, id2, centred TOF bin, j} where j is the event's position
 // in the list (event index first + j * stride).  Threads of a warp then trace nearby,
@@ -36,8 +30,11 @@ __global__ void __launch_bounds__(256)
               long long n, const float *__restrict__ img, PetPatches pq, float *__restrict__ out,
               int ratio, const float *__restrict__ sadd, const float *__restrict__ gnum,
               int gnum_len) {
-    __shared__ float tab[TOF ? kTofTab + 2 : 1];
-    if (TOF) load_tof_table(g, tab);
+    __shared__ __align__(16) float tab[TOF ? kTofTabLen : 4];
+    if (TOF) {
+        copy_tof_table(g, tab);
+        __syncthreads();
+    }
     long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int4 r = rec[k];
@@ -62,8 +59,11 @@ template <bool TOF, bool PATCH>
 __global__ void __launch_bounds__(256)
     k_pet_bwd(PetDev g, const int4 *__restrict__ rec, long long n,
               const float *__restrict__ proj, int sorted, float *__restrict__ img, PetPatches pq) {
-    __shared__ float tab[TOF ? kTofTab + 2 : 1];
-    if (TOF) load_tof_table(g, tab);
+    __shared__ __align__(16) float tab[TOF ? kTofTabLen : 4];
+    if (TOF) {
+        copy_tof_table(g, tab);
+        __syncthreads();
+    }
     long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int4 r = rec[k];

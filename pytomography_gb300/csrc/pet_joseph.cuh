@@ -30,6 +30,7 @@ namespace gb {
 // in double on the host; linear interpolation in |s| (error below 1e-7 of the peak
 // weight at the benchmark's sigma, bin width and n_sigmas).
 constexpr int kTofTab = 4096;
+constexpr int kTofTabLen = kTofTab + 4;  // with guards: whole 16-byte pieces
 
 // Host: the table for bin width bw, sigma and n_sigmas, and kTofTab / lim.
 inline void tof_weight_table(float bw, float sigma, float n_sigmas, std::vector<float> &tab,
@@ -44,9 +45,18 @@ struct PetDev {
     int tof;
     float bw, sig, co, nsig;
     int bin_shift;
-    const float *tof_tab;  // [kTofTab + 2]
+    const float *tof_tab;  // [kTofTabLen]
     float tof_inv_step;    // kTofTab / lim
 };
+
+// The TOF weight table into shared memory (16-byte aligned; by the whole block, which
+// synchronises afterwards).
+__device__ __forceinline__ void copy_tof_table(const PetDev &g, float *tab) {
+    const float4 *src = reinterpret_cast<const float4 *>(g.tof_tab);
+    float4 *dst = reinterpret_cast<float4 *>(tab);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < kTofTabLen / 4; i += blockDim.x) dst[i] = __ldg(src + i);
+}
 
 __device__ __forceinline__ float pick(float a, float b, float c, int k) {
     return k == 0 ? a : (k == 1 ? b : c);
@@ -369,12 +379,12 @@ inline void tof_weight_table(float bw, float sigma, float n_sigmas, std::vector<
                              float &inv_step) {
     const double h = 0.5 * bw, q = 1.0 / (std::sqrt(2.0) * sigma);
     const double lim = (double)n_sigmas * sigma + h;
-    tab.assign(kTofTab + 2, 0.f);
+    tab.assign(kTofTabLen, 0.f);
     for (int m = 0; m <= kTofTab; m++) {
         const double x = lim * m / kTofTab;
         tab[m] = (float)(0.5 * (std::erfc((x - h) * q) - std::erfc((x + h) * q)));
     }
-    tab[kTofTab + 1] = tab[kTofTab];
+    for (int m = kTofTab + 1; m < kTofTabLen; m++) tab[m] = tab[kTofTab];
     inv_step = (float)(kTofTab / lim);
 }
 

@@ -165,13 +165,12 @@ template <bool TOF>
 __global__ void __launch_bounds__(256)
     k_sino_fwd_line(PetDev g, SinoGeom sg, int first, int stride, int nb, int chunk,
                     const float *__restrict__ img, float *__restrict__ proj, int atten) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     const int line = blockIdx.x, a = first + (line / sg.R) * stride, r = line % sg.R;
     const Line l = sino_line(g, sg, a, r);
     const int nz = g.n[2], zs = nz + 2;  // one zero below and above each column
-    float *tab = sm + (size_t)chunk * zs;
-    if (TOF)
-        for (int i = threadIdx.x; i < kTofTab + 2; i += blockDim.x) tab[i] = g.tof_tab[i];
+    float *tab = sm + ((size_t)chunk * zs + 3) / 4 * 4;
+    if (TOF) copy_tof_table(g, tab);
     const int per = (sg.P + gridDim.y - 1) / gridDim.y;
     const int pa = blockIdx.y * per, pb = min(sg.P, pa + per);
     const int nq = (pb - pa) * nb;  // (ring pair, bin) elements of this CTA
@@ -247,7 +246,7 @@ template <bool TOF>
 __global__ void __launch_bounds__(128)
     k_sino_bwd_line(PetDev g, SinoGeom sg, int first, int stride, int nb,
                     const float *__restrict__ proj, float *__restrict__ img) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     const int line = blockIdx.x, a = first + (line / sg.R) * stride, r = line % sg.R;
     const Line l = sino_line(g, sg, a, r);
     const int nz = g.n[2], T = blockDim.x, tid = threadIdx.x;
@@ -272,8 +271,7 @@ __global__ void __launch_bounds__(128)
     float *vals = reinterpret_cast<float *>(lor + kLineBatch);  // TOF: [kLineBatch][nb]
     float *tab = vals + kLineBatch * nb;
     for (int i = tid; i < (nz + 2) * T; i += T) prof[i] = 0.f;
-    if (TOF)
-        for (int i = tid; i < kTofTab + 2; i += T) tab[i] = g.tof_tab[i];
+    if (TOF) copy_tof_table(g, tab);
     const int i = blockIdx.y * T + tid;
     const float f = fmaf((float)i, l.df, l.f0), fl = floorf(f);
     const int j = (int)fl;
@@ -403,14 +401,15 @@ struct gb_pet_sino_plan {
 // Shared memory of the line kernels, raised once per process and device context.
 static size_t bwd_line_smem(int nz, int T, int nb, bool tof) {
     return sizeof(float) * (((size_t)(nz + 2) * T + 3) / 4 * 4 + 4 * kLineBatch +
-                            (tof ? kLineBatch * nb + kTofTab + 2 : 0));
+                            (tof ? kLineBatch * nb + kTofTabLen : 0));
 }
 static int fwd_line_chunk(const PetDev &g) {  // planes staged at a time
     const int nk = std::max(g.n[0], g.n[1]), zs = g.n[2] + 2;
     return std::max(1, std::min(nk, (int)(kLineStage / (sizeof(float) * zs))));
 }
 static size_t fwd_line_smem(const PetDev &g, bool tof) {
-    return sizeof(float) * ((size_t)fwd_line_chunk(g) * (g.n[2] + 2) + (tof ? kTofTab + 2 : 0));
+    return sizeof(float) * (((size_t)fwd_line_chunk(g) * (g.n[2] + 2) + 3) / 4 * 4 +
+                            (tof ? kTofTabLen : 0));
 }
 // The line kernels need the profiles of 128 planes (and the TOF table and values) in shared
 // memory: up to 390 slices.
