@@ -409,8 +409,11 @@ static gb_status build_tiles(gb_pet_plan *p, int n_subsets) {
 //   100 x 100 x 48, 13 TOF bins      29 -> 31     40 -> 35    89 -> 67    237 -> 161
 //                                    40 -> 36     87 -> 50    215 -> 98   542 -> 218
 // The forward, bound by the L1 lines its lanes touch (one per plane instead of up to four),
-// breaks even near 2.8 planes per voxel, the back projection near 1.
+// breaks even near 2.8 planes per voxel, the back projection near 1.  Below about 40k LORs the
+// forward is bound by latency, which the patches leave as it is, and the launch that builds
+// them costs 1.5-2 us more (77 x 77 x 35, no TOF, 32k LORs: 27.1 -> 28.6 us).
 constexpr double kPatchFwd = 2.8, kPatchBwd = 1.0;
+constexpr long long kPatchFwdMin = 40000;
 static bool patch_pays(const PetDev &g, double n, bool tof, double planes_per_voxel) {
     double planes = 0.6 * std::max(g.n[0], g.n[1]);
     if (tof) {
@@ -455,7 +458,7 @@ static cudaError_t pet_forward(const gb_pet_plan *p, const int4 *rec, long long 
                                int ratio, const float *sadd, const float *gnum, int gnum_len,
                                bool tof, cudaStream_t st) {
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    const bool patch = use_patches(p, n, tof, kPatchFwd);
+    const bool patch = n >= kPatchFwdMin && use_patches(p, n, tof, kPatchFwd);
     if (patch) {
         cudaError_t e = build_patches(p, img, st);
         if (e != cudaSuccess) return e;

@@ -21,6 +21,11 @@ CASES = [
     ((16, 16, 1), (8.0, 8.0, 8.0), 32, 2, 90.0, 8, 4000, 1),
     ((12, 12, 33), (6.0, 6.0, 4.0), 16, 40, 50.0, 0, 8000, 1),   # steep LORs
     ((33, 40, 5), (4.0, 3.0, 4.0), 48, 4, 90.0, 13, 9000, 60),   # subsets below the rule
+    # the smallest lists that the forward takes the layout for, and one event less
+    ((21, 30, 7), (6.0, 4.0, 4.0), 40, 8, 90.0, 0, 40000, 1),
+    ((31, 20, 8), (4.0, 6.0, 4.0), 40, 8, 90.0, 9, 80001, 2),
+    ((16, 15, 1), (8.0, 8.0, 8.0), 32, 2, 90.0, 8, 39999, 1),
+    ((12, 13, 33), (6.0, 6.0, 4.0), 16, 40, 50.0, 13, 40001, 1),
 ]
 
 
