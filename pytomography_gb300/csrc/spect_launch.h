@@ -61,6 +61,11 @@ cudaError_t launch_b1_strip(const SpectDev &g, const float *proj, const int *ali
                             const int4 *items, int n_items, float *W, cudaStream_t st);
 cudaError_t launch_b2_gather(const SpectDev &g, const float *W, const int *alist, int n_slots,
                              float *out, int mode, const UpdateArgs &u, cudaStream_t st);
+// Plans without PSF: B1 and the gather in one kernel.  It takes whole z quads, 16-byte aligned
+// projections and blocks whose sample table fits; other calls run B1 and the gather.
+bool b2_nopsf_ok(const SpectDev &g, const float *proj, int n_slots);
+cudaError_t launch_b2_nopsf(const SpectDev &g, const float *proj, const int *alist, int n_slots,
+                            float *out, int mode, const UpdateArgs &u, cudaStream_t st);
 cudaError_t launch_b2_adjoint(const SpectDev &g, const float *W, const int *alist, int n_slots,
                               float *out, bool first, cudaStream_t st);
 cudaError_t launch_atten(const SpectDev &g, const float *mu, float dx, int n_angles, float *A,

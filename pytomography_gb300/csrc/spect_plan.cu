@@ -1015,8 +1015,14 @@ static gb_status run_backward(gb_spect_plan *p, const float *proj, int li, int a
     const int n_groups = (n + p->G - 1) / p->G;
     for (int gi = 0; gi < n_groups; gi++) {
         int a0 = gi * p->G, na = std::min(p->G, n - a0);
-        GB_CUDA(launch_b1(p->dev, proj + a0 * NZ, alist + a0, na, p->d_items + L.gitem_off[gi],
-                          L.n_gitems[gi], p->Zt_b1, p->d_W, st));
+        const bool fused = !adjoint && b2_nopsf_ok(p->dev, proj + a0 * NZ, na);
+        if (!fused)
+            GB_CUDA(launch_b1(p->dev, proj + a0 * NZ, alist + a0, na, p->d_items + L.gitem_off[gi],
+                              L.n_gitems[gi], p->Zt_b1, p->d_W, st));
+        auto gather = [&](float *dst, int mode, const UpdateArgs &a) {
+            return fused ? launch_b2_nopsf(p->dev, proj + a0 * NZ, alist + a0, na, dst, mode, a, st)
+                         : launch_b2_gather(p->dev, p->d_W, alist + a0, na, dst, mode, a, st);
+        };
         if (adjoint) {
             GB_CUDA(launch_b2_adjoint(p->dev, p->d_W, alist + a0, na, out, gi == 0, st));
             continue;
@@ -1026,11 +1032,10 @@ static gb_status run_backward(gb_spect_plan *p, const float *proj, int li, int a
         if (!last || final_mode == B2_WRITE) {
             // accumulate into `out` (plain backward) or the bp scratch (fused updates)
             float *dst = final_mode == B2_WRITE ? out : p->d_bp;
-            GB_CUDA(launch_b2_gather(p->dev, p->d_W, alist + a0, na, dst,
-                                     gi == 0 ? B2_WRITE : B2_ADD, ua, st));
+            GB_CUDA(gather(dst, gi == 0 ? B2_WRITE : B2_ADD, ua));
         } else {
             u.acc = n_groups > 1 ? p->d_bp : nullptr;
-            GB_CUDA(launch_b2_gather(p->dev, p->d_W, alist + a0, na, out, final_mode, u, st));
+            GB_CUDA(gather(out, final_mode, u));
         }
     }
     return GB_OK;
