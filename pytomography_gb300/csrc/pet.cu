@@ -7,6 +7,7 @@
 // (TOF bin centring by (num_bins - 1) // 2 at :280).
 #include <algorithm>
 #include <cmath>
+#include <mutex>
 #include <vector>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -308,8 +309,13 @@ struct gb_pet_plan {
     unsigned long long *d_acc64 = nullptr;
     unsigned *d_maxbits = nullptr;
     float *d_scale = nullptr;
-    // patch layout (pet_joseph.cuh), null where it cannot pay
-    PetPatches patch{};
+    // patch layouts (pet_joseph.cuh), null where they cannot pay: the fused step's, and the
+    // other calls', which take turns (PatchLease)
+    PetPatches osem_patch{}, call_patch{};
+    std::mutex call_lock;
+    cudaEvent_t call_done = nullptr;  // end of the layout's last use
+    cudaStream_t call_stream = nullptr;
+    bool call_used = false;
 };
 
 static void pet_free(gb_pet_plan *p) {
@@ -323,8 +329,11 @@ static void pet_free(gb_pet_plan *p) {
     dev_free(p->d_acc64);
     dev_free(p->d_maxbits);
     dev_free(p->d_scale);
-    dev_free(p->patch.qx);
-    dev_free(p->patch.qy);
+    for (const PetPatches &q : {p->osem_patch, p->call_patch}) {
+        dev_free(q.qx);
+        dev_free(q.qy);
+    }
+    if (p->call_done) cudaEventDestroy(p->call_done);
     delete p;
 }
 
@@ -422,69 +431,109 @@ static bool patch_pays(const PetDev &g, double n, bool tof, double planes_per_vo
     }
     return n * planes > planes_per_voxel * (double)g.n_vox;
 }
-// The largest patch layout a plan keeps.
-constexpr size_t kPatchMaxBytes = (size_t)2 << 30;
+// The largest patch layouts a plan keeps, in all.
+constexpr size_t kPatchMaxBytes = (size_t)4 << 30;
 
-static bool use_patches(const gb_pet_plan *p, long long n, bool tof, double planes_per_voxel) {
-    return p->patch.qx && patch_pays(p->dev, (double)n, tof, planes_per_voxel);
+static bool fwd_patches_pay(const PetDev &g, long long n, bool tof) {
+    return n >= kPatchFwdMin && patch_pays(g, (double)n, tof, kPatchFwd);
 }
 
-static cudaError_t build_patches(const gb_pet_plan *p, const float *img, cudaStream_t st) {
+// Forward and back projections of one plan may run on several streams and threads at once, so
+// the layout they share is lent to one at a time: the host lock is held while a call enqueues
+// its kernels, and a call on another stream than the last one's waits for that one's end.  A
+// capturing stream cannot wait for outside work (and its graph would not take turns later):
+// there, and where the plan has no layout, `q` stays null and the call goes without.
+struct PatchLease {
+    PetPatches q{};
+    PatchLease(gb_pet_plan *p, bool want, cudaStream_t st) : plan(p), st(st) {
+        if (!want || !p->call_patch.qx) return;
+        cudaStreamCaptureStatus cs;
+        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        if (cs != cudaStreamCaptureStatusNone) return;
+        p->call_lock.lock();
+        if (p->call_used && p->call_stream != st &&
+            cudaStreamWaitEvent(st, p->call_done) != cudaSuccess) {
+            cudaGetLastError();
+            p->call_lock.unlock();
+            return;
+        }
+        q = p->call_patch;
+    }
+    ~PatchLease() {
+        if (!q.qx) return;
+        cudaEventRecord(plan->call_done, st);
+        plan->call_stream = st;
+        plan->call_used = true;
+        plan->call_lock.unlock();
+    }
+    PatchLease(const PatchLease &) = delete;
+    PatchLease &operator=(const PatchLease &) = delete;
+
+   private:
+    gb_pet_plan *plan;
+    cudaStream_t st;
+};
+
+static cudaError_t build_patches(const gb_pet_plan *p, const PetPatches &q, const float *img,
+                                 cudaStream_t st) {
     const PetDev &g = p->dev;
     const dim3 grid(((g.n[1] + 1) * (g.n[2] + 1) + 255) / 256, (g.n[0] + kBuildX) / kBuildX);
-    k_patch_build<<<grid, 256, 0, st>>>(g, img, p->patch);
+    k_patch_build<<<grid, 256, 0, st>>>(g, img, q);
     return cudaGetLastError();
 }
-static cudaError_t clear_patches(const gb_pet_plan *p, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(p->patch.qx, 0, patch_elems_x(p->dev) * sizeof(float4), st);
+static cudaError_t clear_patches(const gb_pet_plan *p, const PetPatches &q, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(q.qx, 0, patch_elems_x(p->dev) * sizeof(float4), st);
     if (e != cudaSuccess) return e;
-    return cudaMemsetAsync(p->patch.qy, 0, patch_elems_y(p->dev) * sizeof(float4), st);
+    return cudaMemsetAsync(q.qy, 0, patch_elems_y(p->dev) * sizeof(float4), st);
 }
 // img += patches, or (f) the OSEM update of f with bp = img + patches
-static cudaError_t fold_patches(const gb_pet_plan *p, float *img, float *f, const float *nbp,
-                                cudaStream_t st) {
+static cudaError_t fold_patches(const gb_pet_plan *p, const PetPatches &q, float *img, float *f,
+                                const float *nbp, cudaStream_t st) {
     const PetDev &g = p->dev;
     const dim3 block(32, 8), grid((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]);
     if (f)
-        k_patch_fold<true><<<grid, block, 0, st>>>(g, p->patch, img, f, nbp);
+        k_patch_fold<true><<<grid, block, 0, st>>>(g, q, img, f, nbp);
     else
-        k_patch_fold<false><<<grid, block, 0, st>>>(g, p->patch, img, nullptr, nullptr);
+        k_patch_fold<false><<<grid, block, 0, st>>>(g, q, img, nullptr, nullptr);
     return cudaGetLastError();
 }
 
-// Forward projection of n tiles (k_pet_fwd's outputs), building the patch layout if it pays.
-static cudaError_t pet_forward(const gb_pet_plan *p, const int4 *rec, long long first,
-                               long long stride, long long n, const float *img, float *out,
-                               int ratio, const float *sadd, const float *gnum, int gnum_len,
-                               bool tof, cudaStream_t st) {
+// Forward projection of n tiles (k_pet_fwd's outputs), by way of the patch layout q if not null.
+static cudaError_t pet_forward(const gb_pet_plan *p, const PetPatches &q, const int4 *rec,
+                               long long first, long long stride, long long n, const float *img,
+                               float *out, int ratio, const float *sadd, const float *gnum,
+                               int gnum_len, bool tof, cudaStream_t st) {
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    const bool patch = n >= kPatchFwdMin && use_patches(p, n, tof, kPatchFwd);
+    const bool patch = q.qx;
     if (patch) {
-        cudaError_t e = build_patches(p, img, st);
+        cudaError_t e = build_patches(p, q, img, st);
         if (e != cudaSuccess) return e;
     }
     auto *fn = tof ? (patch ? k_pet_fwd<true, true> : k_pet_fwd<true, false>)
                    : (patch ? k_pet_fwd<false, true> : k_pet_fwd<false, false>);
-    fn<<<blocks, 256, 0, st>>>(p->dev, rec, first, stride, n, img, p->patch, out, ratio, sadd, gnum,
+    fn<<<blocks, 256, 0, st>>>(p->dev, rec, first, stride, n, img, q, out, ratio, sadd, gnum,
                                gnum_len);
     return cudaGetLastError();
 }
 
-// Back projection of n tiles into img, which is cleared first; f: followed by the OSEM update
-// of f (img is then scratch).
-static cudaError_t pet_backward(const gb_pet_plan *p, const int4 *rec, long long n,
-                                const float *proj, int sorted, float *img, float *f,
+// Back projection of n tiles into img, which is cleared first, by way of the patch layout q if
+// not null; f: followed by the OSEM update of f (img is then scratch).
+static cudaError_t pet_backward(const gb_pet_plan *p, const PetPatches &q, const int4 *rec,
+                                long long n, const float *proj, int sorted, float *img, float *f,
                                 const float *nbp, cudaStream_t st) {
-    const bool tof = p->dev.tof, patch = use_patches(p, n, tof, kPatchBwd);
+    const bool tof = p->dev.tof, patch = q.qx;
     cudaError_t e = cudaMemsetAsync(img, 0, (size_t)p->img_size * sizeof(float), st);
-    if (e == cudaSuccess && patch) e = clear_patches(p, st);
+    if (e == cudaSuccess && patch) e = clear_patches(p, q, st);
     if (e != cudaSuccess) return e;
     if (n > 0) {
         auto *fn = tof ? (patch ? k_pet_bwd<true, true> : k_pet_bwd<true, false>)
                        : (patch ? k_pet_bwd<false, true> : k_pet_bwd<false, false>);
-        fn<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p->dev, rec, n, proj, sorted, img, p->patch);
+        fn<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p->dev, rec, n, proj, sorted, img, q);
     }
-    if (patch) return fold_patches(p, img, f, nbp, st);
+    if (patch) return fold_patches(p, q, img, f, nbp, st);
     if (f)
         k_pet_update<<<(unsigned)((p->img_size + 255) / 256), 256, 0, st>>>(f, img, nbp,
                                                                             p->img_size);
@@ -570,14 +619,21 @@ gb_status gb_pet_plan_create(const gb_pet_desc *d, gb_pet_plan **out) {
                 }
             }
     }
-    // patch layout where the longest list, or a sensitivity image of as many LORs, pays for it
+    // patch layouts where the longest list, or a sensitivity image of as many LORs, pays for
+    // them; without the memory for them the plan does without
     const size_t pb = (patch_elems_x(g) + patch_elems_y(g)) * sizeof(float4);
-    if (pb <= kPatchMaxBytes && patch_pays(g, (double)d->n_events, d->tof, kPatchBwd)) {
-        if ((e = dev_alloc(&p->patch.qx, patch_elems_x(g) * sizeof(float4))) != cudaSuccess ||
-            (e = dev_alloc(&p->patch.qy, patch_elems_y(g) * sizeof(float4))) != cudaSuccess) {
-            set_error("patch layout allocation failed: %s", cudaGetErrorString(e));
+    if (2 * pb <= kPatchMaxBytes && patch_pays(g, (double)d->n_events, d->tof, kPatchBwd)) {
+        for (PetPatches *q : {&p->osem_patch, &p->call_patch})
+            if (dev_alloc(&q->qx, patch_elems_x(g) * sizeof(float4)) != cudaSuccess ||
+                dev_alloc(&q->qy, patch_elems_y(g) * sizeof(float4)) != cudaSuccess) {
+                dev_free(q->qx);
+                *q = PetPatches{};
+                cudaGetLastError();
+            }
+        if ((e = cudaEventCreateWithFlags(&p->call_done, cudaEventDisableTiming)) != cudaSuccess) {
+            set_error("event creation failed: %s", cudaGetErrorString(e));
             pet_free(p);
-            return e == cudaErrorMemoryAllocation ? GB_ERR_OOM : GB_ERR_CUDA;
+            return GB_ERR_CUDA;
         }
     }
     gb_status st = build_tiles(p, 1);
@@ -617,8 +673,9 @@ gb_status gb_pet_forward(gb_pet_plan *p, const float *img, float *proj, int32_t 
     long long first, stride, n;
     subset_range(p, subset, first, stride, n);
     if (n == 0) return GB_OK;
-    GB_CUDA(pet_forward(p, list_tiles(p, subset), first, stride, n, img, proj, 0, nullptr, nullptr,
-                        0, p->dev.tof, as_stream(stream)));
+    PatchLease lease(p, fwd_patches_pay(p->dev, n, p->dev.tof), as_stream(stream));
+    GB_CUDA(pet_forward(p, lease.q, list_tiles(p, subset), first, stride, n, img, proj, 0, nullptr,
+                        nullptr, 0, p->dev.tof, as_stream(stream)));
     return GB_OK;
 }
 
@@ -654,7 +711,8 @@ gb_status gb_pet_backward(gb_pet_plan *p, const float *proj, float *img, int32_t
         GB_LAUNCH_CHECK();
         return GB_OK;
     }
-    GB_CUDA(pet_backward(p, rec, n, proj, 0, img, nullptr, nullptr, st));
+    PatchLease lease(p, patch_pays(p->dev, (double)n, p->dev.tof, kPatchBwd), st);
+    GB_CUDA(pet_backward(p, lease.q, rec, n, proj, 0, img, nullptr, nullptr, st));
     return GB_OK;
 }
 
@@ -688,10 +746,14 @@ gb_status gb_pet_osem_step(gb_pet_plan *p, float *img, const float *numerator,
     subset_range(p, subset, first, stride, n);
     cudaStream_t st = as_stream(stream);
     const int4 *rec = list_tiles(p, subset);
+    const bool tof = p->dev.tof;
+    const PetPatches none{};
     if (n > 0)
-        GB_CUDA(pet_forward(p, rec, first, stride, n, img, p->d_ratio, 1, additive, numerator,
-                            (int)numerator_len, p->dev.tof, st));
-    GB_CUDA(pet_backward(p, rec, n, p->d_ratio, 1, p->d_bp, img, norm_bp, st));
+        GB_CUDA(pet_forward(p, fwd_patches_pay(p->dev, n, tof) ? p->osem_patch : none, rec, first,
+                            stride, n, img, p->d_ratio, 1, additive, numerator, (int)numerator_len,
+                            tof, st));
+    GB_CUDA(pet_backward(p, patch_pays(p->dev, (double)n, tof, kPatchBwd) ? p->osem_patch : none,
+                         rec, n, p->d_ratio, 1, p->d_bp, img, norm_bp, st));
     return GB_OK;
 }
 
@@ -706,17 +768,18 @@ gb_status gb_pet_sensitivity(gb_pet_plan *p, const int32_t *pairs, int64_t n_pai
     GB_CHECK_ARG(n_pairs >= 0, "negative pair count");
     cudaStream_t st = as_stream(stream);
     GB_CUDA(cudaMemsetAsync(img, 0, (size_t)p->img_size * sizeof(float), st));
-    const bool patch = use_patches(p, n_pairs, false, kPatchBwd);
-    if (patch) GB_CUDA(clear_patches(p, st));
+    PatchLease lease(p, patch_pays(p->dev, (double)n_pairs, false, kPatchBwd), st);
+    const bool patch = lease.q.qx;
+    if (patch) GB_CUDA(clear_patches(p, lease.q, st));
     const long long chunk = 1LL << 28;  // launch in chunks of 2^28 LORs
     for (long long first = 0; first < n_pairs; first += chunk) {
         long long n = std::min(chunk, (long long)n_pairs - first);
         auto *fn = patch ? k_pet_sens<true> : k_pet_sens<false>;
-        fn<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p->dev, p->patch, pairs, first, n, weights,
+        fn<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p->dev, lease.q, pairs, first, n, weights,
                                                         mu, add, img);
         GB_LAUNCH_CHECK();
     }
-    if (patch) GB_CUDA(fold_patches(p, img, nullptr, nullptr, st));
+    if (patch) GB_CUDA(fold_patches(p, lease.q, img, nullptr, nullptr, st));
     return GB_OK;
 }
 
@@ -728,8 +791,10 @@ gb_status gb_pet_lor_forward(gb_pet_plan *p, const float *img, float *proj, int3
     long long first, stride, n;
     subset_range(p, subset, first, stride, n);
     if (n == 0) return GB_OK;
-    GB_CUDA(pet_forward(p, list_tiles(p, subset), first, stride, n, img, proj, 0, nullptr, nullptr,
-                        0, use_tof && p->dev.tof, as_stream(stream)));
+    const bool tof = use_tof && p->dev.tof;
+    PatchLease lease(p, fwd_patches_pay(p->dev, n, tof), as_stream(stream));
+    GB_CUDA(pet_forward(p, lease.q, list_tiles(p, subset), first, stride, n, img, proj, 0, nullptr,
+                        nullptr, 0, tof, as_stream(stream)));
     return GB_OK;
 }
 

@@ -201,7 +201,8 @@ struct gb_spect_plan {
     // scratch
     float *d_partials = nullptr;
     size_t partials_cap = 0;
-    float *d_W = nullptr;
+    float *d_W = nullptr;   // back projection
+    float *d_Wf = nullptr;  // strip plans: forward (a call of each may run at the same time)
     int G = 0;
     float *d_ratio = nullptr, *d_bp = nullptr;
     int2 *d_wrange = nullptr;
@@ -228,7 +229,7 @@ static void free_plan(gb_spect_plan *p) {
     dev_free(p->d_staps);
     dev_free(p->dev.phase);
     dev_free(p->d_alist); dev_free(p->d_items); dev_free(p->d_ioff);
-    dev_free(p->d_partials); dev_free(p->d_W); dev_free(p->d_ratio);
+    dev_free(p->d_partials); dev_free(p->d_W); dev_free(p->d_Wf); dev_free(p->d_ratio);
     dev_free(p->d_bp);
     dev_free(p->d_wrange);
     dev_free(p->d_err);
@@ -766,6 +767,7 @@ gb_status gb_spect_plan_create(const gb_spect_desc *d, gb_spect_plan **out) {
     // scratch: W for one angle group, likelihood ratio of all angles, multi-group bp
     p->G = std::min(n, 16);
     FAIL_CUDA(dev_alloc(&p->d_W, p->G * stack_slot(g) * sizeof(float)));
+    if (g.strip) FAIL_CUDA(dev_alloc(&p->d_Wf, p->G * stack_slot(g) * sizeof(float)));
     FAIL_CUDA(dev_alloc(&p->d_ratio, (size_t)n * p->N * p->nz * sizeof(float)));
     FAIL_CUDA(dev_alloc(&p->d_bp, (size_t)p->N * p->N * p->nz * sizeof(float)));
     FAIL_CUDA(dev_alloc(&p->d_wrange, (size_t)p->G * Lp * sizeof(int2)));
@@ -971,7 +973,7 @@ static cudaError_t launch_fwd_group(gb_spect_plan *p, const gb_spect_plan::FwdGr
     if (p->dev.strip) {
         const int g0 = half == 1 ? F.gather_half : 0, g1 = half == 0 ? F.gather_half : F.n_gather;
         return launch_fwd_strip(p->dev, obj, alist, p->d_items + F.gather_off + g0, g1 - g0, items,
-                                i1 - i0, p->d_W, partials, st);
+                                i1 - i0, p->d_Wf, partials, st);
     }
     return launch_fwd(p->dev, obj, alist, items, i1 - i0, p->Zt_fwd, p->fwd_tpb, partials, st);
 }

@@ -80,3 +80,43 @@ def test_patch_layout_matches_oracle(case, cuda):
     bp = o.backward(1 / (o.forward(img, es) + 0.3 + 1e-11), es)
     ref = np.maximum(img + img / (nb + 1e-11) * (bp - nb), 0)
     assert rel_l2(f.cpu().numpy(), ref) < TOL
+
+
+def test_calls_on_two_streams_take_turns(cuda):
+    """Forward and back projections of one plan enqueued on two streams, and a forward recorded
+    in a graph, give what one stream gives (1e-5: the additions' order differs)."""
+    from pytomography_gb300.metadata import ObjectMeta
+    from pytomography_gb300.metadata.PET import PETLMProjMeta
+    from pytomography_gb300.projectors.PET import PETLMSystemMatrix
+    nt, nr, n, shape = 64, 16, 200_000, (60, 60, 24)
+    info = dict(crystalTransNr=1, crystalTransSpacing=4.0, submoduleTransNr=1,
+                submoduleTransSpacing=0.0, moduleTransNr=1, moduleTransSpacing=0.0,
+                rsectorTransNr=nt, crystalAxialNr=nr, crystalAxialSpacing=4.0,
+                submoduleAxialNr=1, submoduleAxialSpacing=0.0, moduleAxialNr=1,
+                moduleAxialSpacing=0.0, rsectorAxialNr=1, radius=150.0, firstCrystalAxis=1,
+                NrCrystalsPerRing=nt, NrRings=nr)
+    rng = np.random.default_rng(5)
+    i = rng.integers(0, nt * nr, n)
+    j = rng.integers(0, nt * nr - 1, n)
+    pairs = torch.as_tensor(np.stack([i, j + (j >= i)], 1))
+    sm = PETLMSystemMatrix(ObjectMeta([3.0] * 3, shape),
+                           PETLMProjMeta(pairs, info=info,
+                                         detector_ids_sensitivity=pairs[:100].clone()))
+    imgs = [torch.rand(shape, device=cuda) + k for k in range(8)]
+    want = [sm.forward(x) for x in imgs]
+    back = [sm.backward(y) for y in want]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    got, gback = [], []
+    for k, x in enumerate(imgs):
+        with torch.cuda.stream(streams[k % 2]):
+            got.append(sm.forward(x))
+            gback.append(sm.backward(want[k]))
+    torch.cuda.synchronize()
+    gr = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(gr, stream=streams[0]):
+        rec = sm.forward(imgs[0])
+    gr.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(got + gback + [rec], want + back + [want[0]]):
+        assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < TOL
