@@ -14,8 +14,8 @@ angles over 360 deg at 22 cm, PSF sigma(d) = 0.03 d + 0.11 cm, Poisson projectio
   e2e      : OSEM(likelihood)(4, 10) through the public API from host tensors
              (system matrix construction, H2D of projections and mu, normalisation,
              40 sub-iterations, D2H of the result), reported per sub-iteration
-  roofline : forward projector (k_fwd_psf + k_reduce), algorithmic bytes per launch from
-             the padded-volume model 12 x (4P(1+a) + 4Q), P = 182*182*128, Q = 182*128
+  roofline : forward projector (k_fwd_strip + k_fwd_ysum + k_reduce), algorithmic bytes per
+             launch from the padded-volume model 12 x (4P(1+a) + 4Q), P = 182*182*128, Q = 182*128
   cpu_baseline : the float32 C oracle port of the same sub-iteration on the host cores
 
 ``--impl reference`` times the CPU implementation of the path (the oracle port, all host
@@ -36,10 +36,10 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "OSEM subiter/s at 128^3x120 ang (att+PSF)"
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one 12-angle k_fwd_psf launch
-# of this workload, from a separate ncu capture of the same kernel (a constant: this
-# script does not run ncu)
-FWD_DRAM_BYTES_PER_LAUNCH = 114.981e6 + 3.262e6
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one 12-angle k_fwd_strip and one
+# k_fwd_ysum launch of this workload, from a separate ncu capture of the same kernels (a
+# constant: this script does not run ncu)
+FWD_DRAM_BYTES_PER_LAUNCH = 118e6 + 66e6 + 113e6 + 3e6
 PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 
 
@@ -721,7 +721,8 @@ def run_osem(args, dev, w, rank, world, dist, full=True):
                                               / (w.n_iters * w.n_subsets)),
                     "d2h_bytes_per_step": int(out_host.numel() * 4 / (w.n_iters * w.n_subsets)),
                     "what": "OSEM(4,10) from host tensors incl. plan build and normalisation"},
-            "roofline": {"bound": "hbm", "kernel": "forward projector (k_fwd_psf + k_reduce)"
+            "roofline": {"bound": "hbm", "kernel": "forward projector (k_fwd_strip + k_fwd_ysum + "
+                                                   "k_reduce)"
                          if w.psf else "forward projector (k_fwd_nopsf + k_reduce)",
                          "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                          "peak_kind": peak_kind,
@@ -733,7 +734,7 @@ def run_osem(args, dev, w, rank, world, dist, full=True):
                          "fma_cobound": fma_cobound(w, n_sel, fwd_ms, dev)},
             "backward_ms": bwd_ms,
             "alg_gbs_per_subiter": sub_bytes / (fused_ms / 1000) / 1e9,
-            "gpu_launches": 4 * args.steps,
+            "gpu_launches": (5 if w.psf else 3) * args.steps,
             "clocks": clocks.summary() if clocks else None,
             "cpu_baseline": cpu,
             "cpu_torch_reference": cpu_torch,
@@ -789,7 +790,7 @@ def main():
                     help="with --workload pet: also time the all-pairs sensitivity image once")
     ap.add_argument("--profile-forward", type=int, default=0, choices=[0, 1, 2],
                     help="run three 12-angle forward projections of the 128^3 workload with "
-                         "forward variant 1 or 2 and exit (for ncu)")
+                         "forward tuning 1 or 2 (the same kernels) and exit (for ncu)")
     ap.add_argument("--profile-case", action="store_true",
                     help="run 3 fused sub-iterations of the workload and exit (for ncu)")
     ap.add_argument("--workload", default="osem128",  # osem64: the 64^3 / 64-angle att case
