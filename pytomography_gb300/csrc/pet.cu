@@ -304,6 +304,7 @@ struct gb_pet_plan {
     int4 *d_rec = nullptr;
     float *d_tof_tab = nullptr;
     std::vector<long long> list_off;
+    bool tiles_ready = false;
     // deterministic back projection: fixed-point sums [img_size], the list's max |proj|
     // bits and the fixed-point scale
     unsigned long long *d_acc64 = nullptr;
@@ -351,14 +352,18 @@ static void subset_range(const gb_pet_plan *p, int subset, long long &first, lon
 }
 
 // Sort the events of every list by their locality key (device radix sort, stable, so
-// equal keys keep list order) and pack the tiles.
+// equal keys keep list order) and pack the tiles.  The tiles of the split before make room
+// first (they may fill most of the memory); after a failure the plan has none, and its
+// projections are refused (tiles_ready) until a split succeeds.
 static gb_status build_tiles(gb_pet_plan *p, int n_subsets) {
     const long long E = p->n_events;
     dev_free(p->d_rec);
     p->d_rec = nullptr;
+    p->tiles_ready = false;
     p->list_off.assign(1, 0);
     if (E == 0) {
         for (int s = 0; s < n_subsets; s++) p->list_off.push_back(0);
+        p->tiles_ready = true;
         return GB_OK;
     }
     GB_CUDA(dev_alloc(&p->d_rec, (size_t)(2 * E) * sizeof(int4)));
@@ -405,7 +410,14 @@ static gb_status build_tiles(gb_pet_plan *p, int n_subsets) {
     }
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return fail(e);
     dev_free(keys); dev_free(keys2); dev_free(vals); dev_free(vals2); dev_free(tmp);
+    p->tiles_ready = true;
     return GB_OK;
+}
+
+static gb_status check_tiles(const gb_pet_plan *p) {
+    if (p->tiles_ready) return GB_OK;
+    set_error("the plan has no event tiles (its last subset split failed): set the subsets again");
+    return GB_ERR_STATE;
 }
 
 // Whether n LORs pay for the passes over the patch layout: their planes (bounded by the image
@@ -670,6 +682,7 @@ gb_status gb_pet_forward(gb_pet_plan *p, const float *img, float *proj, int32_t 
     GB_CHECK_ARG(p && img && proj, "null argument");
     GB_CHECK_ARG(subset < p->n_subsets, "subset out of range");
     GB_INJECT_LAUNCH();
+    if (gb_status ts = check_tiles(p)) return ts;
     long long first, stride, n;
     subset_range(p, subset, first, stride, n);
     if (n == 0) return GB_OK;
@@ -687,6 +700,7 @@ gb_status gb_pet_backward(gb_pet_plan *p, const float *proj, float *img, int32_t
     GB_CHECK_ARG(((uintptr_t)img & 15) == 0, "image buffer must be 16-byte aligned");
     GB_INJECT_LAUNCH();
     GB_CHECK_ARG(subset < p->n_subsets, "subset out of range");
+    if (gb_status ts = check_tiles(p)) return ts;
     long long first, stride, n;
     subset_range(p, subset, first, stride, n);
     cudaStream_t st = as_stream(stream);
@@ -742,6 +756,7 @@ gb_status gb_pet_osem_step(gb_pet_plan *p, float *img, const float *numerator,
     GB_CHECK_ARG(numerator_len == 1 || numerator_len == p->n_events,
                  "numerator must hold 1 or n_events values");
     GB_CHECK_ARG(subset < p->n_subsets, "subset out of range");
+    if (gb_status ts = check_tiles(p)) return ts;
     long long first, stride, n;
     subset_range(p, subset, first, stride, n);
     cudaStream_t st = as_stream(stream);
@@ -788,6 +803,7 @@ gb_status gb_pet_lor_forward(gb_pet_plan *p, const float *img, float *proj, int3
     clear_error();
     GB_CHECK_ARG(p && img && proj, "null argument");
     GB_CHECK_ARG(subset < p->n_subsets, "subset out of range");
+    if (gb_status ts = check_tiles(p)) return ts;
     long long first, stride, n;
     subset_range(p, subset, first, stride, n);
     if (n == 0) return GB_OK;

@@ -391,20 +391,23 @@ static double sum_of(const std::vector<double> &v) {
     return t;
 }
 
-static gb_status upload_lists(gb_spect_plan *p, int n_subsets) {
+// Builds and uploads the angle lists and work items of a split: `subsets` if not empty, else
+// i::n_subsets.  A failure leaves the plan's current split in place.
+static gb_status upload_lists(gb_spect_plan *p, int n_subsets,
+                              const std::vector<std::vector<int>> &subsets) {
     std::vector<int> all;
     std::vector<int4> items;
     std::vector<int> ioff;
-    p->lists.clear();
+    std::vector<gb_spect_plan::List> lists;
     std::vector<std::vector<int>> angle_lists;
     {
         std::vector<int> l;
         for (int a = 0; a < p->n_angles; a++) l.push_back(a);
         angle_lists.push_back(l);
     }
-    if (!p->explicit_subsets.empty()) {
-        n_subsets = (int)p->explicit_subsets.size();
-        for (const auto &l : p->explicit_subsets) angle_lists.push_back(l);
+    if (!subsets.empty()) {
+        n_subsets = (int)subsets.size();
+        for (const auto &l : subsets) angle_lists.push_back(l);
     } else {
         for (int s = 0; s < n_subsets; s++) {
             std::vector<int> l;
@@ -484,31 +487,46 @@ static gb_status upload_lists(gb_spect_plan *p, int n_subsets) {
             }
             L.n_gitems.push_back((int)items.size() - L.gitem_off.back());
         }
-        p->lists.push_back(L);
+        lists.push_back(L);
+    }
+    int *d_alist = nullptr, *d_ioff = nullptr;
+    int4 *d_items = nullptr;
+    float *d_partials = nullptr;
+    const size_t need = max_items * p->N * p->nz;
+    cudaError_t e;
+    if ((e = dev_alloc(&d_alist, all.size() * sizeof(int))) != cudaSuccess ||
+        (e = cudaMemcpy(d_alist, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice)) !=
+            cudaSuccess ||
+        (e = dev_alloc(&d_items, std::max<size_t>(1, items.size()) * sizeof(int4))) !=
+            cudaSuccess ||
+        (!items.empty() && (e = cudaMemcpy(d_items, items.data(), items.size() * sizeof(int4),
+                                           cudaMemcpyHostToDevice)) != cudaSuccess) ||
+        (e = dev_alloc(&d_ioff, ioff.size() * sizeof(int))) != cudaSuccess ||
+        (e = cudaMemcpy(d_ioff, ioff.data(), ioff.size() * sizeof(int), cudaMemcpyHostToDevice)) !=
+            cudaSuccess ||
+        (need > p->partials_cap &&
+         (e = dev_alloc(&d_partials, need * sizeof(float))) != cudaSuccess)) {
+        dev_free(d_alist);
+        dev_free(d_items);
+        dev_free(d_ioff);
+        set_error("subset lists: %s", cudaGetErrorString(e));
+        return e == cudaErrorMemoryAllocation ? GB_ERR_OOM : GB_ERR_CUDA;
     }
     dev_free(p->d_alist);
     dev_free(p->d_items);
     dev_free(p->d_ioff);
-    p->d_alist = nullptr;
-    p->d_items = nullptr;
-    p->d_ioff = nullptr;
-    GB_CUDA(dev_alloc(&p->d_alist, all.size() * sizeof(int)));
-    GB_CUDA(cudaMemcpy(p->d_alist, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice));
-    GB_CUDA(dev_alloc(&p->d_items, std::max<size_t>(1, items.size()) * sizeof(int4)));
-    if (!items.empty())
-        GB_CUDA(cudaMemcpy(p->d_items, items.data(), items.size() * sizeof(int4),
-                           cudaMemcpyHostToDevice));
-    GB_CUDA(dev_alloc(&p->d_ioff, ioff.size() * sizeof(int)));
-    GB_CUDA(cudaMemcpy(p->d_ioff, ioff.data(), ioff.size() * sizeof(int), cudaMemcpyHostToDevice));
-    p->n_subsets = n_subsets;
-    p->lists_version++;
-    size_t need = max_items * p->N * p->nz;
-    if (need > p->partials_cap) {
+    p->d_alist = d_alist;
+    p->d_items = d_items;
+    p->d_ioff = d_ioff;
+    if (d_partials) {
         dev_free(p->d_partials);
-        p->d_partials = nullptr;
-        GB_CUDA(dev_alloc(&p->d_partials, need * sizeof(float)));
+        p->d_partials = d_partials;
         p->partials_cap = need;
     }
+    p->lists = std::move(lists);
+    p->explicit_subsets = subsets;
+    p->n_subsets = n_subsets;
+    p->lists_version++;
     return GB_OK;
 }
 
@@ -813,7 +831,7 @@ gb_status gb_spect_plan_create(const gb_spect_desc *d, gb_spect_plan **out) {
         g.wranges = p->d_wranges;
     }
 #undef FAIL_CUDA
-    gb_status st = upload_lists(p, 1);
+    gb_status st = upload_lists(p, 1, {});
     if (st != GB_OK) {
         free_plan(p);
         return st;
@@ -859,8 +877,7 @@ gb_status gb_spect_set_subsets(gb_spect_plan *p, int32_t n_subsets) {
     GB_CHECK_ARG(p, "null plan");
     GB_CHECK_ARG(n_subsets >= 1 && n_subsets <= p->n_angles, "n_subsets must be in [1, %d]",
                  p->n_angles);
-    p->explicit_subsets.clear();
-    return upload_lists(p, n_subsets);
+    return upload_lists(p, n_subsets, {});
 }
 
 gb_status gb_spect_set_subset_lists(gb_spect_plan *p, int32_t n_subsets, const int32_t *angle_idx,
@@ -880,8 +897,7 @@ gb_status gb_spect_set_subset_lists(gb_spect_plan *p, int32_t n_subsets, const i
         }
         off += counts[s];
     }
-    p->explicit_subsets = lists;
-    return upload_lists(p, n_subsets);
+    return upload_lists(p, n_subsets, lists);
 }
 
 int32_t gb_spect_subset_size(const gb_spect_plan *p, int32_t subset) {
@@ -959,7 +975,8 @@ gb_status gb_spect_set_tuning(gb_spect_plan *p, const gb_spect_tuning *tuning) {
     p->fwd_items = t.fwd_items;
     p->Zt_b1 = t.b1_zt;
     p->b1_items = t.b1_items;
-    return upload_lists(p, std::max(1, p->n_subsets));
+    return upload_lists(p, std::max(1, p->n_subsets),
+                        std::vector<std::vector<int>>(p->explicit_subsets));
 }
 
 // A forward group's angles of one half (0: slots before n / 2, 1: the others) or all of them

@@ -122,9 +122,11 @@ class PETLMSystemMatrix(SystemMatrix):
         if self.subset_indices_array is not None and int(n_subsets) == self.n_subsets:
             return  # the same split: indices and the plan's sorted event tiles are unchanged
         idx = torch.arange(self.proj_meta.detector_ids.shape[0]).to(torch.long).cpu()
-        self.subset_indices_array = [idx[i::n_subsets] for i in range(n_subsets)]
-        self.n_subsets = n_subsets
+        subsets = [idx[i::n_subsets] for i in range(n_subsets)]
+        self.subset_indices_array = None  # a failed split leaves the plan without tiles
         _lib.check(self._lib.gb_pet_set_subsets(self._plan, int(n_subsets)))
+        self.subset_indices_array = subsets
+        self.n_subsets = n_subsets
 
     def get_projection_subset(self, projections, subset_idx):
         if projections.shape[0] > 1 and subset_idx is not None:
@@ -341,9 +343,9 @@ class PETSinogramSystemMatrix(SystemMatrix):
     # ------------------------------------------------------------ subsets
     def set_n_subsets(self, n_subsets: int) -> None:
         indices = torch.arange(self.proj_meta.N_angles).to(torch.long).to(self.output_device)
+        _lib.check(self._lib.gb_pet_sino_set_subsets(self._plan, int(n_subsets)))
         self.subset_indices_array = [indices[i::n_subsets] for i in range(n_subsets)]
         self._n_subsets = n_subsets
-        _lib.check(self._lib.gb_pet_sino_set_subsets(self._plan, int(n_subsets)))
 
     def get_projection_subset(self, projections, subset_idx):
         if subset_idx is None:

@@ -216,9 +216,11 @@ class SPECTSystemMatrix(SystemMatrix):
         if self.subset_indices_array is not None and int(n_subsets) == self.n_subsets:
             return  # the same split: indices and the plan's work lists are unchanged
         indices = torch.arange(self.proj_meta.shape[0]).to(torch.long).to(self.device)
-        self.subset_indices_array = [indices[i::n_subsets] for i in range(n_subsets)]
-        self.n_subsets = n_subsets
+        subsets = [indices[i::n_subsets] for i in range(n_subsets)]
+        # (a failed call leaves the plan and this object with the split before)
         _lib.check(self._lib.gb_spect_set_subsets(self._plan, int(n_subsets)))
+        self.subset_indices_array = subsets
+        self.n_subsets = n_subsets
         self._lists_epoch += 1
         if self.autotune_enabled:
             self.autotune()
@@ -450,13 +452,13 @@ class StarGuideSystemMatrix(SystemMatrix):
         angles = torch.as_tensor(self.proj_meta.angles)
         groups = [torch.where(angles == a)[0] for a in torch.unique(angles)]
         lists = [torch.cat(groups[i::n_subsets]) for i in range(n_subsets)]
-        self.subset_indices_array = [ix.to(self.device) for ix in lists]
-        self.n_subsets = n_subsets
         flat = torch.cat(lists).to(torch.int32).numpy()
         counts = np.array([len(ix) for ix in lists], np.int32)
         _lib.check(self._lib.gb_spect_set_subset_lists(
             self._H._plan, int(n_subsets), flat.ctypes.data_as(ctypes.c_void_p),
             counts.ctypes.data_as(ctypes.c_void_p)))
+        self.subset_indices_array = [ix.to(self.device) for ix in lists]
+        self.n_subsets = n_subsets
         self._H.subset_indices_array = self.subset_indices_array
         self._H.n_subsets = n_subsets
 

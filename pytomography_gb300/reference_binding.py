@@ -156,8 +156,8 @@ def bind(reference_system_matrix_class):
             self._gb = make_plan(self)
 
         def set_n_subsets(self, n_subsets: int) -> None:
-            super().set_n_subsets(n_subsets)
             _lib.check(self._gb.lib.gb_spect_set_subsets(self._gb.handle, int(n_subsets)))
+            super().set_n_subsets(n_subsets)
 
         def _n_sel(self, subset_idx):
             return self.proj_meta.num_projections if subset_idx is None else \
