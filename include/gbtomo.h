@@ -98,14 +98,15 @@ gb_status gb_spect_plan_create(const gb_spect_desc *desc, gb_spect_plan **plan);
 gb_status gb_spect_plan_destroy(gb_spect_plan *plan);
 
 /* Device-side error word of the plan (synchronous read): 0, or 1 when a kernel's
- * bounded wait on its TMA copies gave up (the kernel then returned without output).
+ * bounded wait on its TMA copies gave up (the call's output is then not valid).
  * No counterpart in the reference (which has no device code). */
 gb_status gb_spect_device_status(gb_spect_plan *plan, int32_t *code);
 /* Reset the device error word to 0. */
 gb_status gb_spect_clear_device_status(gb_spect_plan *plan);
 /* Test hook of the bounded waits (no counterpart in the reference): skip_first_copy = 1
- * makes the fused forward projector (attenuation before PSF, nz % 4 == 0) leave its first
- * attenuation copy of every work item unissued, so its wait for that copy runs out after
+ * makes the forward projector leave the first TMA copy of every work item unissued (of the
+ * attenuation rows in the plane-at-a-time kernel, attenuation before PSF and nz % 4 == 0; of
+ * the rows between the two strip kernels), so that the wait for that copy runs out after
  * wait_polls polls (each at most 20 us; 0 restores the default of 65536) and the kernel
  * returns with the error word set to 1.  Nothing is left in flight. */
 gb_status gb_spect_set_debug(gb_spect_plan *plan, int32_t skip_first_copy, int32_t wait_polls);

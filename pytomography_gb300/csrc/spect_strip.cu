@@ -412,6 +412,7 @@ __global__ void __launch_bounds__(512, 1) k_fwd_strip_batch(const __grid_constan
 // of the summing warps, the copies cost that warp 1,300 cycles a plane and held up the
 // others.)  Rows outside the plane's range read as zero.
 constexpr int kYStages = 2;
+constexpr unsigned kDrainPolls = 65536;  // polls (20 us at most) for copies that were issued
 
 struct YsumLayout {  // dynamic shared memory, in floats
     size_t item, taps, zero, total;
@@ -450,17 +451,18 @@ __device__ __forceinline__ void ysum_item(const SpectDev &g, const float *__rest
     const int np = it->n_planes;
     if (warp >= nw) {
         if (warp > nw || lane != 0) return;
-        int n = 0;
-        for (; n < np; n++) {
+        // A stage is filled again only when every summing warp has left it, and a warp leaves a
+        // stage only after its copy has landed: at most one copy per stage is in flight.
+        unsigned issued[kYStages] = {};
+        for (int n = 0; n < np; n++) {
+            // (the test hook leaves the first copy out: the summing warps give up on it)
+            if (n == 0 && g.dbg_skip_first_copy) continue;
             const int s = n % kYStages;
-            // the stage's previous plane has been left by every warp
             if (n >= kYStages &&
                 !mbar_wait_bounded(empty + s, (n / kYStages - 1) & 1, g.wait_polls)) {
                 if (g.err) atomicExch(g.err, GB_ERR_WAIT_TIMEOUT);
                 break;
             }
-            // (the test hook leaves the first copy out: its wait gives up)
-            if (n == 0 && g.dbg_skip_first_copy) continue;
             const int4 pi = it->plane[n];
             const unsigned bytes = (unsigned)(pi.y - pi.x + 1) * 128u;
             mbar_arrive_expect_tx(full + s, bytes);
@@ -468,13 +470,16 @@ __device__ __forceinline__ void ysum_item(const SpectDev &g, const float *__rest
                         Ws + (((size_t)(pi.w >> 4) * strip_slabs(g) + slab) * g.nya +
                               (pi.x - g.ya_lo)) * 32,
                         bytes, full + s);
+#pragma unroll
+            for (int k = 0; k < kYStages; k++) issued[k] += k == s;
         }
-        // no copy may be in flight when the CTA ends, not even after a wait that gave up
-        for (int k = max(n - kYStages, g.dbg_skip_first_copy ? 1 : 0); k < n; k++)
-            mbar_wait_bounded(full + k % kYStages, (k / kYStages) & 1, g.wait_polls);
+        // no copy may be in flight when the CTA ends, not even after a wait that gave up: the
+        // j-th copy of a stage completes phase j - 1 of its barrier
+#pragma unroll
+        for (int s = 0; s < kYStages; s++)
+            if (issued[s]) mbar_wait_bounded(full + s, (issued[s] - 1) & 1, kDrainPolls);
         return;
     }
-    bool failed = false;
     const int q = lane & 7, o0 = 32 * warp + 8 * (lane >> 3);  // quad of the slab, first row
     const float *zero = sm + L.zero + 4 * q;
     float2 acc[8][2];
@@ -482,11 +487,13 @@ __device__ __forceinline__ void ysum_item(const SpectDev &g, const float *__rest
     for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = make_float2(0.f, 0.f);
     for (int n = 0; n < np; n++) {
         const int s = n % kYStages;
-        if (!failed && !mbar_wait_bounded(full + s, (n / kYStages) & 1, g.wait_polls)) {
-            failed = true;
-            if (g.err) atomicExch(g.err, GB_ERR_WAIT_TIMEOUT);
+        // A warp that gives up leaves for good, without a result and without releasing the
+        // stage: the copying warp then gives up on the stage as well and drains.
+        const bool ok = mbar_wait_bounded(full + s, (n / kYStages) & 1, g.wait_polls);
+        if (!__all_sync(0xffffffffu, ok)) {
+            if (lane == 0 && g.err) atomicExch(g.err, GB_ERR_WAIT_TIMEOUT);
+            return;
         }
-        __syncwarp();
         const int4 pi = it->plane[n];
         const float *st = sm + (size_t)s * g.nya * 32 + 4 * q;
         const float *tap = taps + ((pi.w >> 4) - x0) * kStripTaps;
