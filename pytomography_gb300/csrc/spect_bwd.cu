@@ -471,7 +471,7 @@ extern "C" int gb_debug_b1_phase_reset(void) {
 // (row, z quad) (16-byte loads and stores).
 template <bool VEC>
 __global__ void __launch_bounds__(256)
-    k_b1_nopsf(SpectDev g, const float *__restrict__ proj, const int *__restrict__ alist,
+    k_b1_nopsf(SpectDev g, const float *proj, const int *__restrict__ alist,
                float *__restrict__ W) {
     constexpr int V = VEC ? 4 : 1;
     grid_release();
@@ -627,7 +627,7 @@ cudaError_t launch_b1(const SpectDev &g, const float *proj, const int *alist, in
 // sum_s w_rs phi1(f_r, f_s) over the 26 neighbours with replicate boundary, in the
 // loop order of NearestNeighbourPrior._pair_contribution (nearest_neighbour.py:56-72);
 // phi1 of RelativeDifferencePrior (nearest_neighbour.py:176-177).
-__device__ __forceinline__ float rdp_sum(const float *__restrict__ f, int nx, int ny, int nz,
+__device__ __forceinline__ float rdp_sum(const float *f, int nx, int ny, int nz,
                                          int x, int y, int z, float fr, const UpdateArgs &u) {
     float acc = 0.f;
     int n = 0;
@@ -642,7 +642,7 @@ __device__ __forceinline__ float rdp_sum(const float *__restrict__ f, int nx, in
             for (int k = -1; k <= 1; k++) {
                 if (i == 0 && j == 0 && k == 0) continue;
                 int zk = min(max(z + k, 0), nz - 1);
-                float fs = __ldg(f + ((size_t)xi * ny + yj) * nz + zk);
+                float fs = ld_data(f + ((size_t)xi * ny + yj) * nz + zk);
                 float d = __fsub_rn(fr, fs);
                 float ad = fabsf(d);
                 float num = __fmul_rn(
@@ -675,7 +675,7 @@ __device__ __forceinline__ float fast_rcp(float x) {
 }
 
 template <bool FAST>
-__device__ __forceinline__ void rdp_sum4(const float *__restrict__ f, int nx, int ny, int nz,
+__device__ __forceinline__ void rdp_sum4(const float *f, int nx, int ny, int nz,
                                          int x, int y, int z, const float (&fr)[4],
                                          const UpdateArgs &u, float (&acc)[4], float &low) {
 #pragma unroll
@@ -686,9 +686,9 @@ __device__ __forceinline__ void rdp_sum4(const float *__restrict__ f, int nx, in
         const int xi = min(max(x + ij / 3 - 1, 0), nx - 1);
         const int yj = min(max(y + ij % 3 - 1, 0), ny - 1);
         const float *p = f + ((size_t)xi * ny + yj) * nz;
-        const float4 c = __ldg(reinterpret_cast<const float4 *>(p + z));
-        const float row[6] = {__ldg(p + max(z - 1, 0)), c.x, c.y, c.z, c.w,
-                              __ldg(p + min(z + 4, nz - 1))};
+        const float4 c = ld_data4(p + z);
+        const float row[6] = {ld_data(p + max(z - 1, 0)), c.x, c.y, c.z, c.w,
+                              ld_data(p + min(z + 4, nz - 1))};
         float sd[6], s2[6];  // f_s + delta, 2 f_s + delta
         if (FAST) {
 #pragma unroll
@@ -860,7 +860,7 @@ __device__ __forceinline__ void apply_update4(int mode, const UpdateArgs &u, siz
 // Reference back-projector: for every object voxel, bilinear sample of W at the
 // back-rotation (angle 270 - beta) of each angle of the group, summed.  Threads own
 // (x, y, z quad); two angles are sampled before accumulating to keep loads in flight.
-__device__ __forceinline__ float4 b2_gather_sum4(const SpectDev &g, const float *__restrict__ W,
+__device__ __forceinline__ float4 b2_gather_sum4(const SpectDev &g, const float *W,
                                                   const int *__restrict__ alist, int n_slots,
                                                   int x, int y, int z) {
     const int nz = g.nzs;  // z: first value of the quad in its W row
@@ -948,16 +948,16 @@ __host__ __device__ __forceinline__ bool b2_tab_fits(const SpectDev &g, int n_ro
     return n_rows * n_slots <= kB2Taps && (long long)g.Lp * g.nya * g.nzs < (1LL << 31);
 }
 
-__device__ __forceinline__ float4 b2_tap_sample(const float *__restrict__ Ws, const B2Tap &t,
+__device__ __forceinline__ float4 b2_tap_sample(const float *Ws, const B2Tap &t,
                                                 int nya, int nz, int z) {
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     if (t.mask == 0) return zero;
     const float *p = Ws + t.off + z;
     const int rs = nya * nz;
-    const float4 vnw = (t.mask & 1) ? __ldg(reinterpret_cast<const float4 *>(p)) : zero;
-    const float4 vne = (t.mask & 2) ? __ldg(reinterpret_cast<const float4 *>(p + nz)) : zero;
-    const float4 vsw = (t.mask & 4) ? __ldg(reinterpret_cast<const float4 *>(p + rs)) : zero;
-    const float4 vse = (t.mask & 8) ? __ldg(reinterpret_cast<const float4 *>(p + rs + nz)) : zero;
+    const float4 vnw = ld_data4_if(t.mask & 1, p);
+    const float4 vne = ld_data4_if(t.mask & 2, p + nz);
+    const float4 vsw = ld_data4_if(t.mask & 4, p + rs);
+    const float4 vse = ld_data4_if(t.mask & 8, p + rs + nz);
     Bilin b;
     b.nw = t.nw;
     b.ne = t.ne;
@@ -974,7 +974,7 @@ __device__ __forceinline__ float4 b2_tap_sample(const float *__restrict__ Ws, co
 // Sum over the slots of one row's table entries; U slots are sampled before accumulating
 // (loads in flight), the additions run in slot order.
 template <int U>
-__device__ __forceinline__ float4 b2_gather_sum4_tab(const float *__restrict__ W, size_t slab,
+__device__ __forceinline__ float4 b2_gather_sum4_tab(const float *W, size_t slab,
                                                       const B2Tap *tab, int n_slots, int nya,
                                                       int nz, int z) {
     float4 bp = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1008,13 +1008,13 @@ __device__ __forceinline__ float4 b2_gather_sum4_tab(const float *__restrict__ W
 // A sample of W = A (.) P (no PSF) made at its corners from A (null: none) and the slot's
 // projection rows: the products B1 would have stored, so the same sums.
 __device__ __forceinline__ float4 b2_tap_sample_fused(const float *__restrict__ As,
-                                                      const float *__restrict__ Ps,
+                                                      const float *Ps,
                                                       const B2Tap &t, int nya, int nz, int z) {
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     if (t.mask == 0) return zero;
     const float *pp = Ps + t.poff + z;
-    const float4 pw = (t.mask & 5) ? __ldg(reinterpret_cast<const float4 *>(pp)) : zero;
-    const float4 pe = (t.mask & 10) ? __ldg(reinterpret_cast<const float4 *>(pp + nz)) : zero;
+    const float4 pw = ld_data4_if(t.mask & 5, pp);
+    const float4 pe = ld_data4_if(t.mask & 10, pp + nz);
     float4 vnw = (t.mask & 1) ? pw : zero, vne = (t.mask & 2) ? pe : zero;
     float4 vsw = (t.mask & 4) ? pw : zero, vse = (t.mask & 8) ? pe : zero;
     if (As) {
@@ -1045,8 +1045,8 @@ constexpr int kB2Unroll = 2;
 // (with the prior's shorter terms).
 template <bool PRIOR>
 __global__ void __launch_bounds__(256)
-    k_b2_nopsf4(SpectDev g, const float *__restrict__ proj, const int *__restrict__ alist,
-                int n_slots, float *__restrict__ out, int mode, UpdateArgs u) {
+    k_b2_nopsf4(SpectDev g, const float *proj, const int *__restrict__ alist,
+                int n_slots, float *out, int mode, UpdateArgs u) {
     __shared__ B2Tap tab[kB2Taps];
     grid_release();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1091,10 +1091,12 @@ __global__ void __launch_bounds__(256)
     apply_update4<PRIOR>(mode, u, i, x, y, z, N, N, nz, bp, out);
 }
 
+// (Blocks an SM: five of 48 registers without the prior, which waits for W and gains from warps,
+// 95.6 us against 98.2 for four at 128^3, 12 angles; four of 64 with it.)
 template <bool PRIOR>
-__global__ void __launch_bounds__(256)
-    k_b2_gather4(SpectDev g, const float *__restrict__ W, const int *__restrict__ alist,
-                 int n_slots, float *__restrict__ out, int mode, UpdateArgs u) {
+__global__ void __launch_bounds__(256, PRIOR ? 4 : 5)
+    k_b2_gather4(SpectDev g, const float *W, const int *__restrict__ alist,
+                 int n_slots, float *out, int mode, UpdateArgs u) {
     __shared__ B2Tap tab[kB2Taps];
     grid_release();
     if (!g.strip) grid_wait();  // the row ranges come from the kernel before (strip: the plan)
@@ -1180,8 +1182,8 @@ cudaError_t launch_b2_gather_batch(const B2Batch &p, int n_blocks, cudaStream_t 
 }
 
 __global__ void __launch_bounds__(256)
-    k_b2_gather(SpectDev g, const float *__restrict__ W, const int *__restrict__ alist,
-                int n_slots, float *__restrict__ out, int mode, UpdateArgs u) {
+    k_b2_gather(SpectDev g, const float *W, const int *__restrict__ alist,
+                int n_slots, float *out, int mode, UpdateArgs u) {
     const int z = blockIdx.x * 32 + threadIdx.x;
     const int y = blockIdx.y * 8 + threadIdx.y;
     const int x = blockIdx.z;
@@ -1290,9 +1292,9 @@ __device__ __forceinline__ int adj_list(const SpectDev &g, int ga, int slot, int
 }
 
 // Block of 256 (row, quad position) elements from q0 on; mode B2_WRITE or B2_ADD.
-__device__ __forceinline__ void b2_adjoint_block(const SpectDev &g, const float *__restrict__ W,
+__device__ __forceinline__ void b2_adjoint_block(const SpectDev &g, const float *W,
                                                  const int *__restrict__ alist, int n_slots,
-                                                 long long q0, float *__restrict__ out, int mode,
+                                                 long long q0, float *out, int mode,
                                                  AdjTable &t) {
     const int N = g.N, nz = g.nz, nq = g.nzs / 4;
     const long long total = (long long)N * N * nq, q = q0 + threadIdx.x;
@@ -1326,7 +1328,7 @@ __device__ __forceinline__ void b2_adjoint_block(const SpectDev &g, const float 
                 if (u < n) {
                     const float2 tp = t.tap[e][u];
                     w[u] = tp.y;
-                    v[u] = __ldg(reinterpret_cast<const float4 *>(Wk + __float_as_int(tp.x)));
+                    v[u] = ld_data4(Wk + __float_as_int(tp.x));
                 }
             }
 #pragma unroll
@@ -1338,7 +1340,7 @@ __device__ __forceinline__ void b2_adjoint_block(const SpectDev &g, const float 
             }
             for (int u = U; u < n; u++) {
                 const float2 tp = t.tap[e][u];
-                const float4 x = __ldg(reinterpret_cast<const float4 *>(Wk + __float_as_int(tp.x)));
+                const float4 x = ld_data4(Wk + __float_as_int(tp.x));
                 s.x = fmaf(tp.y, x.x, s.x);
                 s.y = fmaf(tp.y, x.y, s.y);
                 s.z = fmaf(tp.y, x.z, s.z);
@@ -1363,8 +1365,8 @@ __device__ __forceinline__ void b2_adjoint_block(const SpectDev &g, const float 
 }
 
 __global__ void __launch_bounds__(256)
-    k_b2_adjoint(SpectDev g, const float *__restrict__ W, const int *__restrict__ alist,
-                 int n_slots, float *__restrict__ out, int mode) {
+    k_b2_adjoint(SpectDev g, const float *W, const int *__restrict__ alist,
+                 int n_slots, float *out, int mode) {
     __shared__ AdjTable t;
     grid_release();
     grid_wait();

@@ -29,7 +29,7 @@ GB_FOR_EACH_K(GB_DECL_FWD)
 // plane order, so those loads are in flight together.
 template <bool VEC>
 __global__ void __launch_bounds__(256)
-    k_fwd_nopsf(SpectDev g, const float *__restrict__ f, const int *__restrict__ alist,
+    k_fwd_nopsf(SpectDev g, const float *f, const int *__restrict__ alist,
                 const int4 *__restrict__ items, float *__restrict__ partials) {
     constexpr int V = VEC ? 4 : 1, PU = VEC ? 4 : 8;
     grid_release();
@@ -89,10 +89,9 @@ __global__ void __launch_bounds__(256)
 // --------------------------------------------------------------- reduction
 // out[slot][i] = sum of the partials of the slot's items, in item order.  With
 // `ratio`, out = g[ga][i] / (sum + s[ga][i] + delta) and pred (optional) = sum + s.
-__global__ void k_reduce(const int *__restrict__ ioff, int NZ, const float *__restrict__ partials,
-                         float *__restrict__ out, int ratio, const float *__restrict__ gproj,
-                         const float *__restrict__ sadd, const int *__restrict__ alist,
-                         float *__restrict__ pred) {
+__global__ void k_reduce(const int *__restrict__ ioff, int NZ, const float *partials, float *out,
+                         int ratio, const float *gproj, const float *sadd,
+                         const int *__restrict__ alist, float *pred) {
     const int slot = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     grid_release();

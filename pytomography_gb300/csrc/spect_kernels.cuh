@@ -136,9 +136,37 @@ __device__ __forceinline__ float bilin_combine(const Bilin &b, float vnw, float 
     return fmaf(vse, b.se, fmaf(vsw, b.sw, fmaf(vne, b.ne, vnw * b.nw)));
 }
 
+// Loads of what kernels write: objects, projections, W, partial sums, ratios.  A dependent
+// launch (below) starts while its predecessors still write, so these are ordinary loads through
+// pointers without __restrict__; a read-only load (__ldg, or const __restrict__) is defined only
+// for data that nobody writes while the kernel lives, and may move above grid_wait().  Plan
+// tables (A, taps, rotations, lists) keep read-only loads.
+__device__ __forceinline__ float ld_data(const float *p) { return *p; }
+__device__ __forceinline__ float4 ld_data4(const float *p) {
+    return *reinterpret_cast<const float4 *>(p);
+}
+// The same where `ok`, else zeros: a predicated load (volatile, so that it stays below
+// grid_wait(); a plain conditional load becomes a branch around it).
+__device__ __forceinline__ float ld_data_if(bool ok, const float *p) {
+    float v = 0.f;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.f32 %0, [%1];\n\t}"
+                 : "+f"(v)
+                 : "l"(p), "r"((unsigned)ok));
+    return v;
+}
+__device__ __forceinline__ float4 ld_data4_if(bool ok, const float *p) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
+        "@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
+        : "l"(p), "r"((unsigned)ok));
+    return v;
+}
+
 // Bilinear sample of a [rows][cols][nz] array whose (row, col) origin is shifted by
 // (row_off, col_off): value at (r, c) = src[r - row_off][c - col_off] when inside.
-__device__ __forceinline__ float sample(const float *__restrict__ src, int rows, int cols,
+__device__ __forceinline__ float sample(const float *src, int rows, int cols,
                                         int nz, int row_off, int col_off, const Bilin &b,
                                         int z) {
     int r = b.r0 - row_off, c = b.c0 - col_off;
@@ -146,16 +174,16 @@ __device__ __forceinline__ float sample(const float *__restrict__ src, int rows,
     bool c0 = (unsigned)c < (unsigned)cols, c1 = (unsigned)(c + 1) < (unsigned)cols;
     if (!((r0 || r1) && (c0 || c1))) return 0.f;
     const float *p = src + ((long long)r * cols + c) * nz + z;
-    float vnw = (r0 && c0) ? __ldg(p) : 0.f;
-    float vne = (r0 && c1) ? __ldg(p + nz) : 0.f;
-    float vsw = (r1 && c0) ? __ldg(p + (long long)cols * nz) : 0.f;
-    float vse = (r1 && c1) ? __ldg(p + (long long)cols * nz + nz) : 0.f;
+    float vnw = ld_data_if(r0 && c0, p);
+    float vne = ld_data_if(r0 && c1, p + nz);
+    float vsw = ld_data_if(r1 && c0, p + (long long)cols * nz);
+    float vse = ld_data_if(r1 && c1, p + (long long)cols * nz + nz);
     return bilin_combine(b, vnw, vne, vsw, vse);
 }
 
 // Four consecutive z values (z % 4 == 0, nz % 4 == 0) of the bilinear sample; returns
 // false (and zeros) when no tap is inside the array.
-__device__ __forceinline__ bool sample4(const float *__restrict__ src, int rows, int cols, int nz,
+__device__ __forceinline__ bool sample4(const float *src, int rows, int cols, int nz,
                                         int row_off, int col_off, const Bilin &b, int z,
                                         float4 &out) {
     // branch-free: the four (predicated) loads of a sample can be in flight together
@@ -164,11 +192,10 @@ __device__ __forceinline__ bool sample4(const float *__restrict__ src, int rows,
     bool c0 = (unsigned)c < (unsigned)cols, c1 = (unsigned)(c + 1) < (unsigned)cols;
     const float *p = src + ((long long)r * cols + c) * nz + z;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 vnw = (r0 && c0) ? __ldg(reinterpret_cast<const float4 *>(p)) : zero;
-    float4 vne = (r0 && c1) ? __ldg(reinterpret_cast<const float4 *>(p + nz)) : zero;
-    float4 vsw = (r1 && c0) ? __ldg(reinterpret_cast<const float4 *>(p + (long long)cols * nz)) : zero;
-    float4 vse = (r1 && c1) ? __ldg(reinterpret_cast<const float4 *>(p + (long long)cols * nz + nz))
-                            : zero;
+    float4 vnw = ld_data4_if(r0 && c0, p);
+    float4 vne = ld_data4_if(r0 && c1, p + nz);
+    float4 vsw = ld_data4_if(r1 && c0, p + (long long)cols * nz);
+    float4 vse = ld_data4_if(r1 && c1, p + (long long)cols * nz + nz);
     out.x = bilin_combine(b, vnw.x, vne.x, vsw.x, vse.x);
     out.y = bilin_combine(b, vnw.y, vne.y, vsw.y, vse.y);
     out.z = bilin_combine(b, vnw.z, vne.z, vsw.z, vse.z);
@@ -178,8 +205,8 @@ __device__ __forceinline__ bool sample4(const float *__restrict__ src, int rows,
 
 // Same as sample4 for the back-projection stack W of one angle slot: plane r holds data
 // only in columns [wr[r].x, wr[r].y); everything else reads as zero.
-__device__ __forceinline__ bool sample4_ranged(const float *__restrict__ src, int rows, int cols,
-                                               int nz, int col_off, const int2 *__restrict__ wr,
+__device__ __forceinline__ bool sample4_ranged(const float *src, int rows, int cols,
+                                               int nz, int col_off, const int2 *wr,
                                                const Bilin &b, int z, float4 &out) {
     int r = b.r0, c = b.c0 - col_off;
     out = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -191,10 +218,10 @@ __device__ __forceinline__ bool sample4_ranged(const float *__restrict__ src, in
     if (!(a00 || a01 || a10 || a11)) return false;
     const float *p = src + ((long long)r * cols + c) * nz + z;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 vnw = a00 ? __ldg(reinterpret_cast<const float4 *>(p)) : zero;
-    float4 vne = a01 ? __ldg(reinterpret_cast<const float4 *>(p + nz)) : zero;
-    float4 vsw = a10 ? __ldg(reinterpret_cast<const float4 *>(p + (long long)cols * nz)) : zero;
-    float4 vse = a11 ? __ldg(reinterpret_cast<const float4 *>(p + (long long)cols * nz + nz)) : zero;
+    float4 vnw = ld_data4_if(a00, p);
+    float4 vne = ld_data4_if(a01, p + nz);
+    float4 vsw = ld_data4_if(a10, p + (long long)cols * nz);
+    float4 vse = ld_data4_if(a11, p + (long long)cols * nz + nz);
     out.x = bilin_combine(b, vnw.x, vne.x, vsw.x, vse.x);
     out.y = bilin_combine(b, vnw.y, vne.y, vsw.y, vse.y);
     out.z = bilin_combine(b, vnw.z, vne.z, vsw.z, vse.z);
@@ -202,8 +229,8 @@ __device__ __forceinline__ bool sample4_ranged(const float *__restrict__ src, in
     return true;
 }
 
-__device__ __forceinline__ float sample_ranged(const float *__restrict__ src, int rows, int cols,
-                                               int nz, int col_off, const int2 *__restrict__ wr,
+__device__ __forceinline__ float sample_ranged(const float *src, int rows, int cols,
+                                               int nz, int col_off, const int2 *wr,
                                                const Bilin &b, int z) {
     int r = b.r0, c = b.c0 - col_off;
     bool r0 = (unsigned)r < (unsigned)rows, r1 = (unsigned)(r + 1) < (unsigned)rows;
@@ -213,10 +240,10 @@ __device__ __forceinline__ float sample_ranged(const float *__restrict__ src, in
     bool a10 = r1 && c >= g1.x && c < g1.y, a11 = r1 && c + 1 >= g1.x && c + 1 < g1.y;
     if (!(a00 || a01 || a10 || a11)) return 0.f;
     const float *p = src + ((long long)r * cols + c) * nz + z;
-    float vnw = a00 ? __ldg(p) : 0.f;
-    float vne = a01 ? __ldg(p + nz) : 0.f;
-    float vsw = a10 ? __ldg(p + (long long)cols * nz) : 0.f;
-    float vse = a11 ? __ldg(p + (long long)cols * nz + nz) : 0.f;
+    float vnw = ld_data_if(a00, p);
+    float vne = ld_data_if(a01, p + nz);
+    float vsw = ld_data_if(a10, p + (long long)cols * nz);
+    float vse = ld_data_if(a11, p + (long long)cols * nz + nz);
     return bilin_combine(b, vnw, vne, vsw, vse);
 }
 

@@ -43,14 +43,11 @@ __host__ __device__ inline B1StripLayout b1_strip_layout(const SpectDev &g, int 
     return L;
 }
 
-// Four z values from z on (< nz) at p; vec: one 16-byte load.
-__device__ __forceinline__ float4 ld_quad(const float *__restrict__ p, int z, int nz, bool vec) {
-    if (vec) return __ldg(reinterpret_cast<const float4 *>(p));
-    float4 v = make_float4(__ldg(p), 0.f, 0.f, 0.f);
-    if (z + 1 < nz) v.y = __ldg(p + 1);
-    if (z + 2 < nz) v.z = __ldg(p + 2);
-    if (z + 3 < nz) v.w = __ldg(p + 3);
-    return v;
+// Four z values from z on (< nz) at p where `ok`, else zeros; vec: one 16-byte load.
+__device__ __forceinline__ float4 ld_quad(bool ok, const float *p, int z, int nz, bool vec) {
+    if (vec) return ld_data4_if(ok, p);
+    return make_float4(ld_data_if(ok, p), ld_data_if(ok && z + 1 < nz, p + 1),
+                       ld_data_if(ok && z + 2 < nz, p + 2), ld_data_if(ok && z + 3 < nz, p + 3));
 }
 
 // 16-byte load that stays behind the last __syncwarp: hoisted above the z pass, the loads of a
@@ -65,7 +62,7 @@ __device__ __forceinline__ float4 ldg_here(const float *p) {
 }
 
 template <int QL, int HB>
-__device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *__restrict__ P,
+__device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *P,
                                               const int ga, const int x0, const int x1,
                                               float *__restrict__ Ws, float *__restrict__ sm) {
     constexpr int G = 32 / QL, RS = 8 * G, ZG = QL / 4, SC = 4 * QL;
@@ -90,9 +87,7 @@ __device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *__
             cp_async16(sm + 4 * i, p);
             continue;
         }
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (in) v = ld_quad(p, z, nz, false);
-        *reinterpret_cast<float4 *>(sm + 4 * i) = v;
+        *reinterpret_cast<float4 *>(sm + 4 * i) = ld_quad(in, p, z, nz, false);
     }
     cp_async_wait_all();
     __syncthreads();
@@ -151,7 +146,7 @@ __device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *__
 
 template <int QL, int HB>
 __global__ void __launch_bounds__(512, 1)
-    k_b1_strip(SpectDev g, const float *__restrict__ proj, const int *__restrict__ alist,
+    k_b1_strip(SpectDev g, const float *proj, const int *__restrict__ alist,
                const int4 *__restrict__ items, float *__restrict__ W) {
     extern __shared__ __align__(128) float sm[];
     grid_release();
@@ -211,7 +206,7 @@ __host__ __device__ inline FwdStripLayout fwd_strip_layout(int QL, int HB, int w
 }
 
 // Rotated samples of four rows at z quad q, times A (Ap: the first row's quad, or null).
-__device__ __forceinline__ void gather_rows(const float *__restrict__ f, const SpectDev &g,
+__device__ __forceinline__ void gather_rows(const float *f, const SpectDev &g,
                                             const RowTap *rt, int q, bool zin, bool vec,
                                             const float *__restrict__ Ap, float4 (&v)[4]) {
     const int nz = g.nz, step_r = g.N * nz;
@@ -222,10 +217,10 @@ __device__ __forceinline__ void gather_rows(const float *__restrict__ f, const S
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const float *p = f + rt[u].off + 4 * q;
-            c[u][0] = __ldg(reinterpret_cast<const float4 *>(p));
-            c[u][1] = __ldg(reinterpret_cast<const float4 *>(p + nz));
-            c[u][2] = __ldg(reinterpret_cast<const float4 *>(p + step_r));
-            c[u][3] = __ldg(reinterpret_cast<const float4 *>(p + step_r + nz));
+            c[u][0] = ld_data4(p);
+            c[u][1] = ld_data4(p + nz);
+            c[u][2] = ld_data4(p + step_r);
+            c[u][3] = ld_data4(p + step_r + nz);
             a[u] = Ap ? __ldg(reinterpret_cast<const float4 *>(Ap + u * g.nzs))
                       : make_float4(1.f, 1.f, 1.f, 1.f);
         }
@@ -250,10 +245,10 @@ __device__ __forceinline__ void gather_rows(const float *__restrict__ f, const S
         const RowTap t = rt[u];
         const int m = zin ? t.mask : 0;
         const float *p = f + t.off + 4 * q;
-        const float4 vnw = (m & 1) ? ld_quad(p, 4 * q, nz, vec) : zero;
-        const float4 vne = (m & 2) ? ld_quad(p + nz, 4 * q, nz, vec) : zero;
-        const float4 vsw = (m & 4) ? ld_quad(p + step_r, 4 * q, nz, vec) : zero;
-        const float4 vse = (m & 8) ? ld_quad(p + step_r + nz, 4 * q, nz, vec) : zero;
+        const float4 vnw = ld_quad(m & 1, p, 4 * q, nz, vec);
+        const float4 vne = ld_quad(m & 2, p + nz, 4 * q, nz, vec);
+        const float4 vsw = ld_quad(m & 4, p + step_r, 4 * q, nz, vec);
+        const float4 vse = ld_quad(m & 8, p + step_r + nz, 4 * q, nz, vec);
         const float4 a = Ap && m ? __ldg(reinterpret_cast<const float4 *>(Ap + u * g.nzs)) : zero;
         Bilin b;
         b.nw = t.nw;
@@ -274,7 +269,7 @@ __device__ __forceinline__ void gather_rows(const float *__restrict__ f, const S
 }
 
 template <int QL, int HB>
-__device__ __forceinline__ void fwd_strip_item(const SpectDev &g, const float *__restrict__ f,
+__device__ __forceinline__ void fwd_strip_item(const SpectDev &g, const float *f,
                                                const int ga, const int x0, const int x1,
                                                float *__restrict__ Ws, float *__restrict__ sm) {
     constexpr int G = 32 / QL, RS = 8 * G, ZG = QL / 4, PS = strip_pair(QL, HB);
@@ -373,7 +368,7 @@ __device__ __forceinline__ void fwd_strip_item(const SpectDev &g, const float *_
 
 template <int QL, int HB>
 __global__ void __launch_bounds__(512, 1)
-    k_fwd_strip(SpectDev g, const float *__restrict__ f, const int *__restrict__ alist,
+    k_fwd_strip(SpectDev g, const float *f, const int *__restrict__ alist,
                 const int4 *__restrict__ items, float *__restrict__ W) {
     extern __shared__ __align__(128) float sm[];
     grid_release();
@@ -428,7 +423,7 @@ __host__ __device__ inline YsumLayout ysum_layout(const SpectDev &g) {
 
 // Ws: the slot's W rows; out: the item's partial ray sums [N][nz].  Whole-CTA call of at least
 // nw + 1 warps, nw = ceil(N / 32).
-__device__ __forceinline__ void ysum_item(const SpectDev &g, const float *__restrict__ Ws,
+__device__ __forceinline__ void ysum_item(const SpectDev &g, const float *Ws,
                                           const int ga, const int x0, const int x1,
                                           const int slab, float *__restrict__ out,
                                           float *__restrict__ sm, unsigned long long *full,
@@ -530,7 +525,7 @@ __device__ __forceinline__ void ysum_item(const SpectDev &g, const float *__rest
 
 __global__ void __launch_bounds__(160, 4)
     k_fwd_ysum(SpectDev g, const int *__restrict__ alist, const int4 *__restrict__ items,
-               const float *__restrict__ W, float *__restrict__ partials) {
+               const float *W, float *partials) {
     extern __shared__ __align__(128) float sm[];
     __shared__ unsigned long long full[kYStages], empty[kYStages];
     grid_release();
