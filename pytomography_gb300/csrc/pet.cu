@@ -315,7 +315,6 @@ struct gb_pet_plan {
     PetPatches osem_patch{}, call_patch{};
     std::mutex call_lock;
     cudaEvent_t call_done = nullptr;  // end of the layout's last use
-    cudaStream_t call_stream = nullptr;
     bool call_used = false;
 };
 
@@ -452,7 +451,8 @@ static bool fwd_patches_pay(const PetDev &g, long long n, bool tof) {
 
 // Forward and back projections of one plan may run on several streams and threads at once, so
 // the layout they share is lent to one at a time: the host lock is held while a call enqueues
-// its kernels, and a call on another stream than the last one's waits for that one's end.  A
+// its kernels, and its stream waits for the end of the last use (on the same stream as well: one
+// handle may name two streams, the per-thread default stream or a destroyed one used again).  A
 // capturing stream cannot wait for outside work (and its graph would not take turns later):
 // there, and where the plan has no layout, `q` stays null and the call goes without.
 struct PatchLease {
@@ -466,8 +466,7 @@ struct PatchLease {
         }
         if (cs != cudaStreamCaptureStatusNone) return;
         p->call_lock.lock();
-        if (p->call_used && p->call_stream != st &&
-            cudaStreamWaitEvent(st, p->call_done) != cudaSuccess) {
+        if (p->call_used && cudaStreamWaitEvent(st, p->call_done) != cudaSuccess) {
             cudaGetLastError();
             p->call_lock.unlock();
             return;
@@ -476,9 +475,11 @@ struct PatchLease {
     }
     ~PatchLease() {
         if (!q.qx) return;
-        cudaEventRecord(plan->call_done, st);
-        plan->call_stream = st;
-        plan->call_used = true;
+        plan->call_used = cudaEventRecord(plan->call_done, st) == cudaSuccess;
+        if (!plan->call_used) {  // no event to wait for: the next use must find this one over
+            cudaGetLastError();
+            cudaStreamSynchronize(st);
+        }
         plan->call_lock.unlock();
     }
     PatchLease(const PatchLease &) = delete;
