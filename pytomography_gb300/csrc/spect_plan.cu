@@ -710,15 +710,13 @@ gb_status gb_spect_plan_create(const gb_spect_desc *d, gb_spect_plan **out) {
                 }
             }
         // tap tier of every plane: the narrowest unrolled loop that holds its nonzero taps
-        if (!d->psf_2d)  // the strip kernels' z pass copies the plane then
-            for (size_t r = 0; r < (size_t)ng * Lp; r++) tz[r * K + K / 2] = 1.f;
         std::vector<signed char> tier((size_t)ng * Lp, kTiers - 1);
         std::vector<signed char> ladder((size_t)ng * Lp, 0);
         const int Hk = K / 2;
         for (int gi = 0; gi < ng; gi++)
             for (int x = 0; x < Lp; x++) {
                 int h = 0;
-                for (int which = 0; which < 2; which++) {
+                for (int which = 0; which < (d->psf_2d ? 2 : 1); which++) {
                     const std::vector<float> &tab = which == 0 ? tr : tz;
                     for (int t = 0; t < K; t++)
                         if (tab[((size_t)gi * Lp + x) * K + t] != 0.f) h = std::max(h, std::abs(t - Hk));

@@ -61,7 +61,7 @@ __device__ __forceinline__ float4 ldg_here(const float *p) {
     return v;
 }
 
-template <int QL, int HB>
+template <int QL, int HB, bool Z2>
 __device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *P,
                                               const int ga, const int x0, const int x1,
                                               float *__restrict__ Ws, float *__restrict__ sm) {
@@ -116,7 +116,10 @@ __device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *P,
                 }
                 __syncwarp();
                 float2 o[16];
-                strip_z_pass<KK, HB>(buf + pr * PS + 18 * c, tap + kStripTaps, o);
+                if constexpr (Z2)
+                    strip_z_pass<KK, HB>(buf + pr * PS + 18 * c, tap + kStripTaps, o);
+                else
+                    strip_z_copy<HB>(buf + pr * PS + 18 * c, o);
                 __syncwarp();  // the buffer is free for the next strip
                 const size_t off = ((size_t)xp * g.nya + (y - g.ya_lo)) * g.nzs + 4 * c;
                 const bool st0 = c < g.zg && y <= yl, st1 = c < g.zg && y + 1 <= yl;
@@ -144,19 +147,37 @@ __device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *P,
     }
 }
 
-template <int QL, int HB>
+template <int QL, int HB, bool Z2>
 __global__ void __launch_bounds__(512, 1)
     k_b1_strip(SpectDev g, const float *proj, const int *__restrict__ alist,
                const int4 *__restrict__ items, float *__restrict__ W) {
     extern __shared__ __align__(128) float sm[];
     grid_release();
     const int4 item = items[blockIdx.x];
-    b1_strip_item<QL, HB>(g, proj + (size_t)item.x * g.N * g.nz, alist[item.x], item.y, item.z,
+    b1_strip_item<QL, HB, Z2>(g, proj + (size_t)item.x * g.N * g.nz, alist[item.x], item.y, item.z,
                           W + (size_t)item.x * g.Lp * g.nya * g.nzs, sm);
 }
 
+// Calls f(QL, Z2) (as types) for a batch entry: the lanes of its rows, whether the PSF blurs z.
+template <typename F>
+__device__ __forceinline__ void strip_dispatch(const SpectDev &g, F &&f) {
+    const int ql = strip_ql(g.nz);
+    auto both = [&](auto q) {
+        if (g.psf2d)
+            f(q, std::true_type{});
+        else
+            f(q, std::false_type{});
+    };
+    if (ql == 32)
+        both(std::integral_constant<int, 32>{});
+    else if (ql == 16)
+        both(std::integral_constant<int, 16>{});
+    else
+        both(std::integral_constant<int, 8>{});
+}
+
 // Persistent batch form: one CTA per SM dequeues the work items of every entry, largest
-// first.  The entries share the tap bucket (HB); their row widths may differ.
+// first.  The entries share the tap bucket (HB); their row widths and PSF dimensions may differ.
 template <int HB>
 __global__ void __launch_bounds__(512, 1) k_b1_strip_batch(const __grid_constant__ B1Batch p) {
     extern __shared__ __align__(128) float sm[];
@@ -173,11 +194,10 @@ __global__ void __launch_bounds__(512, 1) k_b1_strip_batch(const __grid_constant
         const float *P = p.proj[e] + (size_t)slot * g.N * g.nz;
         const int ga = p.alist[e][slot];
         float *W = p.W[e] + (size_t)slot * g.Lp * g.nya * g.nzs;
-        switch (strip_ql(g.nz)) {
-            case 32: b1_strip_item<32, HB>(g, P, ga, item.y, item.z, W, sm); break;
-            case 16: b1_strip_item<16, HB>(g, P, ga, item.y, item.z, W, sm); break;
-            default: b1_strip_item<8, HB>(g, P, ga, item.y, item.z, W, sm); break;
-        }
+        strip_dispatch(g, [&](auto ql, auto z2) {
+            b1_strip_item<decltype(ql)::value, HB, decltype(z2)::value>(g, P, ga, item.y, item.z,
+                                                                        W, sm);
+        });
     }
 }
 
@@ -342,25 +362,33 @@ __device__ __forceinline__ void fwd_strip_item(const SpectDev &g, const float *f
         const float *tap = taps + (xp - x0) * kStripTaps;
         const int y = y0 + 2 * pr;
         float *Wp = Ws + ((size_t)xp * ns * g.nya + (y - g.ya_lo)) * 32;
+        auto store = [&](const float2 (&o)[16]) {
+            __syncwarp();  // the buffer is free for the next strip
+            if (c >= g.zg) return;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int pos = k * g.zg + c;
+                float *d = Wp + (size_t)(pos >> 3) * g.nya * 32 + 4 * (pos & 7);
+                if (y <= yl)
+                    *reinterpret_cast<float4 *>(d) =
+                        make_float4(o[4 * k].x, o[4 * k + 1].x, o[4 * k + 2].x, o[4 * k + 3].x);
+                if (y + 1 <= yl)
+                    *reinterpret_cast<float4 *>(d + 32) =
+                        make_float4(o[4 * k].y, o[4 * k + 1].y, o[4 * k + 2].y, o[4 * k + 3].y);
+            }
+        };
+        if (!g.psf2d) {
+            float2 o[16];
+            strip_z_copy<HB>(buf + pr * PS + 18 * c, o);
+            store(o);
+            continue;
+        }
         ladder_dispatch(pi.w & 15, [&](auto kk) {
             constexpr int KK = decltype(kk)::value;
             if constexpr (KK / 2 <= HB) {
                 float2 o[16];
                 strip_z_pass<KK, HB>(buf + pr * PS + 18 * c, tap, o);
-                __syncwarp();  // the buffer is free for the next strip
-                if (c < g.zg) {
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const int pos = k * g.zg + c;
-                        float *d = Wp + (size_t)(pos >> 3) * g.nya * 32 + 4 * (pos & 7);
-                        if (y <= yl)
-                            *reinterpret_cast<float4 *>(d) = make_float4(
-                                o[4 * k].x, o[4 * k + 1].x, o[4 * k + 2].x, o[4 * k + 3].x);
-                        if (y + 1 <= yl)
-                            *reinterpret_cast<float4 *>(d + 32) = make_float4(
-                                o[4 * k].y, o[4 * k + 1].y, o[4 * k + 2].y, o[4 * k + 3].y);
-                    }
-                }
+                store(o);
             }
         });
     }
@@ -591,8 +619,8 @@ cudaError_t launch_b1_strip(const SpectDev &g, const float *proj, const int *ali
     const size_t smem = b1_strip_layout(g, QL, warps).total * sizeof(float);
 #define GB_CASE(Q, B)                                                                        \
     if (QL == Q && HB == B)                                                                  \
-        return launch_dependent(k_b1_strip<Q, B>, n_items, 32 * warps, smem, st, g, proj,     \
-                                alist, items, W);
+        return launch_dependent(g.psf2d ? k_b1_strip<Q, B, true> : k_b1_strip<Q, B, false>,  \
+                                n_items, 32 * warps, smem, st, g, proj, alist, items, W);
     GB_FOR_EACH_STRIP(GB_CASE)
 #undef GB_CASE
     return cudaErrorInvalidValue;
@@ -653,7 +681,8 @@ cudaError_t setup_strip(size_t cap) {
           (const void *)k_fwd_ysum, (const void *)k_fwd_ysum_batch})
         if ((e = raise(fn)) != cudaSuccess) return e;
 #define GB_CASE(Q, B)                                                        \
-    if ((e = raise((const void *)k_b1_strip<Q, B>)) != cudaSuccess ||        \
+    if ((e = raise((const void *)k_b1_strip<Q, B, true>)) != cudaSuccess ||  \
+        (e = raise((const void *)k_b1_strip<Q, B, false>)) != cudaSuccess || \
         (e = raise((const void *)k_fwd_strip<Q, B>)) != cudaSuccess)         \
         return e;
     GB_FOR_EACH_STRIP(GB_CASE)

@@ -146,6 +146,19 @@ __device__ __forceinline__ void strip_z_pass(const float2 *__restrict__ bp,
     }
 }
 
+// The z pass of a 1-D PSF: the lane's 16 values as they are (a pass of one tap of 1 and zeros
+// would spread an infinity or NaN over the taps' width).
+template <int HB>
+__device__ __forceinline__ void strip_z_copy(const float2 *__restrict__ bp, float2 (&o)[16]) {
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+        const int rel = HB + j;
+        const float4 v = *reinterpret_cast<const float4 *>(bp + rel + 2 * (rel >> 4));
+        o[j] = make_float2(v.x, v.y);
+        o[j + 1] = make_float2(v.z, v.w);
+    }
+}
+
 // Shared bookkeeping of one work item (planes [x0, x1) of one angle, at most kStripPlanes):
 // its occupied planes in order and the plane of every strip.
 struct StripItem {
