@@ -658,9 +658,9 @@ __device__ __forceinline__ float rdp_sum(const float *f, int nx, int ny, int nz,
     return acc;
 }
 
-// rdp_sum for the four voxels z..z+3 of a z quad (z % 4 == 0, nz % 4 == 0), used by the
-// fused BSREM step: each (x, y) neighbour row is loaded once (z-1, the quad, z+4,
-// clamped), and every voxel adds its 26 terms in rdp_sum's order.  FAST: a term is
+// rdp_sum for the four voxels z..z+3 of a z quad (z % 4 == 0), used by the fused BSREM step:
+// each (x, y) neighbour row is loaded once (z-1, the quad, z+4, clamped; QUAD: nz % 4 == 0, the
+// quad in one piece), and every voxel adds its 26 terms in rdp_sum's order.  FAST: a term is
 // num / den^2 with num = d (den + 2 f_s + delta), that is d/den (1 + (2 f_s + delta)/den): one
 // fast reciprocal (1 ulp) of den, seven other instructions and no branch, where the division
 // by den^2 with its range test took about twenty; what depends on f_s alone is made once per
@@ -674,7 +674,7 @@ __device__ __forceinline__ float fast_rcp(float x) {
     return r;
 }
 
-template <bool FAST>
+template <bool FAST, bool QUAD>
 __device__ __forceinline__ void rdp_sum4(const float *f, int nx, int ny, int nz,
                                          int x, int y, int z, const float (&fr)[4],
                                          const UpdateArgs &u, float (&acc)[4], float &low) {
@@ -686,9 +686,19 @@ __device__ __forceinline__ void rdp_sum4(const float *f, int nx, int ny, int nz,
         const int xi = min(max(x + ij / 3 - 1, 0), nx - 1);
         const int yj = min(max(y + ij % 3 - 1, 0), ny - 1);
         const float *p = f + ((size_t)xi * ny + yj) * nz;
-        const float4 c = ld_data4(p + z);
-        const float row[6] = {ld_data(p + max(z - 1, 0)), c.x, c.y, c.z, c.w,
-                              ld_data(p + min(z + 4, nz - 1))};
+        float row[6];
+        if constexpr (QUAD) {
+            const float4 c = ld_data4(p + z);
+            row[0] = ld_data(p + max(z - 1, 0));
+            row[1] = c.x;
+            row[2] = c.y;
+            row[3] = c.z;
+            row[4] = c.w;
+            row[5] = ld_data(p + min(z + 4, nz - 1));
+        } else {
+#pragma unroll
+            for (int m = 0; m < 6; m++) row[m] = ld_data(p + min(max(z - 1 + m, 0), nz - 1));
+        }
         float sd[6], s2[6];  // f_s + delta, 2 f_s + delta
         if (FAST) {
 #pragma unroll
@@ -818,30 +828,38 @@ __device__ __forceinline__ void apply_update(int mode, const UpdateArgs &u, size
     }
 }
 
-// apply_update for the z quad z..z+3 (z % 4 == 0; values from nz on are left out).  PRIOR (BSREM with the
-// RDP prior): the prior term comes from rdp_sum4, one neighbourhood load for the four
-// voxels; a separate instantiation, so the other modes keep their register count.
-template <bool PRIOR>
+// Prior term of a gather kernel's epilogue, a separate instantiation each: none (or a step that
+// never has one), z quads whole (nz % 4 == 0), the last quad of a row partial.
+enum PriorRows { NO_PRIOR, PRIOR_QUADS, PRIOR_RAGGED };
+
+// apply_update for the z quad z..z+3 (z % 4 == 0; values from nz on are left out).  With a prior
+// (BSREM), its term comes from rdp_sum4, one neighbourhood load for the four voxels.  (Ragged
+// rows a voxel at a time, with the exact divisions of rdp_sum: 12 BSREM steps of 5 angles at
+// 40 x 40 x 39 took 1054 us, this way 736.)
+template <PriorRows PRIOR>
 __device__ __forceinline__ void apply_update4(int mode, const UpdateArgs &u, size_t i, int x,
                                               int y, int z, int nx, int ny, int nz, float4 bp4,
                                               float *out) {
     const float bp[4] = {bp4.x, bp4.y, bp4.z, bp4.w};
-    if (!PRIOR || nz % 4 != 0) {  // the last quad of a row may be partial
+    if constexpr (PRIOR == NO_PRIOR) {
 #pragma unroll
         for (int v = 0; v < 4; v++)
             if (z + v < nz)
-                apply_update<PRIOR>(mode, u, i + v, x, y, z + v, nx, ny, nz, bp[v], out);
+                apply_update<false>(mode, u, i + v, x, y, z + v, nx, ny, nz, bp[v], out);
         return;
     }
+    constexpr bool QUAD = PRIOR == PRIOR_QUADS;
+    const int nv = QUAD ? 4 : min(4, nz - z);  // voxels of the quad
     float f[4], rdp[4];
 #pragma unroll
-    for (int v = 0; v < 4; v++) f[v] = u.f_in[i + v];
+    for (int v = 0; v < 4; v++) f[v] = u.f_in[i + (QUAD ? v : min(v, nv - 1))];
     float low = 1.f;
-    rdp_sum4<true>(u.f_in, nx, ny, nz, x, y, z, f, u, rdp, low);
+    rdp_sum4<true, QUAD>(u.f_in, nx, ny, nz, x, y, z, f, u, rdp, low);
     if (low < 8.8818e-16f)  // 2^-50
-        rdp_sum4<false>(u.f_in, nx, ny, nz, x, y, z, f, u, rdp, low);
+        rdp_sum4<false, QUAD>(u.f_in, nx, ny, nz, x, y, z, f, u, rdp, low);
 #pragma unroll
     for (int v = 0; v < 4; v++) {
+        if (!QUAD && v >= nv) break;
         float b = bp[v];
         if (u.acc) b = __fadd_rn(u.acc[i + v], b);
         const float nb = u.nbp[i + v];
@@ -1043,7 +1061,7 @@ constexpr int kB2Unroll = 2;
 // latency of the A reads, like k_b2_gather4 by those of W.  OSEM iteration of 8 subsets of 8
 // angles at 64^3: 213 -> 185 us; BSREM, 10 subsets of 9 angles of 96 x 96 x 128: 1300 -> 905 us
 // (with the prior's shorter terms).
-template <bool PRIOR>
+template <PriorRows PRIOR>
 __global__ void __launch_bounds__(256)
     k_b2_nopsf4(SpectDev g, const float *proj, const int *__restrict__ alist,
                 int n_slots, float *out, int mode, UpdateArgs u) {
@@ -1093,8 +1111,8 @@ __global__ void __launch_bounds__(256)
 
 // (Blocks an SM: five of 48 registers without the prior, which waits for W and gains from warps,
 // 95.6 us against 98.2 for four at 128^3, 12 angles; four of 64 with it.)
-template <bool PRIOR>
-__global__ void __launch_bounds__(256, PRIOR ? 4 : 5)
+template <PriorRows PRIOR>
+__global__ void __launch_bounds__(256, PRIOR == NO_PRIOR ? 5 : 4)
     k_b2_gather4(SpectDev g, const float *W, const int *__restrict__ alist,
                  int n_slots, float *out, int mode, UpdateArgs u) {
     __shared__ B2Tap tab[kB2Taps];
@@ -1172,7 +1190,7 @@ __global__ void __launch_bounds__(256) k_b2_gather_batch(const __grid_constant__
     u.f = p.out[e];
     u.nbp = p.nbp[e];
     u.acc = p.acc[e];
-    apply_update4<false>(p.mode[e], u, i, x, y, z, N, N, nz, bp, p.out[e]);
+    apply_update4<NO_PRIOR>(p.mode[e], u, i, x, y, z, N, N, nz, bp, p.out[e]);
 }
 
 cudaError_t launch_b2_gather_batch(const B2Batch &p, int n_blocks, cudaStream_t st) {
@@ -1222,7 +1240,8 @@ cudaError_t launch_b2_nopsf(const SpectDev &g, const float *proj, const int *ali
                             float *out, int mode, const UpdateArgs &u, cudaStream_t st) {
     const dim3 b4 = b2_block(g);
     const dim3 grid((g.nz / 4 + b4.x - 1) / b4.x, (g.N + b4.y - 1) / b4.y, g.N);
-    return launch_dependent(mode == B2_BSREM && u.prior ? k_b2_nopsf4<true> : k_b2_nopsf4<false>,
+    return launch_dependent(mode == B2_BSREM && u.prior ? k_b2_nopsf4<PRIOR_QUADS>
+                                                        : k_b2_nopsf4<NO_PRIOR>,
                             grid, b4, 0, st, g, proj, alist, n_slots, out, mode, u);
 }
 
@@ -1234,8 +1253,10 @@ cudaError_t launch_b2_gather(const SpectDev &g, const float *W, const int *alist
         const dim3 b4 = b2_block(g);
         dim3 grid((qx + b4.x - 1) / b4.x, (g.N + b4.y - 1) / b4.y, g.N);
         block = b4;
-        return launch_dependent(mode == B2_BSREM && u.prior ? k_b2_gather4<true> : k_b2_gather4<false>,
-                                grid, block, 0, st, g, W, alist, n_slots, out, mode, u);
+        auto *fn = mode != B2_BSREM || !u.prior ? k_b2_gather4<NO_PRIOR>
+                   : g.nz % 4 == 0              ? k_b2_gather4<PRIOR_QUADS>
+                                                : k_b2_gather4<PRIOR_RAGGED>;
+        return launch_dependent(fn, grid, block, 0, st, g, W, alist, n_slots, out, mode, u);
     } else {
         dim3 grid((g.nz + 31) / 32, (g.N + 7) / 8, g.N);
         k_b2_gather<<<grid, block, 0, st>>>(g, W, alist, n_slots, out, mode, u);
