@@ -1253,10 +1253,10 @@ cudaError_t launch_b2_gather(const SpectDev &g, const float *W, const int *alist
         const dim3 b4 = b2_block(g);
         dim3 grid((qx + b4.x - 1) / b4.x, (g.N + b4.y - 1) / b4.y, g.N);
         block = b4;
-        auto *fn = mode != B2_BSREM || !u.prior ? k_b2_gather4<NO_PRIOR>
-                   : g.nz % 4 == 0              ? k_b2_gather4<PRIOR_QUADS>
-                                                : k_b2_gather4<PRIOR_RAGGED>;
-        return launch_dependent(fn, grid, block, 0, st, g, W, alist, n_slots, out, mode, u);
+        return launch_dependent(mode != B2_BSREM || !u.prior ? k_b2_gather4<NO_PRIOR>
+                                : g.nz % 4 == 0              ? k_b2_gather4<PRIOR_QUADS>
+                                                             : k_b2_gather4<PRIOR_RAGGED>,
+                                grid, block, 0, st, g, W, alist, n_slots, out, mode, u);
     } else {
         dim3 grid((g.nz + 31) / 32, (g.N + 7) / 8, g.N);
         k_b2_gather<<<grid, block, 0, st>>>(g, W, alist, n_slots, out, mode, u);
