@@ -7,10 +7,10 @@
 // plane_z[p][1]) (_get_xyz_sinogram_coordinates, :50-85); subsets are angles i::n
 // (:131-144).  TOF sinograms hold every bin of every LOR (bin fastest); one thread traces
 // one (LOR, bin) restricted to that bin's TOF window, so the threads of a warp trace the
-// bins of the same or neighbouring LORs.  That is the form for images with more slices than
-// profiles that fit shared memory and for the rare LORs steeper than 45 degrees; every other LOR takes the
-// line kernels (k_sino_fwd_line, k_sino_bwd_line), which use that all ring pairs of a
-// transaxial line share its path.  The listmode binning restates
+// bins of the same or neighbouring LORs.  That is the form for few ring pairs or many slices
+// (line_pays) and for the rare LORs steeper than 45 degrees; every other LOR takes the line
+// kernels (k_sino_fwd_line, k_sino_bwd_line), which use that all ring pairs of a transaxial line
+// share its path.  The listmode binning restates
 // listmode_to_sinogram / _listmodeTOF_to_sinogramTOF (io/PET/shared.py:175-272).
 #include <algorithm>
 #include <cmath>
@@ -411,10 +411,62 @@ static size_t fwd_line_smem(const PetDev &g, bool tof) {
     return sizeof(float) * (((size_t)fwd_line_chunk(g) * (g.n[2] + 2) + 3) / 4 * 4 +
                             (tof ? kTofTabLen : 0));
 }
-// The line kernels need the profiles of 128 planes (and the TOF table and values) in shared
-// memory: up to 390 slices.
-static bool line_ok(const PetDev &g, int nb, bool tof) {
+static int bwd_line_threads(const PetDev &g) {
+    const int nk = std::max(g.n[0], g.n[1]);
+    return nk <= 32 ? 32 : nk <= 64 ? 64 : nk <= 96 ? 96 : 128;
+}
+// The line kernels' tiles must fit: the back projection's profiles of 128 planes (446 slices
+// without TOF, 407 with 13 bins).
+static bool line_fits(const PetDev &g, int nb, bool tof) {
     return bwd_line_smem(g.n[2], 128, nb, tof) <= 225 * 1024 && fwd_line_smem(g, tof) <= 225 * 1024;
+}
+// Planes that the LORs of a line add up, as multiples of the planes of the image.
+static double line_work(const PetDev &g, int P, int nb, bool tof) {
+    if (!tof) return P;
+    const double nk = std::max(g.n[0], g.n[1]);
+    const double win = (2.0 * (g.nsig * g.sig) + g.bw) / std::min(g.vox[0], g.vox[1]);
+    return (double)P * nb * std::min(win, nk) / nk;
+}
+// Blocks of an SM by their shared memory (228 KB, 1 KB of it reserved for each).
+static int sm_blocks(size_t smem) { return (int)(228 * 1024 / (smem + 1024)); }
+
+// Whether the line kernels pay: they blend (forward) or clear and add (back) nz values per plane
+// and line whatever the number P of ring pairs is, and their tiles leave few blocks to an SM
+// when nz is large; tracing each LOR costs the same for any nz.  Measured, traced -> line, us
+// (4515 lines, 128 x 128 x nz of 4 mm, 13 TOF bins over 650 mm, FWHM 58.5 mm):
+//   nz               8            24           48           100            200            380
+//   forward    P=16  43 -> 41     43 -> 56     43 -> 85     43 -> 197      43 -> 560      43 -> 996
+//              P=64  105 -> 45    106 -> 60    105 -> 88    105 -> 199     106 -> 562     105 -> 1002
+//              P=144 197 -> 75    198 -> 86                 199 -> 191     198 -> 499     199 -> 868
+//   TOF        P=4   60 -> 55     61 -> 76     64 -> 112    62 -> 247      62 -> 579      62 -> 1076
+//              P=16  189 -> 110   189 -> 126   192 -> 150   190 -> 204     190 -> 422     190 -> 754
+//              P=64  704 -> 322   705 -> 338   713 -> 363   710 -> 417     709 -> 744     711 -> 1238
+//              P=144                                                       1612 -> 1410   1602 -> 2245
+//   back       P=1   39 -> 24     40 -> 25     39 -> 28     39 -> 42       40 -> 86       42 -> 213
+//              P=16  102 -> 27    100 -> 29    96 -> 31     80 -> 49       95 -> 96       83 -> 236
+//              P=144 348 -> 61    386 -> 65                 357 -> 109     350 -> 205     348 -> 449
+//   TOF        P=1   49 -> 29     48 -> 35     47 -> 43     33 -> 62       47 -> 168      35 -> 241
+//              P=16  214 -> 65    197 -> 76    197 -> 97    174 -> 131     190 -> 357     176 -> 434
+//              P=64  683 -> 191   634 -> 218   634 -> 282   639 -> 366     606 -> 1004    647 -> 1133
+// A forward of more slices than are staged at once re-reads its sums: 908 -> 946 us at 200 slices
+// and P=784 without TOF; with TOF 3635 -> 2676 at 200 slices, 3619 -> 4160 at 380 (P=324).
+static bool line_pays(const PetDev &g, int P, int nb, bool tof, bool back) {
+    if (!line_fits(g, nb, tof)) return false;
+    const int nk = std::max(g.n[0], g.n[1]), nz = g.n[2];
+    const double work = line_work(g, P, nb, tof);
+    if (back) {
+        const int T = bwd_line_threads(g);
+        const int warps = sm_blocks(bwd_line_smem(nz, T, nb, tof)) * T / 32;
+        return tof ? warps >= (T >= 96 ? 8 : 10) && work >= nz - 70
+                   : warps >= 8 && 8 * work >= nz - 64;
+    }
+    const size_t all = sizeof(float) * nk * ((size_t)nz + 2);
+    if (all > (tof ? 165 * 1024 : kLineStage)) return false;
+    if (tof && (long long)P * nb < 48) return false;  // (the 16 KB weight table of a block)
+    const int blocks = sm_blocks(fwd_line_smem(g, tof));
+    const double per_slice = tof ? (blocks >= 3 ? 1.2 : 3.1)
+                                 : (blocks >= 7 ? 1.2 : blocks >= 4 ? 1.6 : 4.0);
+    return work >= per_slice * (nz + 4);
 }
 static cudaError_t setup_lines() {
     cudaError_t e;
@@ -439,7 +491,7 @@ static cudaError_t sino_forward(gb_pet_sino_plan *p, const float *img, float *pr
                                 int stride, int n, bool tof, int atten, cudaStream_t st) {
     const int nb = tof ? p->nb : 1;
     const int lines = n * p->geom.R;
-    if (line_ok(p->dev, nb, tof)) {
+    if (line_pays(p->dev, p->geom.P, nb, tof, false)) {
         const dim3 grid(lines, line_split(lines, p->geom.P));
         const size_t smem = fwd_line_smem(p->dev, tof);
         const int chunk = fwd_line_chunk(p->dev);
@@ -604,9 +656,8 @@ gb_status gb_pet_sino_backward(gb_pet_sino_plan *p, const float *proj, float *im
                             (size_t)p->dev.n[0] * p->dev.n[1] * p->dev.n[2] * sizeof(float), st));
     if (total == 0) return GB_OK;
     const int nb = tof ? p->nb : 1;
-    if (line_ok(p->dev, nb, tof)) {
-        const int nk = std::max(p->dev.n[0], p->dev.n[1]);
-        const int T = nk <= 32 ? 32 : nk <= 64 ? 64 : nk <= 96 ? 96 : 128;
+    if (line_pays(p->dev, p->geom.P, nb, tof, true)) {
+        const int nk = std::max(p->dev.n[0], p->dev.n[1]), T = bwd_line_threads(p->dev);
         const int chunks = (nk + T - 1) / T, lines = n * p->geom.R;
         const dim3 grid(lines, chunks, line_split(lines * chunks, p->geom.P));
         const size_t smem = bwd_line_smem(p->dev.n[2], T, nb, tof);
