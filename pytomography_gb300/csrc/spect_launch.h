@@ -152,12 +152,20 @@ cudaError_t launch_b2_adjoint_batch(const B2Batch &p, int n_blocks, cudaStream_t
 // blocks of 256 threads of one entry in the batched gather and adjoint kernels
 int b2_gather_blocks(const SpectDev &g);
 
-// One forward projection of a plan with the caller's partial-sum buffer (for entry points
-// defined outside spect_plan.cu): the work items and partial floats a subset needs (false when
-// the subset is out of range), and the projection itself.
+// Scratch of gb_spect_forward_static: partial sums, and the strip kernels' rows of as many
+// angles at a time as fit (static_slots).
+struct StaticScratch {
+    float *partials, *rows;
+};
+constexpr size_t kStaticPartials = (size_t)4 << 20, kStaticRows = (size_t)16 << 20;  // floats
+inline int static_slots(const SpectDev &g) { return (int)(kStaticRows / stack_slot(g)); }
+
+// One forward projection of a plan in that scratch (for entry points defined outside
+// spect_plan.cu): the work items and partial floats a subset needs (false when the subset is out
+// of range), and the projection itself.
 bool plan_forward_need(const gb_spect_plan *p, int subset, int *n_sel, int *n_items,
                        size_t *floats);
 gb_status plan_forward(gb_spect_plan *p, const float *obj, int subset, float *out,
-                       float *partials, cudaStream_t st);
+                       const StaticScratch &fixed, cudaStream_t st);
 
 }  // namespace gb

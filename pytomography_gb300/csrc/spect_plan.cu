@@ -192,7 +192,8 @@ struct gb_spect_plan {
     struct List {
         int alist_off = 0, n = 0;
         std::vector<FwdGroup> fgroups;
-        int max_fitems = 0;  // largest group's items
+        std::vector<FwdGroup> sgroups;  // the groups of gb_spect_forward_static
+        int max_fitems = 0, max_sitems = 0;  // largest group's items
         std::vector<int> gitem_off, n_gitems;  // B1 items of each angle group
         int b_half = 0;  // first group-0 B1 item of slot n / 2
     };
@@ -431,45 +432,58 @@ static gb_status upload_lists(gb_spect_plan *p, int n_subsets,
         L.alist_off = (int)all.size();
         L.n = (int)l.size();
         all.insert(all.end(), l.begin(), l.end());
-        // forward items
-        const int gf = p->dev.strip ? p->G : L.n;
-        for (int a0 = 0; a0 < L.n; a0 += gf) {
-            gb_spect_plan::FwdGroup F;
-            F.a0 = a0;
-            F.n = std::min(gf, L.n - a0);
-            F.item_off = (int)items.size();
-            F.ioff_off = (int)ioff.size();
-            std::vector<int> cnt(F.n, psf ? 0 : nopsf_chunks(p, L.n));
-            if (psf) {
-                std::vector<double> wa(F.n);
-                for (int i = 0; i < F.n; i++) wa[i] = sum_of(wf[l[a0 + i]]);
-                cnt = chunk_counts(p, wa, zs_f, p->fwd_items);
-            }
-            for (int i = 0; i < F.n; i++) {
-                ioff.push_back((int)items.size() - F.item_off);
-                if (i == F.n / 2) F.half = (int)items.size() - F.item_off;
-                if (psf)
-                    split_planes(wf[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p), kStripEmpty);
-                else
-                    for (int k = 0; k < cnt[i]; k++)
-                        items.push_back(
-                            make_int4(i, k * p->Lp / cnt[i], (k + 1) * p->Lp / cnt[i], 0));
-            }
-            F.n_items = (int)items.size() - F.item_off;
-            ioff.push_back(F.n_items);
-            L.max_fitems = std::max(L.max_fitems, F.n_items);
-            if (p->dev.strip) {
-                F.gather_off = (int)items.size();
-                std::vector<double> wa(F.n);
-                for (int i = 0; i < F.n; i++) wa[i] = sum_of(wg[l[a0 + i]]);
-                cnt = chunk_counts(p, wa, 1);
-                for (int i = 0; i < F.n; i++) {
-                    if (i == F.n / 2) F.gather_half = (int)items.size() - F.gather_off;
-                    split_planes(wg[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p), kStripEmpty);
+        // forward items, gf angles a group
+        auto forward_groups = [&](int gf, std::vector<gb_spect_plan::FwdGroup> &groups) {
+            int most = 0;
+            for (int a0 = 0; a0 < L.n; a0 += gf) {
+                gb_spect_plan::FwdGroup F;
+                F.a0 = a0;
+                F.n = std::min(gf, L.n - a0);
+                F.item_off = (int)items.size();
+                F.ioff_off = (int)ioff.size();
+                std::vector<int> cnt(F.n, psf ? 0 : nopsf_chunks(p, L.n));
+                if (psf) {
+                    std::vector<double> wa(F.n);
+                    for (int i = 0; i < F.n; i++) wa[i] = sum_of(wf[l[a0 + i]]);
+                    cnt = chunk_counts(p, wa, zs_f, p->fwd_items);
                 }
-                F.n_gather = (int)items.size() - F.gather_off;
+                for (int i = 0; i < F.n; i++) {
+                    ioff.push_back((int)items.size() - F.item_off);
+                    if (i == F.n / 2) F.half = (int)items.size() - F.item_off;
+                    if (psf)
+                        split_planes(wf[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p),
+                                     kStripEmpty);
+                    else
+                        for (int k = 0; k < cnt[i]; k++)
+                            items.push_back(
+                                make_int4(i, k * p->Lp / cnt[i], (k + 1) * p->Lp / cnt[i], 0));
+                }
+                F.n_items = (int)items.size() - F.item_off;
+                ioff.push_back(F.n_items);
+                most = std::max(most, F.n_items);
+                if (p->dev.strip) {
+                    F.gather_off = (int)items.size();
+                    std::vector<double> wa(F.n);
+                    for (int i = 0; i < F.n; i++) wa[i] = sum_of(wg[l[a0 + i]]);
+                    cnt = chunk_counts(p, wa, 1);
+                    for (int i = 0; i < F.n; i++) {
+                        if (i == F.n / 2) F.gather_half = (int)items.size() - F.gather_off;
+                        split_planes(wg[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p),
+                                     kStripEmpty);
+                    }
+                    F.n_gather = (int)items.size() - F.gather_off;
+                }
+                groups.push_back(F);
             }
-            L.fgroups.push_back(F);
+            return most;
+        };
+        L.max_fitems = forward_groups(p->dev.strip ? p->G : L.n, L.fgroups);
+        const int gs = p->dev.strip ? std::min(p->G, static_slots(p->dev)) : L.n;
+        if (p->dev.strip && gs < std::min(p->G, L.n))
+            L.max_sitems = forward_groups(gs, L.sgroups);
+        else {
+            L.sgroups = L.fgroups;
+            L.max_sitems = L.max_fitems;
         }
         max_items = std::max(max_items, (size_t)L.max_fitems);
         // B1 items per angle group
@@ -978,24 +992,24 @@ gb_status gb_spect_set_tuning(gb_spect_plan *p, const gb_spect_tuning *tuning) {
 }
 
 // A forward group's angles of one half (0: slots before n / 2, 1: the others) or all of them
-// (-1); partials: of the whole group.
+// (-1); rows: of the strip kernels, of the whole group like the partials.
 static cudaError_t launch_fwd_group(gb_spect_plan *p, const gb_spect_plan::FwdGroup &F, int half,
-                                    const float *obj, const int *alist, float *partials,
-                                    cudaStream_t st) {
+                                    const float *obj, const int *alist, float *rows,
+                                    float *partials, cudaStream_t st) {
     const int i0 = half == 1 ? F.half : 0, i1 = half == 0 ? F.half : F.n_items;
     const int4 *items = p->d_items + F.item_off + i0;
     partials += (size_t)i0 * p->N * p->nz;
     if (p->dev.strip) {
         const int g0 = half == 1 ? F.gather_half : 0, g1 = half == 0 ? F.gather_half : F.n_gather;
         return launch_fwd_strip(p->dev, obj, alist, p->d_items + F.gather_off + g0, g1 - g0, items,
-                                i1 - i0, p->d_Wf, partials, st);
+                                i1 - i0, rows, partials, st);
     }
     return launch_fwd(p->dev, obj, alist, items, i1 - i0, p->Zt_fwd, p->fwd_tpb, partials, st);
 }
 
 static gb_status run_forward(gb_spect_plan *p, const float *obj, int subset, float *out,
                              int ratio, const float *gproj, const float *sadd, float *pred,
-                             float *partials, cudaStream_t st) {
+                             cudaStream_t st, const StaticScratch *fixed = nullptr) {
     const int li = list_index(p, subset);
     if (li < 0) {
         set_error("subset %d out of range (n_subsets=%d)", subset, p->n_subsets);
@@ -1003,9 +1017,11 @@ static gb_status run_forward(gb_spect_plan *p, const float *obj, int subset, flo
     }
     const gb_spect_plan::List &L = p->lists[li];
     const size_t NZ = (size_t)p->N * p->nz;
-    for (const gb_spect_plan::FwdGroup &F : L.fgroups) {
+    float *rows = fixed ? fixed->rows : p->d_Wf;
+    float *partials = fixed ? fixed->partials : p->d_partials;
+    for (const gb_spect_plan::FwdGroup &F : fixed ? L.sgroups : L.fgroups) {
         const int *alist = p->d_alist + L.alist_off + F.a0;
-        GB_CUDA(launch_fwd_group(p, F, -1, obj, alist, partials, st));
+        GB_CUDA(launch_fwd_group(p, F, -1, obj, alist, rows, partials, st));
         GB_CUDA(launch_reduce(F.n, p->d_ioff + F.ioff_off, (int)NZ, partials, out + F.a0 * NZ,
                               ratio, gproj, sadd, alist, pred ? pred + F.a0 * NZ : nullptr, st));
     }
@@ -1018,8 +1034,7 @@ gb_status gb_spect_forward(gb_spect_plan *p, const float *obj, float *proj, int3
     GB_INJECT_ARG();
     GB_CHECK_ARG(p && obj && proj, "null argument");
     GB_INJECT_LAUNCH();
-    return run_forward(p, obj, subset, proj, 0, nullptr, nullptr, nullptr, p->d_partials,
-                       as_stream(stream));
+    return run_forward(p, obj, subset, proj, 0, nullptr, nullptr, nullptr, as_stream(stream));
 }
 
 // Back-project `proj` (rows = the angles of list li) in groups of G angles.
@@ -1135,7 +1150,7 @@ gb_status gb_spect_autotune(gb_spect_plan *p, int32_t subset, int32_t reps,
         return ms / reps;
     };
     auto fwd_call = [&]() {
-        return run_forward(p, obj, subset, proj, 0, nullptr, nullptr, nullptr, p->d_partials, st);
+        return run_forward(p, obj, subset, proj, 0, nullptr, nullptr, nullptr, st);
     };
     auto bwd_call = [&]() { return run_backward(p, proj, li, 0, back, B2_WRITE, UpdateArgs{}, st); };
     // forward candidates
@@ -1216,8 +1231,8 @@ static gb_status osem_split_step(gb_spect_plan *p, const gb_spect_plan::List &L,
     cudaStream_t s2 = p->st2;
     GB_CUDA(cudaEventRecord(p->ev_fork, st));
     GB_CUDA(cudaStreamWaitEvent(s2, p->ev_fork, 0));
-    GB_CUDA(launch_fwd_group(p, F, 0, obj, alist, p->d_partials, st));
-    GB_CUDA(launch_fwd_group(p, F, 1, obj, alist, p->d_partials, s2));
+    GB_CUDA(launch_fwd_group(p, F, 0, obj, alist, p->d_Wf, p->d_partials, st));
+    GB_CUDA(launch_fwd_group(p, F, 1, obj, alist, p->d_Wf, p->d_partials, s2));
     GB_CUDA(launch_reduce(h, ioff, (int)NZ, p->d_partials, p->d_ratio, 1, g, s, alist, pred, st));
     GB_CUDA(launch_reduce(L.n - h, ioff + h, (int)NZ, p->d_partials, p->d_ratio + h * NZ, 1, g, s,
                           alist + h, pred ? pred + h * NZ : nullptr, s2));
@@ -1244,7 +1259,7 @@ gb_status gb_spect_osem_step(gb_spect_plan *p, float *obj, const float *g, const
     const int li = list_index(p, subset);
     if (li >= 0 && p->osem_split && p->dev.psf && p->lists[li].n >= 4 && p->lists[li].n <= p->G)
         return osem_split_step(p, p->lists[li], obj, g, s, nbp, pred, st);
-    gb_status r = run_forward(p, obj, subset, p->d_ratio, 1, g, s, pred, p->d_partials, st);
+    gb_status r = run_forward(p, obj, subset, p->d_ratio, 1, g, s, pred, st);
     if (r != GB_OK) return r;
     UpdateArgs u{};
     u.f = obj;
@@ -1273,7 +1288,7 @@ gb_status gb_spect_bsrem_step(gb_spect_plan *p, const float *in, float *out, con
     GB_CHECK_ARG(in != out, "BSREM needs distinct input and output objects");
     GB_INJECT_LAUNCH();
     cudaStream_t st = as_stream(stream);
-    gb_status r = run_forward(p, in, subset, p->d_ratio, 1, g, s, nullptr, p->d_partials, st);
+    gb_status r = run_forward(p, in, subset, p->d_ratio, 1, g, s, nullptr, st);
     if (r != GB_OK) return r;
     UpdateArgs u{};
     u.f_in = in;
@@ -1355,14 +1370,14 @@ bool plan_forward_need(const gb_spect_plan *p, int subset, int *n_sel, int *n_it
     const int li = p ? list_index(p, subset) : -1;
     if (li < 0) return false;
     *n_sel = p->lists[li].n;
-    *n_items = p->lists[li].max_fitems;
-    *floats = (size_t)*n_items * p->N * p->nz;
+    *n_items = std::max(p->lists[li].max_fitems, p->lists[li].max_sitems);
+    *floats = (size_t)std::max(*n_items, *n_sel) * p->N * p->nz;
     return true;
 }
 
 gb_status plan_forward(gb_spect_plan *p, const float *obj, int subset, float *out,
-                       float *partials, cudaStream_t st) {
-    return run_forward(p, obj, subset, out, 0, nullptr, nullptr, nullptr, partials, st);
+                       const StaticScratch &fixed, cudaStream_t st) {
+    return run_forward(p, obj, subset, out, 0, nullptr, nullptr, nullptr, st, &fixed);
 }
 
 }  // namespace gb

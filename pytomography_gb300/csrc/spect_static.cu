@@ -1,23 +1,24 @@
-// Forward projection that allocates nothing: its cross-chunk partial sums live in a
-// fixed file-scope device array instead of the plan's scratch buffer.
+// Forward projection that allocates nothing: its cross-chunk partial sums, and the rows between
+// the two strip kernels, live in fixed file-scope device arrays instead of the plan's scratch.
 //
 // Who needs it: callers that must not allocate device memory while they run — code on a
 // stream whose memory pool forbids further cudaMalloc, host processes whose device memory
 // is owned by another framework's allocator, or long-running services that budget every
 // allocation up front.  They
 // create their plan once at set-up; afterwards this entry point touches only the plan's
-// read-only tables, the caller's input and output, and the static array below.
+// read-only tables, the caller's input and output, and the static arrays below.
 //
 // Limits and behaviour:
-//   * the array holds GB_FWD_STATIC_FLOATS floats (16 MiB); every GPU that loads the
-//     library keeps it until the process exits;
+//   * the arrays hold kStaticPartials (16 MiB) and kStaticRows floats (64 MiB: the rows of 4
+//     angles of 128 x 128 x 128, of 16 or more of smaller planes, at a time); every GPU that
+//     loads the library keeps them until the process exits;
 //   * the plan's work items times nx * nz partial sums must fit (at least one item per
 //     angle); larger requests are rejected with GB_ERR_SHAPE;
-//   * every call shares the array and the kernels overwrite every partial they later
+//   * every call shares the arrays and the kernels overwrite every partial they later
 //     read (nothing needs to start at zero), so calls that overlap on the GPU (other
 //     streams, other threads) race: order them on one stream;
-//   * the first call on a device looks the array's device address up with
-//     cudaGetSymbolAddress (with that device current) and caches it; make that first
+//   * the first call on a device looks the arrays' device addresses up with
+//     cudaGetSymbolAddress (with that device current) and caches them; make that first
 //     call before any stream capture.
 #include <algorithm>
 #include <mutex>
@@ -25,17 +26,18 @@
 #include "common.cuh"
 #include "spect_launch.h"
 
-#define GB_FWD_STATIC_FLOATS (4u * 1024u * 1024u)
-
 namespace gb {
 
-static __device__ __align__(256) float g_fwd_static_scratch[GB_FWD_STATIC_FLOATS];
+static __device__ __align__(256) float g_fwd_static_scratch[kStaticPartials];
+static __device__ __align__(256) float g_fwd_static_rows[kStaticRows];
+// (a strip plan's largest slot: 182 planes of at most 172 rows of 128 values)
+static_assert(kStaticRows >= (size_t)182 * 182 * 128, "the rows of one angle fit");
 
 static std::mutex g_static_mu;
-static float *g_static_ptr[64] = {nullptr};
+static StaticScratch g_static_ptr[64] = {};
 
-// Device address of the static array on the current device (looked up once per device).
-static gb_status static_scratch(float **out) {
+// Device addresses of the static arrays on the current device (looked up once per device).
+static gb_status static_scratch(StaticScratch *out) {
     int dev = 0;
     GB_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) {
@@ -43,10 +45,11 @@ static gb_status static_scratch(float **out) {
         return GB_ERR_ARG;
     }
     std::lock_guard<std::mutex> lock(g_static_mu);
-    if (!g_static_ptr[dev]) {
-        void *p = nullptr;
+    if (!g_static_ptr[dev].partials) {
+        void *p = nullptr, *r = nullptr;
+        GB_CUDA(cudaGetSymbolAddress(&r, g_fwd_static_rows));
         GB_CUDA(cudaGetSymbolAddress(&p, g_fwd_static_scratch));
-        g_static_ptr[dev] = static_cast<float *>(p);
+        g_static_ptr[dev] = {static_cast<float *>(p), static_cast<float *>(r)};
     }
     *out = g_static_ptr[dev];
     return GB_OK;
@@ -66,13 +69,13 @@ extern "C" gb_status gb_spect_forward_static(gb_spect_plan *plan, const float *o
         set_error("subset %d out of range", subset);
         return GB_ERR_STATE;
     }
-    if (need > GB_FWD_STATIC_FLOATS) {
+    if (need > kStaticPartials) {
         set_error("forward of %d angles (%d work items) needs %zu floats of scratch; the static "
                   "array holds %u",
-                  n_sel, n_items, need, (unsigned)GB_FWD_STATIC_FLOATS);
+                  n_sel, n_items, need, (unsigned)kStaticPartials);
         return GB_ERR_SHAPE;
     }
-    float *scratch = nullptr;
+    StaticScratch scratch{};
     gb_status s = static_scratch(&scratch);
     if (s != GB_OK) return s;
     return plan_forward(plan, object, subset, proj, scratch, as_stream(stream));
