@@ -458,7 +458,7 @@ static bool fwd_patches_pay(const PetDev &g, long long n, bool tof) {
 struct PatchLease {
     PetPatches q{};
     PatchLease(gb_pet_plan *p, bool want, cudaStream_t st) : plan(p), st(st) {
-        if (!want || !p->call_patch.qx) return;
+        if (!want) return;
         cudaStreamCaptureStatus cs;
         if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
             cudaGetLastError();
@@ -466,6 +466,10 @@ struct PatchLease {
         }
         if (cs != cudaStreamCaptureStatusNone) return;
         p->call_lock.lock();
+        if (!p->call_patch.qx) {
+            p->call_lock.unlock();
+            return;
+        }
         if (p->call_used && cudaStreamWaitEvent(st, p->call_done) != cudaSuccess) {
             cudaGetLastError();
             p->call_lock.unlock();
@@ -512,6 +516,37 @@ static cudaError_t fold_patches(const gb_pet_plan *p, const PetPatches &q, float
     else
         k_patch_fold<false><<<grid, block, 0, st>>>(g, q, img, nullptr, nullptr);
     return cudaGetLastError();
+}
+
+// Patch layouts where the longest list, or a sensitivity image of as many LORs, pays for them;
+// without the memory for them the plan does without.
+static cudaError_t alloc_patches(gb_pet_plan *p) {
+    const PetDev &g = p->dev;
+    const size_t pb = (patch_elems_x(g) + patch_elems_y(g)) * sizeof(float4);
+    if (2 * pb > kPatchMaxBytes || !patch_pays(g, (double)p->n_events, g.tof, kPatchBwd))
+        return cudaSuccess;
+    for (PetPatches *q : {&p->osem_patch, &p->call_patch})
+        if (dev_alloc(&q->qx, patch_elems_x(g) * sizeof(float4)) != cudaSuccess ||
+            dev_alloc(&q->qy, patch_elems_y(g) * sizeof(float4)) != cudaSuccess) {
+            dev_free(q->qx);
+            *q = PetPatches{};
+            cudaGetLastError();
+        }
+    return cudaEventCreateWithFlags(&p->call_done, cudaEventDisableTiming);
+}
+
+// Gives the patch layouts back, so that something the plan needs has their memory; whether there
+// were any.  (The device is idle: dev_free waits for it.)
+static bool drop_patches(gb_pet_plan *p) {
+    bool any = false;
+    std::lock_guard<std::mutex> lock(p->call_lock);
+    for (PetPatches *q : {&p->osem_patch, &p->call_patch}) {
+        any = any || q->qx;
+        dev_free(q->qx);
+        dev_free(q->qy);
+        *q = PetPatches{};
+    }
+    return any;
 }
 
 // Forward projection of n tiles (k_pet_fwd's outputs), by way of the patch layout q if not null.
@@ -632,27 +667,16 @@ gb_status gb_pet_plan_create(const gb_pet_desc *d, gb_pet_plan **out) {
                 }
             }
     }
-    // patch layouts where the longest list, or a sensitivity image of as many LORs, pays for
-    // them; without the memory for them the plan does without
-    const size_t pb = (patch_elems_x(g) + patch_elems_y(g)) * sizeof(float4);
-    if (2 * pb <= kPatchMaxBytes && patch_pays(g, (double)d->n_events, d->tof, kPatchBwd)) {
-        for (PetPatches *q : {&p->osem_patch, &p->call_patch})
-            if (dev_alloc(&q->qx, patch_elems_x(g) * sizeof(float4)) != cudaSuccess ||
-                dev_alloc(&q->qy, patch_elems_y(g) * sizeof(float4)) != cudaSuccess) {
-                dev_free(q->qx);
-                *q = PetPatches{};
-                cudaGetLastError();
-            }
-        if ((e = cudaEventCreateWithFlags(&p->call_done, cudaEventDisableTiming)) != cudaSuccess) {
-            set_error("event creation failed: %s", cudaGetErrorString(e));
-            pet_free(p);
-            return GB_ERR_CUDA;
-        }
-    }
     gb_status st = build_tiles(p, 1);
     if (st != GB_OK) {
         pet_free(p);
         return st;
+    }
+    // last: what the plan cannot do without has its memory
+    if ((e = alloc_patches(p)) != cudaSuccess) {
+        set_error("event creation failed: %s", cudaGetErrorString(e));
+        pet_free(p);
+        return GB_ERR_CUDA;
     }
     *out = p;
     return GB_OK;
@@ -671,6 +695,11 @@ gb_status gb_pet_set_subsets(gb_pet_plan *p, int32_t n_subsets) {
     clear_error();
     GB_CHECK_ARG(p && n_subsets >= 1, "invalid subsets");
     gb_status st = build_tiles(p, n_subsets);
+    if (st == GB_ERR_OOM && drop_patches(p)) {
+        cudaGetLastError();
+        clear_error();
+        st = build_tiles(p, n_subsets);
+    }
     if (st != GB_OK) return st;
     p->n_subsets = n_subsets;
     return GB_OK;
@@ -741,7 +770,12 @@ gb_status gb_pet_set_deterministic(gb_pet_plan *p, int32_t on) {
     p->d_maxbits = nullptr;
     p->d_scale = nullptr;
     if (!on) return GB_OK;
-    GB_CUDA(dev_alloc(&p->d_acc64, (size_t)p->img_size * sizeof(unsigned long long)));
+    const size_t acc_bytes = (size_t)p->img_size * sizeof(unsigned long long);
+    if (dev_alloc(&p->d_acc64, acc_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        drop_patches(p);
+        GB_CUDA(dev_alloc(&p->d_acc64, acc_bytes));
+    }
     GB_CUDA(dev_alloc(&p->d_maxbits, sizeof(unsigned)));
     GB_CUDA(dev_alloc(&p->d_scale, sizeof(float)));
     return GB_OK;

@@ -84,6 +84,9 @@ def test_listmode_plan_without_tiles_refuses_and_recovers(nth, cuda):
                            PETLMProjMeta(ev, info=info, detector_ids_sensitivity=ev))
     img = torch.rand((20, 20, 5), device=cuda)
     whole = sm.forward(img)
+    # a first failure takes the memory of the plan's patch layouts, the next one has none to take
+    assert sm._lib.gb_inject_fault(b"alloc", 1) == 0
+    sm.set_n_subsets(3)
     assert sm._lib.gb_inject_fault(b"alloc", nth) == 0
     with pytest.raises(RuntimeError):
         sm.set_n_subsets(7)
