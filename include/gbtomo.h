@@ -174,7 +174,7 @@ gb_status gb_spect_forward_static(gb_spect_plan *plan, const float *object, floa
  * adjoint = 0: the reference back-projector, which rotates back with bilinear
  *              interpolation by +(270 - beta)
  *              (SPECTSystemMatrix.backward, spect_system_matrix.py:159-201);
- * adjoint = 1: the exact transpose of gb_spect_forward (same taps, scattered). */
+ * adjoint = 1: the exact transpose of gb_spect_forward (same taps and weights). */
 gb_status gb_spect_backward(gb_spect_plan *plan, const float *proj, float *object,
                             int32_t subset, int32_t adjoint, gb_stream_t stream);
 

@@ -288,8 +288,9 @@ __device__ __forceinline__ bool plane_rows(const SpectDev &g, const float *th, i
 // thread calls it before it touches anything an earlier call or kernel writes (objects,
 // projections, scratch), so that completion carries over the whole chain.  Plan tables are
 // written at set-up only and may be read before.  An OSEM iteration of 8 subsets at 64^3 without
-// PSF (32 kernels of 4 to 9 us) goes from 265 to 215 us, one of 5 subsets at 101^3 x 83 from 706
-// to 668 us, at 128^3 it makes no difference.  The batch kernels keep plain launches: their
+// PSF went from 265 to 215 us (32 kernels of 4 to 9 us then; 24 and 188 us since the back
+// projection is one kernel), one of 5 subsets at 101 x 101 x 83 from 706 to 668 us, at 128^3 it
+// makes no difference.  The batch kernels keep plain launches: their
 // waves of uneven blocks ran 5% longer when blocks of the next kernel took SMs early.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() {

@@ -1845,7 +1845,7 @@ gb_status gb_spect_batch_backward(gb_spect_batch *b, const float *const *proj,
     for (int e = 0; e < b->n; e++) {
         GB_CHECK_ARG(proj[e] && objects[e], "null buffer of entry %d", e);
         GB_CHECK_ARG(!adjoint || ((uintptr_t)objects[e] & 15) == 0,
-                     "object %d must be 16-byte aligned (vector atomics)", e);
+                     "object %d must be 16-byte aligned", e);
     }
     GB_INJECT_LAUNCH();
     int li;

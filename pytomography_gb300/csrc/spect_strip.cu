@@ -8,12 +8,14 @@
 //   rotated-frame back projection   128 us (26%) -> 60 us (58%)
 //   forward                         160 us (30%) -> 60 us (38%) + 37 us (55%), k_fwd_strip
 //                                   and k_fwd_ysum; the rows between the two kernels cost
-//                                   105 MB of writes and 105 MB of reads
-// and on 9 angles of 101^3 x 83 (nz odd: scalar object loads, padded rows) one OSEM
-// iteration of 5 subsets went from 1386 to 667 us (its dependent launches included).
-// Larger planes and the PSF-before-attenuation order keep the plane-at-a-time kernels: the
-// staged projection and the warps' buffers do not fit shared memory, and an attenuation
-// inside the blur leaves the back projection no common input for the planes of an angle.
+//                                   66 MB of DRAM writes and 113 MB of reads
+// and on 9 angles of 101 x 101 x 83 (nz odd: scalar object loads, padded rows) one OSEM
+// iteration of 5 subsets went from 1386 to 662 us (its dependent launches included).
+// More than 128 z values do not fit the lanes of a row (32 of 4 values); more than 128 rows
+// would fit shared memory up to about 190, but k_fwd_ysum has four summing warps of 32 rows and
+// its launch bound for them.  Those planes and the PSF-before-attenuation order keep the
+// plane-at-a-time kernels (an attenuation inside the blur leaves the back projection no common
+// input for the planes of an angle).
 #include <algorithm>
 
 #include "spect_launch.h"

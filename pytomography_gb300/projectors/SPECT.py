@@ -319,7 +319,7 @@ class SPECTSystemMatrix(SystemMatrix):
         return self._backward(proj, subset_idx, 0)
 
     def backward_adjoint(self, proj: torch.Tensor, subset_idx: int | None = None) -> torch.Tensor:
-        """Exact transpose of :meth:`forward` (same bilinear taps, scattered)."""
+        """Exact transpose of :meth:`forward` (same bilinear taps and weights)."""
         return self._backward(proj, subset_idx, 1)
 
     def compute_normalization_factor(self, subset_idx: int | None = None) -> torch.Tensor:
