@@ -77,13 +77,13 @@ __global__ void __launch_bounds__(256)
             const Bilin b = bilin(ix, iy);
             if constexpr (VEC) {
                 float4 s4;
-                sample4(mu, g.N, g.N, g.nz, g.pad, g.pad, b, z, s4);
+                sample4<READ_ONLY>(mu, g.N, g.N, g.nz, g.pad, g.pad, b, z, s4);
                 v[u][0] = __fmul_rn(s4.x, dx);
                 v[u][1] = __fmul_rn(s4.y, dx);
                 v[u][2] = __fmul_rn(s4.z, dx);
                 v[u][3] = __fmul_rn(s4.w, dx);
             } else {
-                v[u][0] = __fmul_rn(sample(mu, g.N, g.N, g.nz, g.pad, g.pad, b, z), dx);
+                v[u][0] = __fmul_rn(sample<READ_ONLY>(mu, g.N, g.N, g.nz, g.pad, g.pad, b, z), dx);
             }
         }
 #pragma unroll
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(256)
             const Bilin b = bilin(ix, iy);
             if (vec && nv == 4) {
                 float4 s4;
-                sample4(mu, g.N, g.N, g.nz, g.pad, g.pad, b, z, s4);
+                sample4<READ_ONLY>(mu, g.N, g.N, g.nz, g.pad, g.pad, b, z, s4);
                 v[u][0] = __fmul_rn(s4.x, dx);
                 v[u][1] = __fmul_rn(s4.y, dx);
                 v[u][2] = __fmul_rn(s4.z, dx);
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(256)
             } else {
 #pragma unroll
                 for (int w = 0; w < 4; w++)
-                    v[u][w] = w < nv ? __fmul_rn(sample(mu, g.N, g.N, g.nz, g.pad, g.pad, b, z + w),
+                    v[u][w] = w < nv ? __fmul_rn(sample<READ_ONLY>(mu, g.N, g.N, g.nz, g.pad, g.pad, b, z + w),
                                                  dx)
                                      : 0.f;
             }
@@ -627,6 +627,7 @@ cudaError_t launch_b1(const SpectDev &g, const float *proj, const int *alist, in
 // sum_s w_rs phi1(f_r, f_s) over the 26 neighbours with replicate boundary, in the
 // loop order of NearestNeighbourPrior._pair_contribution (nearest_neighbour.py:56-72);
 // phi1 of RelativeDifferencePrior (nearest_neighbour.py:176-177).
+template <LoadKind L>
 __device__ __forceinline__ float rdp_sum(const float *f, int nx, int ny, int nz,
                                          int x, int y, int z, float fr, const UpdateArgs &u) {
     float acc = 0.f;
@@ -642,7 +643,7 @@ __device__ __forceinline__ float rdp_sum(const float *f, int nx, int ny, int nz,
             for (int k = -1; k <= 1; k++) {
                 if (i == 0 && j == 0 && k == 0) continue;
                 int zk = min(max(z + k, 0), nz - 1);
-                float fs = ld_data(f + ((size_t)xi * ny + yj) * nz + zk);
+                float fs = ld_read<L>(f + ((size_t)xi * ny + yj) * nz + zk);
                 float d = __fsub_rn(fr, fs);
                 float ad = fabsf(d);
                 float num = __fmul_rn(
@@ -737,7 +738,7 @@ __global__ void k_rdp(const float *__restrict__ f, float *__restrict__ grad, int
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)nx * ny * nz) return;
     int z = i % nz, y = (i / nz) % ny, x = i / ((size_t)nz * ny);
-    float s = rdp_sum(f, nx, ny, nz, x, y, z, f[i], u);
+    float s = rdp_sum<READ_ONLY>(f, nx, ny, nz, x, y, z, f[i], u);
     float v = __fmul_rn(scale, s);
     if (u.fov) v = __fmul_rn(v, u.fov[i]);
     grad[i] = v;
@@ -797,7 +798,7 @@ cudaError_t launch_rdp(const float *f, float *grad, int nx, int ny, int nz, cons
 
 // Update epilogue shared by the gather kernel and the standalone update kernel.
 // PRIOR = false compiles out the RDP term (callers that never see BSREM with a prior).
-template <bool PRIOR = true>
+template <bool PRIOR = true, LoadKind L = COHERENT>
 __device__ __forceinline__ void apply_update(int mode, const UpdateArgs &u, size_t i, int x,
                                              int y, int z, int nx, int ny, int nz, float bp,
                                              float *out) {
@@ -817,7 +818,7 @@ __device__ __forceinline__ void apply_update(int mode, const UpdateArgs &u, size
         float grad = __fsub_rn(bp, nb);
         if (PRIOR && u.prior) {
             float v = __fmul_rn(__fmul_rn(u.beta, u.w_m),
-                                rdp_sum(u.f_in, nx, ny, nz, x, y, z, f, u));
+                                rdp_sum<L>(u.f_in, nx, ny, nz, x, y, z, f, u));
             if (u.fov) v = __fmul_rn(v, u.fov[i]);
             grad = __fsub_rn(grad, v);
         }
@@ -872,6 +873,26 @@ __device__ __forceinline__ void apply_update4(int mode, const UpdateArgs &u, siz
         const float fn = __fadd_rn(f[v], __fmul_rn(pre, grad));
         u.f_out[i + v] = fn <= u.floor_v ? u.floor_v : fn;
     }
+}
+
+// One value of sample4_ranged, for k_b2_gather alone: a plain launch, whose W nobody writes while
+// it runs.
+__device__ __forceinline__ float sample_ranged(const float *__restrict__ src, int rows, int cols,
+                                               int nz, int col_off, const int2 *__restrict__ wr,
+                                               const Bilin &b, int z) {
+    int r = b.r0, c = b.c0 - col_off;
+    bool r0 = (unsigned)r < (unsigned)rows, r1 = (unsigned)(r + 1) < (unsigned)rows;
+    int2 g0 = r0 ? wr[r] : make_int2(0, 0);
+    int2 g1 = r1 ? wr[r + 1] : make_int2(0, 0);
+    bool a00 = r0 && c >= g0.x && c < g0.y, a01 = r0 && c + 1 >= g0.x && c + 1 < g0.y;
+    bool a10 = r1 && c >= g1.x && c < g1.y, a11 = r1 && c + 1 >= g1.x && c + 1 < g1.y;
+    if (!(a00 || a01 || a10 || a11)) return 0.f;
+    const float *p = src + ((long long)r * cols + c) * nz + z;
+    float vnw = a00 ? __ldg(p) : 0.f;
+    float vne = a01 ? __ldg(p + nz) : 0.f;
+    float vsw = a10 ? __ldg(p + (long long)cols * nz) : 0.f;
+    float vse = a11 ? __ldg(p + (long long)cols * nz + nz) : 0.f;
+    return bilin_combine(b, vnw, vne, vsw, vse);
 }
 
 // ------------------------------------------------------------- B2 gather
@@ -1077,6 +1098,7 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
     grid_wait();
+    proj = after_wait(proj);
     const int z = 4 * q;
     if (z >= nz || y >= N) return;
     const size_t slab = (size_t)g.Lp * g.nya * nz, NZ = (size_t)N * nz;
@@ -1133,6 +1155,7 @@ __global__ void __launch_bounds__(256, PRIOR == NO_PRIOR ? 5 : 4)
         __syncthreads();
     }
     if (g.strip) grid_wait();
+    W = after_wait(W);
     const int z = z_of_pos(g, q);  // q: quad position in the W rows
     if (4 * q >= g.nzs || z >= nz || y >= N) return;
     const float4 bp = use_tab ? b2_gather_sum4_tab<kB2Unroll>(
@@ -1200,8 +1223,8 @@ cudaError_t launch_b2_gather_batch(const B2Batch &p, int n_blocks, cudaStream_t 
 }
 
 __global__ void __launch_bounds__(256)
-    k_b2_gather(SpectDev g, const float *W, const int *__restrict__ alist,
-                int n_slots, float *out, int mode, UpdateArgs u) {
+    k_b2_gather(SpectDev g, const float *__restrict__ W, const int *__restrict__ alist,
+                int n_slots, float *__restrict__ out, int mode, UpdateArgs u) {
     const int z = blockIdx.x * 32 + threadIdx.x;
     const int y = blockIdx.y * 8 + threadIdx.y;
     const int x = blockIdx.z;
@@ -1220,7 +1243,7 @@ __global__ void __launch_bounds__(256)
                                          g.wrange + (size_t)s * g.Lp, b, z));
     }
     const size_t i = ((size_t)x * N + y) * nz + z;
-    apply_update(mode, u, i, x, y, z, N, N, nz, bp, out);
+    apply_update<true, READ_ONLY>(mode, u, i, x, y, z, N, N, nz, bp, out);
 }
 
 // Blocks of 256 threads shaped to the z quads of a row: when the quads of a row divide a warp
@@ -1313,6 +1336,7 @@ __device__ __forceinline__ int adj_list(const SpectDev &g, int ga, int slot, int
 }
 
 // Block of 256 (row, quad position) elements from q0 on; mode B2_WRITE or B2_ADD.
+template <LoadKind L>
 __device__ __forceinline__ void b2_adjoint_block(const SpectDev &g, const float *W,
                                                  const int *__restrict__ alist, int n_slots,
                                                  long long q0, float *out, int mode,
@@ -1349,7 +1373,7 @@ __device__ __forceinline__ void b2_adjoint_block(const SpectDev &g, const float 
                 if (u < n) {
                     const float2 tp = t.tap[e][u];
                     w[u] = tp.y;
-                    v[u] = ld_data4(Wk + __float_as_int(tp.x));
+                    v[u] = ld_read4<L>(Wk + __float_as_int(tp.x));
                 }
             }
 #pragma unroll
@@ -1361,7 +1385,7 @@ __device__ __forceinline__ void b2_adjoint_block(const SpectDev &g, const float 
             }
             for (int u = U; u < n; u++) {
                 const float2 tp = t.tap[e][u];
-                const float4 x = ld_data4(Wk + __float_as_int(tp.x));
+                const float4 x = ld_read4<L>(Wk + __float_as_int(tp.x));
                 s.x = fmaf(tp.y, x.x, s.x);
                 s.y = fmaf(tp.y, x.y, s.y);
                 s.z = fmaf(tp.y, x.z, s.z);
@@ -1391,14 +1415,15 @@ __global__ void __launch_bounds__(256)
     __shared__ AdjTable t;
     grid_release();
     grid_wait();
-    b2_adjoint_block(g, W, alist, n_slots, (long long)blockIdx.x * 256, out, mode, t);
+    b2_adjoint_block<COHERENT>(g, W, alist, n_slots, (long long)blockIdx.x * 256, out, mode, t);
 }
 
 __global__ void __launch_bounds__(256) k_b2_adjoint_batch(const __grid_constant__ B2Batch p) {
     __shared__ AdjTable t;
     const int e = batch_entry(p.block_off, blockIdx.x);
-    b2_adjoint_block(p.g[e], p.W[e], p.alist[e], p.n_slots[e],
-                     (long long)(blockIdx.x - p.block_off[e]) * 256, p.out[e], p.mode[e], t);
+    b2_adjoint_block<READ_ONLY>(p.g[e], p.W[e], p.alist[e], p.n_slots[e],
+                                (long long)(blockIdx.x - p.block_off[e]) * 256, p.out[e],
+                                p.mode[e], t);
 }
 
 // The same adjoint by scattering, a thread per W element, for plain rows (no strip kernels)

@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(256)
     constexpr int V = VEC ? 4 : 1, PU = VEC ? 4 : 8;
     grid_release();
     grid_wait();
+    f = after_wait(f);
     const int4 item = items[blockIdx.x];
     const int ga = alist[item.x];
     const int N = g.N, nz = g.nz, nzv = nz / V;
@@ -60,14 +61,14 @@ __global__ void __launch_bounds__(256)
             const size_t ao = ((size_t)xp * g.nya + (yp - g.ya_lo)) * nz + z;
             if constexpr (VEC) {
                 float4 s4;
-                sample4(f, N, N, nz, g.pad, g.pad, b, z, s4);
+                sample4<COHERENT>(f, N, N, nz, g.pad, g.pad, b, z, s4);
                 if (A) s4 = mul4(s4, __ldg(reinterpret_cast<const float4 *>(A + ao)));
                 v[u][0] = s4.x;
                 v[u][1] = s4.y;
                 v[u][2] = s4.z;
                 v[u][3] = s4.w;
             } else {
-                float s1 = sample(f, N, N, nz, g.pad, g.pad, b, z);
+                float s1 = sample<COHERENT>(f, N, N, nz, g.pad, g.pad, b, z);
                 if (A) s1 = __fmul_rn(s1, __ldg(A + ao));
                 v[u][0] = s1;
             }

@@ -297,7 +297,7 @@ __device__ __forceinline__ bool fwd_psf_item(const SpectDev &g, const float *__r
                     bool h[RB];
 #pragma unroll
                     for (int u = 0; u < RB; u++)
-                        h[u] = okr[u] && sample4(f, N, N, nz, g.pad, g.pad, b[u], z, v[u]);
+                        h[u] = okr[u] && sample4<READ_ONLY>(f, N, N, nz, g.pad, g.pad, b[u], z, v[u]);
 #pragma unroll
                     for (int u = 0; u < RB; u++) {
                         if (!okr[u]) continue;
@@ -324,7 +324,7 @@ __device__ __forceinline__ bool fwd_psf_item(const SpectDev &g, const float *__r
                     float ix, iy;
                     rot_coords(th, lr, g.lin[y], g.half, ix, iy);
                     Bilin bb = bilin(ix, iy);
-                    v = sample(f, N, N, nz, g.pad, g.pad, bb, z);
+                    v = sample<READ_ONLY>(f, N, N, nz, g.pad, g.pad, bb, z);
                     if (amul && v != 0.f) v = __fmul_rn(v, Ap[(size_t)(y - g.ya_lo) * nz + z]);
                 }
                 S[(y - (g.pad - H)) * SC + c] = v;

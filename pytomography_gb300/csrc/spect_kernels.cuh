@@ -145,18 +145,25 @@ __device__ __forceinline__ float ld_data(const float *p) { return *p; }
 __device__ __forceinline__ float4 ld_data4(const float *p) {
     return *reinterpret_cast<const float4 *>(p);
 }
-// The same where `ok`, else zeros: a predicated load (volatile, so that it stays below
-// grid_wait(); a plain conditional load becomes a branch around it).
+// Data pointer p of a dependent kernel, after its grid_wait(): loads from the result depend on
+// the wait, whatever the compiler moves.
+template <typename T>
+__device__ __forceinline__ T *after_wait(T *p) {
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
+// The same where `ok`, else zeros: a predicated load (a plain conditional load becomes a branch
+// around it).  Free to move, so a dependent kernel's p comes from after_wait().
 __device__ __forceinline__ float ld_data_if(bool ok, const float *p) {
     float v = 0.f;
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.f32 %0, [%1];\n\t}"
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.f32 %0, [%1];\n\t}"
                  : "+f"(v)
                  : "l"(p), "r"((unsigned)ok));
     return v;
 }
 __device__ __forceinline__ float4 ld_data4_if(bool ok, const float *p) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    asm volatile(
+    asm(
         "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
         "@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
         : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
@@ -164,8 +171,36 @@ __device__ __forceinline__ float4 ld_data4_if(bool ok, const float *p) {
     return v;
 }
 
+// How the samples below load: COHERENT as above; READ_ONLY in kernels with plain launches, which
+// start when their predecessors are over, and for arrays that no kernel writes (2-3% faster in
+// k_fwd_psf, which the compiler may then schedule freely).
+enum LoadKind { COHERENT, READ_ONLY };
+template <LoadKind L>
+__device__ __forceinline__ float ld_read(const float *p) {
+    return L == READ_ONLY ? __ldg(p) : ld_data(p);
+}
+template <LoadKind L>
+__device__ __forceinline__ float4 ld_read4(const float *p) {
+    return L == READ_ONLY ? __ldg(reinterpret_cast<const float4 *>(p)) : ld_data4(p);
+}
+template <LoadKind L>
+__device__ __forceinline__ float ld_sample(bool ok, const float *p) {
+    if constexpr (L == READ_ONLY)
+        return ok ? __ldg(p) : 0.f;
+    else
+        return ld_data_if(ok, p);
+}
+template <LoadKind L>
+__device__ __forceinline__ float4 ld_sample4(bool ok, const float *p) {
+    if constexpr (L == READ_ONLY)
+        return ok ? __ldg(reinterpret_cast<const float4 *>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    else
+        return ld_data4_if(ok, p);
+}
+
 // Bilinear sample of a [rows][cols][nz] array whose (row, col) origin is shifted by
 // (row_off, col_off): value at (r, c) = src[r - row_off][c - col_off] when inside.
+template <LoadKind L>
 __device__ __forceinline__ float sample(const float *src, int rows, int cols,
                                         int nz, int row_off, int col_off, const Bilin &b,
                                         int z) {
@@ -174,15 +209,16 @@ __device__ __forceinline__ float sample(const float *src, int rows, int cols,
     bool c0 = (unsigned)c < (unsigned)cols, c1 = (unsigned)(c + 1) < (unsigned)cols;
     if (!((r0 || r1) && (c0 || c1))) return 0.f;
     const float *p = src + ((long long)r * cols + c) * nz + z;
-    float vnw = ld_data_if(r0 && c0, p);
-    float vne = ld_data_if(r0 && c1, p + nz);
-    float vsw = ld_data_if(r1 && c0, p + (long long)cols * nz);
-    float vse = ld_data_if(r1 && c1, p + (long long)cols * nz + nz);
+    float vnw = ld_sample<L>(r0 && c0, p);
+    float vne = ld_sample<L>(r0 && c1, p + nz);
+    float vsw = ld_sample<L>(r1 && c0, p + (long long)cols * nz);
+    float vse = ld_sample<L>(r1 && c1, p + (long long)cols * nz + nz);
     return bilin_combine(b, vnw, vne, vsw, vse);
 }
 
 // Four consecutive z values (z % 4 == 0, nz % 4 == 0) of the bilinear sample; returns
 // false (and zeros) when no tap is inside the array.
+template <LoadKind L>
 __device__ __forceinline__ bool sample4(const float *src, int rows, int cols, int nz,
                                         int row_off, int col_off, const Bilin &b, int z,
                                         float4 &out) {
@@ -192,10 +228,10 @@ __device__ __forceinline__ bool sample4(const float *src, int rows, int cols, in
     bool c0 = (unsigned)c < (unsigned)cols, c1 = (unsigned)(c + 1) < (unsigned)cols;
     const float *p = src + ((long long)r * cols + c) * nz + z;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 vnw = ld_data4_if(r0 && c0, p);
-    float4 vne = ld_data4_if(r0 && c1, p + nz);
-    float4 vsw = ld_data4_if(r1 && c0, p + (long long)cols * nz);
-    float4 vse = ld_data4_if(r1 && c1, p + (long long)cols * nz + nz);
+    float4 vnw = ld_sample4<L>(r0 && c0, p);
+    float4 vne = ld_sample4<L>(r0 && c1, p + nz);
+    float4 vsw = ld_sample4<L>(r1 && c0, p + (long long)cols * nz);
+    float4 vse = ld_sample4<L>(r1 && c1, p + (long long)cols * nz + nz);
     out.x = bilin_combine(b, vnw.x, vne.x, vsw.x, vse.x);
     out.y = bilin_combine(b, vnw.y, vne.y, vsw.y, vse.y);
     out.z = bilin_combine(b, vnw.z, vne.z, vsw.z, vse.z);
@@ -227,24 +263,6 @@ __device__ __forceinline__ bool sample4_ranged(const float *src, int rows, int c
     out.z = bilin_combine(b, vnw.z, vne.z, vsw.z, vse.z);
     out.w = bilin_combine(b, vnw.w, vne.w, vsw.w, vse.w);
     return true;
-}
-
-__device__ __forceinline__ float sample_ranged(const float *src, int rows, int cols,
-                                               int nz, int col_off, const int2 *wr,
-                                               const Bilin &b, int z) {
-    int r = b.r0, c = b.c0 - col_off;
-    bool r0 = (unsigned)r < (unsigned)rows, r1 = (unsigned)(r + 1) < (unsigned)rows;
-    int2 g0 = r0 ? wr[r] : make_int2(0, 0);
-    int2 g1 = r1 ? wr[r + 1] : make_int2(0, 0);
-    bool a00 = r0 && c >= g0.x && c < g0.y, a01 = r0 && c + 1 >= g0.x && c + 1 < g0.y;
-    bool a10 = r1 && c >= g1.x && c < g1.y, a11 = r1 && c + 1 >= g1.x && c + 1 < g1.y;
-    if (!(a00 || a01 || a10 || a11)) return 0.f;
-    const float *p = src + ((long long)r * cols + c) * nz + z;
-    float vnw = ld_data_if(a00, p);
-    float vne = ld_data_if(a01, p + nz);
-    float vsw = ld_data_if(a10, p + (long long)cols * nz);
-    float vse = ld_data_if(a11, p + (long long)cols * nz + nz);
-    return bilin_combine(b, vnw, vne, vsw, vse);
 }
 
 // Rows y in [ylo, yhi) of plane xp whose sample (rotation th) can land within `margin`

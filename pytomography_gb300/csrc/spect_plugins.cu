@@ -56,13 +56,13 @@ __global__ void __launch_bounds__(256)
             const Bilin b = bilin(ix, iy);
             if constexpr (VEC) {
                 float4 s4;
-                sample4(mu, N, N, nz, pad, pad, b, z, s4);
+                sample4<READ_ONLY>(mu, N, N, nz, pad, pad, b, z, s4);
                 v[u][0] = __fmul_rn(s4.x, dx);
                 v[u][1] = __fmul_rn(s4.y, dx);
                 v[u][2] = __fmul_rn(s4.z, dx);
                 v[u][3] = __fmul_rn(s4.w, dx);
             } else {
-                v[u][0] = __fmul_rn(sample(mu, N, N, nz, pad, pad, b, z), dx);
+                v[u][0] = __fmul_rn(sample<READ_ONLY>(mu, N, N, nz, pad, pad, b, z), dx);
             }
         }
 #pragma unroll

@@ -64,7 +64,7 @@ __device__ __forceinline__ float4 ldg_here(const float *p) {
 }
 
 template <int QL, int HB, bool Z2>
-__device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *P,
+__device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *proj,
                                               const int ga, const int x0, const int x1,
                                               float *__restrict__ Ws, float *__restrict__ sm) {
     constexpr int G = 32 / QL, RS = 8 * G, ZG = QL / 4, SC = 4 * QL;
@@ -79,6 +79,7 @@ __device__ __forceinline__ void b1_strip_item(const SpectDev &g, const float *P,
         reinterpret_cast<float4 *>(buf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (warp == 0) strip_planes<RS>(g.planes_bwd + (size_t)ga * g.Lp, x0, x1, it);
     grid_wait();
+    const float *P = after_wait(proj);
     // P with its zero halo
     const bool vec = nz % 4 == 0 && ((uintptr_t)P & 15) == 0;
     for (int i = threadIdx.x; i < L.rows * QL; i += blockDim.x) {
@@ -161,11 +162,13 @@ __global__ void __launch_bounds__(512, 1)
 }
 
 // Calls f(QL, Z2) (as types) for a batch entry: the lanes of its rows, whether the PSF blurs z.
-template <typename F>
+template <bool ONLY2D, typename F>
 __device__ __forceinline__ void strip_dispatch(const SpectDev &g, F &&f) {
     const int ql = strip_ql(g.nz);
     auto both = [&](auto q) {
-        if (g.psf2d)
+        if constexpr (ONLY2D)
+            f(q, std::true_type{});
+        else if (g.psf2d)
             f(q, std::true_type{});
         else
             f(q, std::false_type{});
@@ -180,7 +183,8 @@ __device__ __forceinline__ void strip_dispatch(const SpectDev &g, F &&f) {
 
 // Persistent batch form: one CTA per SM dequeues the work items of every entry, largest
 // first.  The entries share the tap bucket (HB); their row widths and PSF dimensions may differ.
-template <int HB>
+// ONLY2D: every entry's PSF blurs z as well (beside the 1-D forms the kernel is 2% slower).
+template <int HB, bool ONLY2D>
 __global__ void __launch_bounds__(512, 1) k_b1_strip_batch(const __grid_constant__ B1Batch p) {
     extern __shared__ __align__(128) float sm[];
     __shared__ int s_item;
@@ -196,7 +200,7 @@ __global__ void __launch_bounds__(512, 1) k_b1_strip_batch(const __grid_constant
         const float *P = p.proj[e] + (size_t)slot * g.N * g.nz;
         const int ga = p.alist[e][slot];
         float *W = p.W[e] + (size_t)slot * g.Lp * g.nya * g.nzs;
-        strip_dispatch(g, [&](auto ql, auto z2) {
+        strip_dispatch<ONLY2D>(g, [&](auto ql, auto z2) {
             b1_strip_item<decltype(ql)::value, HB, decltype(z2)::value>(g, P, ga, item.y, item.z,
                                                                         W, sm);
         });
@@ -290,8 +294,8 @@ __device__ __forceinline__ void gather_rows(const float *f, const SpectDev &g,
     }
 }
 
-template <int QL, int HB>
-__device__ __forceinline__ void fwd_strip_item(const SpectDev &g, const float *f,
+template <int QL, int HB, bool ONLY2D>
+__device__ __forceinline__ void fwd_strip_item(const SpectDev &g, const float *obj,
                                                const int ga, const int x0, const int x1,
                                                float *__restrict__ Ws, float *__restrict__ sm) {
     constexpr int G = 32 / QL, RS = 8 * G, ZG = QL / 4, PS = strip_pair(QL, HB);
@@ -307,6 +311,7 @@ __device__ __forceinline__ void fwd_strip_item(const SpectDev &g, const float *f
     if (warp == 0) strip_planes<RS>(g.planes_fwd + (size_t)ga * g.Lp, x0, x1, it);
     cp_async_wait_all();
     grid_wait();
+    const float *f = after_wait(obj);
     __syncthreads();
     float th[6];
 #pragma unroll
@@ -364,50 +369,46 @@ __device__ __forceinline__ void fwd_strip_item(const SpectDev &g, const float *f
         const float *tap = taps + (xp - x0) * kStripTaps;
         const int y = y0 + 2 * pr;
         float *Wp = Ws + ((size_t)xp * ns * g.nya + (y - g.ya_lo)) * 32;
-        auto store = [&](const float2 (&o)[16]) {
-            __syncwarp();  // the buffer is free for the next strip
-            if (c >= g.zg) return;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int pos = k * g.zg + c;
-                float *d = Wp + (size_t)(pos >> 3) * g.nya * 32 + 4 * (pos & 7);
-                if (y <= yl)
-                    *reinterpret_cast<float4 *>(d) =
-                        make_float4(o[4 * k].x, o[4 * k + 1].x, o[4 * k + 2].x, o[4 * k + 3].x);
-                if (y + 1 <= yl)
-                    *reinterpret_cast<float4 *>(d + 32) =
-                        make_float4(o[4 * k].y, o[4 * k + 1].y, o[4 * k + 2].y, o[4 * k + 3].y);
-            }
-        };
-        if (!g.psf2d) {
-            float2 o[16];
-            strip_z_copy<HB>(buf + pr * PS + 18 * c, o);
-            store(o);
-            continue;
-        }
         ladder_dispatch(pi.w & 15, [&](auto kk) {
             constexpr int KK = decltype(kk)::value;
             if constexpr (KK / 2 <= HB) {
                 float2 o[16];
-                strip_z_pass<KK, HB>(buf + pr * PS + 18 * c, tap, o);
-                store(o);
+                if (ONLY2D || g.psf2d)
+                    strip_z_pass<KK, HB>(buf + pr * PS + 18 * c, tap, o);
+                else
+                    strip_z_copy<HB>(buf + pr * PS + 18 * c, o);
+                __syncwarp();  // the buffer is free for the next strip
+                if (c < g.zg) {
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int pos = k * g.zg + c;
+                        float *d = Wp + (size_t)(pos >> 3) * g.nya * 32 + 4 * (pos & 7);
+                        if (y <= yl)
+                            *reinterpret_cast<float4 *>(d) = make_float4(
+                                o[4 * k].x, o[4 * k + 1].x, o[4 * k + 2].x, o[4 * k + 3].x);
+                        if (y + 1 <= yl)
+                            *reinterpret_cast<float4 *>(d + 32) = make_float4(
+                                o[4 * k].y, o[4 * k + 1].y, o[4 * k + 2].y, o[4 * k + 3].y);
+                    }
+                }
             }
         });
     }
 }
 
-template <int QL, int HB>
+template <int QL, int HB, bool ONLY2D>
 __global__ void __launch_bounds__(512, 1)
     k_fwd_strip(SpectDev g, const float *f, const int *__restrict__ alist,
                 const int4 *__restrict__ items, float *__restrict__ W) {
     extern __shared__ __align__(128) float sm[];
     grid_release();
     const int4 item = items[blockIdx.x];
-    fwd_strip_item<QL, HB>(g, f, alist[item.x], item.y, item.z,
+    fwd_strip_item<QL, HB, ONLY2D>(g, f, alist[item.x], item.y, item.z,
                            W + (size_t)item.x * g.Lp * g.nya * 32 * strip_slabs(g), sm);
 }
 
-template <int HB>
+// ONLY2D: every entry's PSF blurs z as well.
+template <int HB, bool ONLY2D>
 __global__ void __launch_bounds__(512, 1) k_fwd_strip_batch(const __grid_constant__ FwdBatch p) {
     extern __shared__ __align__(128) float sm[];
     __shared__ int s_item;
@@ -423,9 +424,9 @@ __global__ void __launch_bounds__(512, 1) k_fwd_strip_batch(const __grid_constan
         const int ga = p.alist[item.w][item.x];
         float *W = p.W[item.w] + (size_t)item.x * g.Lp * g.nya * 32 * strip_slabs(g);
         switch (strip_ql(g.nz)) {
-            case 32: fwd_strip_item<32, HB>(g, f, ga, item.y, item.z, W, sm); break;
-            case 16: fwd_strip_item<16, HB>(g, f, ga, item.y, item.z, W, sm); break;
-            default: fwd_strip_item<8, HB>(g, f, ga, item.y, item.z, W, sm); break;
+            case 32: fwd_strip_item<32, HB, ONLY2D>(g, f, ga, item.y, item.z, W, sm); break;
+            case 16: fwd_strip_item<16, HB, ONLY2D>(g, f, ga, item.y, item.z, W, sm); break;
+            default: fwd_strip_item<8, HB, ONLY2D>(g, f, ga, item.y, item.z, W, sm); break;
         }
     }
 }
@@ -605,8 +606,8 @@ cudaError_t launch_fwd_strip(const SpectDev &g, const float *f, const int *alist
     cudaError_t e = cudaErrorInvalidValue;
 #define GB_CASE(Q, B)                                                                        \
     if (QL == Q && HB == B)                                                                  \
-        e = launch_dependent(k_fwd_strip<Q, B>, n_items, 32 * g.strip_fwd, smem, st, g, f,    \
-                             alist, items, W);
+        e = launch_dependent(g.psf2d ? k_fwd_strip<Q, B, true> : k_fwd_strip<Q, B, false>,   \
+                             n_items, 32 * g.strip_fwd, smem, st, g, f, alist, items, W);
     GB_FOR_EACH_STRIP(GB_CASE)
 #undef GB_CASE
     if (e != cudaSuccess) return e;
@@ -632,21 +633,22 @@ cudaError_t launch_b1_strip(const SpectDev &g, const float *proj, const int *ali
 cudaError_t launch_fwd_strip_batch(const FwdBatch &p, int n, int grid, cudaStream_t st) {
     size_t smem = 0, ysmem = 0;
     int slabs = 1, rows = 1, HB = 16, warps = 16;
+    bool only2d = true;
     for (int e = 0; e < n; e++)
         if (p.g[e].strip) warps = std::min(warps, p.g[e].strip_fwd);
     for (int e = 0; e < n; e++) {
         const SpectDev &g = p.g[e];
         if (!g.strip) continue;
         HB = strip_halo(g);
+        only2d = only2d && g.psf2d;
         smem = std::max(smem, fwd_strip_layout(strip_ql(g.nz), HB, warps).total);
         ysmem = std::max(ysmem, ysum_layout(g).total);
         slabs = std::max(slabs, strip_slabs(g));
         rows = std::max(rows, g.N);
     }
-    if (HB == 16)
-        k_fwd_strip_batch<16><<<grid, 32 * warps, smem * sizeof(float), st>>>(p);
-    else
-        k_fwd_strip_batch<24><<<grid, 32 * warps, smem * sizeof(float), st>>>(p);
+    auto *fn = HB == 16 ? (only2d ? k_fwd_strip_batch<16, true> : k_fwd_strip_batch<16, false>)
+                        : (only2d ? k_fwd_strip_batch<24, true> : k_fwd_strip_batch<24, false>);
+    fn<<<grid, 32 * warps, smem * sizeof(float), st>>>(p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_fwd_ysum_batch<<<dim3(p.n_yitems, slabs), 32 * ((rows + 31) / 32 + 1),
@@ -656,6 +658,7 @@ cudaError_t launch_fwd_strip_batch(const FwdBatch &p, int n, int grid, cudaStrea
 
 cudaError_t launch_b1_strip_batch(const B1Batch &p, int n, int grid, cudaStream_t st) {
     int warps = 16, HB = 16;
+    bool only2d = true;
     size_t smem = 0;
     for (int e = 0; e < n; e++)
         if (p.g[e].strip) warps = std::min(warps, p.g[e].strip);
@@ -663,12 +666,12 @@ cudaError_t launch_b1_strip_batch(const B1Batch &p, int n, int grid, cudaStream_
         if (p.g[e].strip) {
             smem = std::max(smem, b1_strip_layout(p.g[e], strip_ql(p.g[e].nz), warps).total);
             HB = strip_halo(p.g[e]);
+            only2d = only2d && p.g[e].psf2d;
         }
     smem *= sizeof(float);
-    if (HB == 16)
-        k_b1_strip_batch<16><<<grid, 32 * warps, smem, st>>>(p);
-    else
-        k_b1_strip_batch<24><<<grid, 32 * warps, smem, st>>>(p);
+    auto *fn = HB == 16 ? (only2d ? k_b1_strip_batch<16, true> : k_b1_strip_batch<16, false>)
+                        : (only2d ? k_b1_strip_batch<24, true> : k_b1_strip_batch<24, false>);
+    fn<<<grid, 32 * warps, smem, st>>>(p);
     return cudaGetLastError();
 }
 
@@ -678,14 +681,17 @@ cudaError_t setup_strip(size_t cap) {
     };
     cudaError_t e;
     for (const void *fn :
-         {(const void *)k_b1_strip_batch<16>, (const void *)k_b1_strip_batch<24>,
-          (const void *)k_fwd_strip_batch<16>, (const void *)k_fwd_strip_batch<24>,
+         {(const void *)k_b1_strip_batch<16, true>, (const void *)k_b1_strip_batch<24, true>,
+          (const void *)k_b1_strip_batch<16, false>, (const void *)k_b1_strip_batch<24, false>,
+          (const void *)k_fwd_strip_batch<16, true>, (const void *)k_fwd_strip_batch<24, true>,
+          (const void *)k_fwd_strip_batch<16, false>, (const void *)k_fwd_strip_batch<24, false>,
           (const void *)k_fwd_ysum, (const void *)k_fwd_ysum_batch})
         if ((e = raise(fn)) != cudaSuccess) return e;
 #define GB_CASE(Q, B)                                                        \
     if ((e = raise((const void *)k_b1_strip<Q, B, true>)) != cudaSuccess ||  \
         (e = raise((const void *)k_b1_strip<Q, B, false>)) != cudaSuccess || \
-        (e = raise((const void *)k_fwd_strip<Q, B>)) != cudaSuccess)         \
+        (e = raise((const void *)k_fwd_strip<Q, B, true>)) != cudaSuccess || \
+        (e = raise((const void *)k_fwd_strip<Q, B, false>)) != cudaSuccess)  \
         return e;
     GB_FOR_EACH_STRIP(GB_CASE)
 #undef GB_CASE

@@ -53,3 +53,30 @@ def test_shared_sampling_code_loads_coherently():
     # the fused form reads the attenuation table (p = As + ...) that way, nothing else
     ldgs = re.findall(r"__ldg\([^;]*;", part)
     assert len(ldgs) == 4 and all("mul4" in ln for ln in part.splitlines() if "__ldg(" in ln)
+
+
+def test_only_plain_launches_sample_read_only():
+    """READ_ONLY samples: in no kernel that is launched while its predecessor runs."""
+    text = "\n".join(_sources().values())
+    for n in ("k_fwd_nopsf", "k_b2_gather4", "k_b2_nopsf4", "k_b2_adjoint", "k_fwd_strip",
+              "k_b1_strip", "k_fwd_ysum", "k_reduce", "k_b1_nopsf"):
+        m = re.search(r"__global__[^;{]*?\b%s\(([^)]*)\)\s*{" % n, text)
+        assert "READ_ONLY" not in text[m.end():text.index("\n}\n", m.end())], n
+    bwd = _sources()["spect_bwd.cu"]
+    part = bwd[bwd.index("b2_gather_sum4("):bwd.index("k_b2_gather(SpectDev")]
+    assert "READ_ONLY" not in part
+    for n in ("k_fwd_psf", "k_b2_gather"):  # plain launches take them
+        assert not re.search(r"launch_dependent\(\s*%s\b" % n, text)
+
+
+def test_movable_loads_depend_on_the_wait():
+    """The predicated loads may move, so every dependent kernel that uses them takes its data
+    pointer from after_wait(), below its wait."""
+    src = _sources()
+    for f, names in (("spect_fwd.cu", ["k_fwd_nopsf"]),
+                     ("spect_strip.cu", ["b1_strip_item", "fwd_strip_item"]),
+                     ("spect_bwd.cu", ["k_b2_nopsf4", "k_b2_gather4"])):
+        for n in names:
+            m = re.search(r"\b%s\([^;{]*\)\s*{" % n, src[f])
+            body = src[f][m.end():src[f].index("\n}\n", m.end())]
+            assert body.rindex("grid_wait()") < body.index("after_wait("), n

@@ -101,3 +101,21 @@ def test_batched_osem_of_mixed_plans(cuda):
     for a, r in zip(batch(2), refs):
         assert torch.isfinite(a).all()
         assert rel_l2(a.cpu().numpy(), r.cpu().numpy()) < TOL
+
+
+def test_batch_of_1d_and_2d_plans(cuda):
+    """Strip plans of a 1-D and a 2-D PSF in one batch."""
+    from pytomography_gb300.batched import SpectBatch, common_psf_bucket
+    from test_spect_strip_gpu import _pair
+    made = [_pair(n, nz, 6, (0.03, 0.11), "ap", two_d, 0.0)
+            for n, nz, two_d in ((40, 36, False), (32, 64, True), (24, 100, False))]
+    Hs = [m[0] for m in made]
+    common_psf_bucket(Hs)
+    for H in Hs:
+        H.set_n_subsets(2)
+    b = SpectBatch(Hs)
+    fs = [torch.tensor(m[2], dtype=torch.float32, device=cuda) for m in made]
+    gs = [torch.tensor(m[3], dtype=torch.float32, device=cuda) for m in made]
+    for (H, o, f, g), p, x in zip(made, b.forward(fs, None), b.backward(gs, None)):
+        assert rel_l2(p.cpu().numpy(), o.forward(f)) < TOL
+        assert rel_l2(x.cpu().numpy(), o.backward(g)) < TOL
