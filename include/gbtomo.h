@@ -162,7 +162,7 @@ gb_status gb_spect_forward(gb_spect_plan *plan, const float *object, float *proj
  * while they run (code on a pool-restricted stream, processes whose device memory belongs
  * to another allocator, services that budget every allocation up front).  No counterpart in
  * the reference.  Its partial sums, and the rows that PSF plans keep between their two kernels,
- * use fixed device arrays (16 and 64 MiB) compiled into the library instead of the plan's
+ * use fixed device arrays (16 and 256 MiB) compiled into the library instead of the plan's
  * scratch; calls needing more than 4,194,304 floats of partials (the plan's work items for the
  * subset, at least one per angle, times nx * nz) return GB_ERR_SHAPE.
  * Calls share those arrays: overlapping calls on the GPU race.  The first call on a device looks

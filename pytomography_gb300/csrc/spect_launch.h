@@ -152,13 +152,14 @@ cudaError_t launch_b2_adjoint_batch(const B2Batch &p, int n_blocks, cudaStream_t
 // blocks of 256 threads of one entry in the batched gather and adjoint kernels
 int b2_gather_blocks(const SpectDev &g);
 
-// Scratch of gb_spect_forward_static: partial sums, and the strip kernels' rows of as many
-// angles at a time as fit (static_slots).
+constexpr int kGroup = 16;  // angles of a plan that share the W stack
+
+// Scratch of gb_spect_forward_static: partial sums, and the strip kernels' rows of a group of
+// angles.
 struct StaticScratch {
     float *partials, *rows;
 };
-constexpr size_t kStaticPartials = (size_t)4 << 20, kStaticRows = (size_t)16 << 20;  // floats
-inline int static_slots(const SpectDev &g) { return (int)(kStaticRows / stack_slot(g)); }
+constexpr size_t kStaticPartials = (size_t)4 << 20, kStaticRows = (size_t)64 << 20;  // floats
 
 // One forward projection of a plan in that scratch (for entry points defined outside
 // spect_plan.cu): the work items and partial floats a subset needs (false when the subset is out

@@ -192,8 +192,7 @@ struct gb_spect_plan {
     struct List {
         int alist_off = 0, n = 0;
         std::vector<FwdGroup> fgroups;
-        std::vector<FwdGroup> sgroups;  // the groups of gb_spect_forward_static
-        int max_fitems = 0, max_sitems = 0;  // largest group's items
+        int max_fitems = 0;  // largest group's items
         std::vector<int> gitem_off, n_gitems;  // B1 items of each angle group
         int b_half = 0;  // first group-0 B1 item of slot n / 2
     };
@@ -432,58 +431,45 @@ static gb_status upload_lists(gb_spect_plan *p, int n_subsets,
         L.alist_off = (int)all.size();
         L.n = (int)l.size();
         all.insert(all.end(), l.begin(), l.end());
-        // forward items, gf angles a group
-        auto forward_groups = [&](int gf, std::vector<gb_spect_plan::FwdGroup> &groups) {
-            int most = 0;
-            for (int a0 = 0; a0 < L.n; a0 += gf) {
-                gb_spect_plan::FwdGroup F;
-                F.a0 = a0;
-                F.n = std::min(gf, L.n - a0);
-                F.item_off = (int)items.size();
-                F.ioff_off = (int)ioff.size();
-                std::vector<int> cnt(F.n, psf ? 0 : nopsf_chunks(p, L.n));
-                if (psf) {
-                    std::vector<double> wa(F.n);
-                    for (int i = 0; i < F.n; i++) wa[i] = sum_of(wf[l[a0 + i]]);
-                    cnt = chunk_counts(p, wa, zs_f, p->fwd_items);
-                }
-                for (int i = 0; i < F.n; i++) {
-                    ioff.push_back((int)items.size() - F.item_off);
-                    if (i == F.n / 2) F.half = (int)items.size() - F.item_off;
-                    if (psf)
-                        split_planes(wf[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p),
-                                     kStripEmpty);
-                    else
-                        for (int k = 0; k < cnt[i]; k++)
-                            items.push_back(
-                                make_int4(i, k * p->Lp / cnt[i], (k + 1) * p->Lp / cnt[i], 0));
-                }
-                F.n_items = (int)items.size() - F.item_off;
-                ioff.push_back(F.n_items);
-                most = std::max(most, F.n_items);
-                if (p->dev.strip) {
-                    F.gather_off = (int)items.size();
-                    std::vector<double> wa(F.n);
-                    for (int i = 0; i < F.n; i++) wa[i] = sum_of(wg[l[a0 + i]]);
-                    cnt = chunk_counts(p, wa, 1);
-                    for (int i = 0; i < F.n; i++) {
-                        if (i == F.n / 2) F.gather_half = (int)items.size() - F.gather_off;
-                        split_planes(wg[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p),
-                                     kStripEmpty);
-                    }
-                    F.n_gather = (int)items.size() - F.gather_off;
-                }
-                groups.push_back(F);
+        // forward items
+        const int gf = p->dev.strip ? p->G : L.n;
+        for (int a0 = 0; a0 < L.n; a0 += gf) {
+            gb_spect_plan::FwdGroup F;
+            F.a0 = a0;
+            F.n = std::min(gf, L.n - a0);
+            F.item_off = (int)items.size();
+            F.ioff_off = (int)ioff.size();
+            std::vector<int> cnt(F.n, psf ? 0 : nopsf_chunks(p, L.n));
+            if (psf) {
+                std::vector<double> wa(F.n);
+                for (int i = 0; i < F.n; i++) wa[i] = sum_of(wf[l[a0 + i]]);
+                cnt = chunk_counts(p, wa, zs_f, p->fwd_items);
             }
-            return most;
-        };
-        L.max_fitems = forward_groups(p->dev.strip ? p->G : L.n, L.fgroups);
-        const int gs = p->dev.strip ? std::min(p->G, static_slots(p->dev)) : L.n;
-        if (p->dev.strip && gs < std::min(p->G, L.n))
-            L.max_sitems = forward_groups(gs, L.sgroups);
-        else {
-            L.sgroups = L.fgroups;
-            L.max_sitems = L.max_fitems;
+            for (int i = 0; i < F.n; i++) {
+                ioff.push_back((int)items.size() - F.item_off);
+                if (i == F.n / 2) F.half = (int)items.size() - F.item_off;
+                if (psf)
+                    split_planes(wf[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p), kStripEmpty);
+                else
+                    for (int k = 0; k < cnt[i]; k++)
+                        items.push_back(
+                            make_int4(i, k * p->Lp / cnt[i], (k + 1) * p->Lp / cnt[i], 0));
+            }
+            F.n_items = (int)items.size() - F.item_off;
+            ioff.push_back(F.n_items);
+            L.max_fitems = std::max(L.max_fitems, F.n_items);
+            if (p->dev.strip) {
+                F.gather_off = (int)items.size();
+                std::vector<double> wa(F.n);
+                for (int i = 0; i < F.n; i++) wa[i] = sum_of(wg[l[a0 + i]]);
+                cnt = chunk_counts(p, wa, 1);
+                for (int i = 0; i < F.n; i++) {
+                    if (i == F.n / 2) F.gather_half = (int)items.size() - F.gather_off;
+                    split_planes(wg[l[a0 + i]], cnt[i], i, items, strip_plane_cap(p), kStripEmpty);
+                }
+                F.n_gather = (int)items.size() - F.gather_off;
+            }
+            L.fgroups.push_back(F);
         }
         max_items = std::max(max_items, (size_t)L.max_fitems);
         // B1 items per angle group
@@ -795,7 +781,7 @@ gb_status gb_spect_plan_create(const gb_spect_desc *d, gb_spect_plan **out) {
         FAIL_CUDA(cudaStreamSynchronize(0));
     }
     // scratch: W for one angle group, likelihood ratio of all angles, multi-group bp
-    p->G = std::min(n, 16);
+    p->G = std::min(n, kGroup);
     FAIL_CUDA(dev_alloc(&p->d_W, p->G * stack_slot(g) * sizeof(float)));
     if (g.strip) FAIL_CUDA(dev_alloc(&p->d_Wf, p->G * stack_slot(g) * sizeof(float)));
     FAIL_CUDA(dev_alloc(&p->d_ratio, (size_t)n * p->N * p->nz * sizeof(float)));
@@ -1019,7 +1005,7 @@ static gb_status run_forward(gb_spect_plan *p, const float *obj, int subset, flo
     const size_t NZ = (size_t)p->N * p->nz;
     float *rows = fixed ? fixed->rows : p->d_Wf;
     float *partials = fixed ? fixed->partials : p->d_partials;
-    for (const gb_spect_plan::FwdGroup &F : fixed ? L.sgroups : L.fgroups) {
+    for (const gb_spect_plan::FwdGroup &F : L.fgroups) {
         const int *alist = p->d_alist + L.alist_off + F.a0;
         GB_CUDA(launch_fwd_group(p, F, -1, obj, alist, rows, partials, st));
         GB_CUDA(launch_reduce(F.n, p->d_ioff + F.ioff_off, (int)NZ, partials, out + F.a0 * NZ,
@@ -1370,7 +1356,7 @@ bool plan_forward_need(const gb_spect_plan *p, int subset, int *n_sel, int *n_it
     const int li = p ? list_index(p, subset) : -1;
     if (li < 0) return false;
     *n_sel = p->lists[li].n;
-    *n_items = std::max(p->lists[li].max_fitems, p->lists[li].max_sitems);
+    *n_items = p->lists[li].max_fitems;
     *floats = (size_t)std::max(*n_items, *n_sel) * p->N * p->nz;
     return true;
 }

@@ -9,9 +9,10 @@
 // read-only tables, the caller's input and output, and the static arrays below.
 //
 // Limits and behaviour:
-//   * the arrays hold kStaticPartials (16 MiB) and kStaticRows floats (64 MiB: the rows of 4
-//     angles of 128 x 128 x 128, of 16 or more of smaller planes, at a time); every GPU that
-//     loads the library keeps them until the process exits;
+//   * the arrays hold kStaticPartials (16 MiB) and kStaticRows floats (256 MiB: the rows of a
+//     group of 16 angles at 128 x 128 x 128); every GPU that loads the library keeps them until
+//     the process exits.  (64 MiB, with item lists of their own for groups of 4 angles, took 140
+//     us where this takes 105, and made every plan's lists 0.4 ms dearer);
 //   * the plan's work items times nx * nz partial sums must fit (at least one item per
 //     angle); larger requests are rejected with GB_ERR_SHAPE;
 //   * every call shares the arrays and the kernels overwrite every partial they later
@@ -30,8 +31,8 @@ namespace gb {
 
 static __device__ __align__(256) float g_fwd_static_scratch[kStaticPartials];
 static __device__ __align__(256) float g_fwd_static_rows[kStaticRows];
-// (a strip plan's largest slot: 182 planes of at most 172 rows of 128 values)
-static_assert(kStaticRows >= (size_t)182 * 182 * 128, "the rows of one angle fit");
+// (a strip plan's largest slot: 128 rows of taps of 22 on both sides, 182 planes, 128 values)
+static_assert(kStaticRows >= (size_t)kGroup * 182 * (128 + 2 * 22) * 128, "a group's rows fit");
 
 static std::mutex g_static_mu;
 static StaticScratch g_static_ptr[64] = {};

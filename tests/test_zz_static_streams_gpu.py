@@ -1,7 +1,6 @@
 """gb_spect_forward_static keeps to its fixed arrays: it may run beside the plan's own projections
-on another stream (interleaved calls with different objects give what one stream gives), in groups
-of as many angles as the arrays hold, and it refuses what needs more partial sums whatever the
-groups."""
+on another stream (interleaved calls with different objects give what one stream gives), and it
+refuses what needs more partial sums whatever the groups."""
 import numpy as np
 import pytest
 import torch
@@ -33,7 +32,6 @@ def test_static_beside_plan_calls(n, nz, angles, cuda):
     torch.cuda.synchronize()
     for k in range(len(objs)):
         assert torch.equal(plan[k], want[-1 - k]) and torch.equal(gback[k], back[k])
-        # (other groups, other chunks of planes: the partial sums round differently)
         assert rel_l2(outs[k].cpu().numpy(), want[k].cpu().numpy()) < 1e-5
 
 
